@@ -1,6 +1,8 @@
 // kernels_aux.cu -- the kernels around the sweep: coupling packing, field and
 // energy preparation, replica exchange + log-omega, visiting orders, f64
 // energies and spin unpacking.
+#include <cooperative_groups.h>
+
 #include "aux.cuh"
 #include "sweep_plain.cuh"
 
@@ -30,12 +32,24 @@ void launch_pack_rows(const float* J, int ld, int n, int nc, int ls,
 }
 
 // -------------------------------------------------- fields and energies
-// CTA per chain, warp per chunk of 256 columns (8 per lane).  F_i = sum_j
-// J_ij s_j in f64, from f32 partial sums over 32 rows (the products J_ij s_j
-// are exact in f32); H_i = f32(F_i + h_i); E = sum_i s_i (F_i / 2 + h_i)
-// (pysa/ising.py:37, pysa/qubo.py:37), summed per lane, then over the warp,
-// then over the chunks in order, so the result does not depend on timing.
+// F_i = sum_j J_ij s_j from f32 partial sums over 32 rows (the products
+// J_ij s_j are exact in f32), the partial sums accumulated as an exact f32
+// pair; H_i = F_i + h_i rounded once to f32; E = sum_i s_i (F_i / 2 + h_i)
+// (pysa/ising.py:37, pysa/qubo.py:37) in the same pairs, reduced over lanes,
+// column groups and cluster ranks in a fixed order, so the result does not
+// depend on timing.
 constexpr int kFieldWarps = 8;
+
+// Instance of chain c: binary search over chain_off.
+__device__ __forceinline__ int chain_instance(const pysa_gb_problems& p,
+                                              int64_t c) {
+  int lo = 0, hi = p.num_instances - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (p.chain_off[mid] <= c) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
 
 // Sparse instances: f_i = sum over row i's stored entries of J_ij s_j in f64
 // (the products are exact; padding entries have value 0), from the fixed
@@ -70,83 +84,27 @@ __device__ __forceinline__ bool is_sparse_inst(const pysa_gb_problems& p,
   return p.csr_row_off && p.csr_row_off[inst] >= 0;
 }
 
-__global__ void __launch_bounds__(32 * kFieldWarps) k_fields(const PrepArgs a) {
+__global__ void __launch_bounds__(32 * kFieldWarps)
+    k_fields_csr(const PrepArgs a) {
   __shared__ double e_s[kFieldWarps];
   const int64_t c = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
-  // instance of chain c: binary search over chain_off
-  int lo = 0, hi = a.p.num_instances - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.p.chain_off[mid] <= c) lo = mid; else hi = mid - 1;
-  }
-  const int inst = lo;
-  const int n = a.p.n[inst], ld = a.p.ld[inst];
+  const int inst = chain_instance(a.p, c);
+  if (!is_sparse_inst(a.p, inst)) return;  // uniform per CTA
+  const int n = a.p.n[inst];
   const bool ising = a.p.problem_type == PYSA_GB_ISING;
-  const float* J = a.p.J + a.p.j_off[inst];
   const float* h = a.p.h + a.p.h_off[inst];
   const uint32_t* sw = a.s.spins + c * a.p.words;
   double e = 0.0;
-  if (is_sparse_inst(a.p, inst)) {  // uniform per CTA
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const double f = csr_row_dot(a.p, inst, i, sw, ising);
-      const uint32_t bit = (sw[i >> 5] >> (i & 31)) & 1u;
-      const double si = bit ? 1.0 : (ising ? -1.0 : 0.0);
-      e += si * (0.5 * f + (double)h[i]);
-      a.fields[c * a.field_ld + i] = (float)(f + (double)h[i]);
-    }
-    e = warp_sum(e);
-    if (lane == 0) e_s[warp] = e;
-    __syncthreads();
-    if (threadIdx.x == 0 && a.set_energies) {
-      double t = 0.0;
-      for (int w = 0; w < nwarps; ++w) t += e_s[w];
-      a.s.energies[c] = (float)t;
-    }
-    return;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double f = csr_row_dot(a.p, inst, i, sw, ising);
+    const uint32_t bit = (sw[i >> 5] >> (i & 31)) & 1u;
+    const double si = bit ? 1.0 : (ising ? -1.0 : 0.0);
+    e += si * (0.5 * f + (double)h[i]);
+    a.fields[c * a.field_ld + i] = (float)(f + (double)h[i]);
   }
-  constexpr int TC = 8;  // columns per lane per chunk
-  for (int base = 256 * warp; base < n; base += 256 * nwarps) {
-    double F[TC];
-    float part[TC];
-#pragma unroll
-    for (int k = 0; k < TC; ++k) {
-      F[k] = 0.0;
-      part[k] = 0.0f;
-    }
-    for (int j = 0; j < n; ++j) {
-      const uint32_t bit = (sw[j >> 5] >> (j & 31)) & 1u;
-      const float sj = bit ? 1.0f : (ising ? -1.0f : 0.0f);
-      if (sj != 0.0f) {
-        const float* row = J + (int64_t)j * ld;  // J symmetric: J[j][i]
-#pragma unroll
-        for (int k = 0; k < TC; ++k) {
-          const int col = base + 32 * k + lane;
-          if (col < n) part[k] += sj * row[col];
-        }
-      }
-      if ((j & 31) == 31 || j == n - 1) {
-#pragma unroll
-        for (int k = 0; k < TC; ++k) {
-          F[k] += (double)part[k];
-          part[k] = 0.0f;
-        }
-      }
-    }
-    double ec = 0.0;
-#pragma unroll
-    for (int k = 0; k < TC; ++k) {
-      const int col = base + 32 * k + lane;
-      if (col < n) {
-        const uint32_t bit = (sw[col >> 5] >> (col & 31)) & 1u;
-        const double si = bit ? 1.0 : (ising ? -1.0 : 0.0);
-        ec += si * (0.5 * F[k] + (double)h[col]);
-        a.fields[c * a.field_ld + col] = (float)(F[k] + (double)h[col]);
-      }
-    }
-    e += warp_sum(ec);
-  }
+  e = warp_sum(e);
   if (lane == 0) e_s[warp] = e;
   __syncthreads();
   if (threadIdx.x == 0 && a.set_energies) {
@@ -154,6 +112,377 @@ __global__ void __launch_bounds__(32 * kFieldWarps) k_fields(const PrepArgs a) {
     for (int w = 0; w < nwarps; ++w) t += e_s[w];
     a.s.energies[c] = (float)t;
   }
+}
+
+// ---- dense instances
+// A CTA of 8 warps holds CH chains x W columns in registers (a warp: 8 chains
+// x 32 TC columns) and walks the n rows 32 at a time: the J tile (cp.async,
+// double-buffered) is read once per CH chains instead of once per chain, and
+// the chains' spins become +-1 / 0 multipliers in shared memory, so a row is
+// one shared load and two broadcasts per 8 TC multiply-adds.  Bound by those
+// shared loads (three 16-byte ones per 32 multiply-adds); a warp of f64
+// instructions takes about 64 times the cycles of an f32 one on this GPU, so
+// f64 is kept out of the loop by adding each 32-row partial sum into an f32
+// pair with an exact two-sum.  The pair holds the sum of the partial sums to
+// 2^-48 of its largest term, and exactly when the sum's bits span fewer than
+// 48 places: fields and energies equal those of the f64 accumulation bit for
+// bit on every size measured (normal couplings, and ones spread over nine
+// decades).  A cluster of up to 8 CTAs splits the columns while there are too
+// few chains to fill the GPU; its energies meet in rank 0 through distributed
+// shared memory.
+// Measured against one CTA per chain with f64 accumulation: n = 2048, 9728
+// chains 14.2 -> 2.7 ms; n = 777, 9728 chains 2.92 -> 0.55 ms; n = 1000, 4096
+// chains 0.97 -> 0.37 ms; n = 64, 20000 chains 0.139 -> 0.052 ms; n = 912,
+// 100 chains 0.24 -> 0.064 ms (times with the launch).
+
+// s + e = a + b exactly (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float& e) {
+  const float s = a + b;
+  const float bb = s - a;
+  e = (a - (s - bb)) + (b - bb);
+  return s;
+}
+
+// Pair (hi, lo) + x.
+__device__ __forceinline__ void pair_add(float2& p, float x) {
+  float e;
+  p.x = two_sum(p.x, x, e);
+  p.y += e;
+}
+
+// Field of one column in f64, for the columns whose f32 pair left the finite
+// range (infinite or NaN couplings, or sums past f32).
+static __device__ __noinline__ double field_f64(const float* J, int ld, int n,
+                                                const uint32_t* sw, bool ising,
+                                                int col) {
+  double F = 0.0;
+  float part = 0.0f;
+  for (int j = 0; j < n; ++j) {
+    const uint32_t bit = (sw[j >> 5] >> (j & 31)) & 1u;
+    if (bit)
+      part += J[(int64_t)j * ld + col];
+    else if (ising)
+      part -= J[(int64_t)j * ld + col];
+    if ((j & 31) == 31 || j == n - 1) {
+      F += (double)part;
+      part = 0.0f;
+    }
+  }
+  return F;
+}
+
+__device__ __forceinline__ void cp_async_zfill16(void* dst, const void* src,
+                                                 int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_zfill4(void* dst, const void* src,
+                                                int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes)
+               : "memory");
+}
+
+template <int TC, int CG>
+struct FieldTile {
+  static constexpr int CH = 8 * (kFieldWarps / CG);  // chains per CTA
+  static constexpr int W = 32 * TC * CG;             // columns per pass
+  static constexpr size_t J_BYTES = (size_t)32 * W * 4;
+  static constexpr size_t M_BYTES = (size_t)32 * CH * 4;
+  static constexpr size_t E_BYTES = (size_t)CG * CH * 8;
+  static constexpr size_t BYTES = 2 * (J_BYTES + M_BYTES) + E_BYTES;
+};
+
+template <int TC, int CG>
+__global__ void __launch_bounds__(32 * kFieldWarps, 2)
+    k_fields(const PrepArgs a) {
+  using T = FieldTile<TC, CG>;
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char fsm[];
+  float* jt = reinterpret_cast<float*>(fsm);                   // [2][32][W]
+  float* mt = reinterpret_cast<float*>(fsm + 2 * T::J_BYTES);  // [2][32][CH]
+  float2* es =                                                 // [CG][CH]
+      reinterpret_cast<float2*>(fsm + 2 * (T::J_BYTES + T::M_BYTES));
+  cg::cluster_group cl = cg::this_cluster();
+  const int csize = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wc = warp % CG, wg = warp / CG;
+  const int64_t tile0 = (int64_t)(blockIdx.x / csize) * T::CH;
+  const int64_t tile1 = tile0 + T::CH < a.p.num_chains ? tile0 + T::CH
+                                                       : a.p.num_chains;
+  const bool ising = a.p.problem_type == PYSA_GB_ISING;
+  const bool vec_out = TC == 4 && a.field_ld % 4 == 0 &&
+                       reinterpret_cast<uintptr_t>(a.fields) % 16 == 0;
+  // the tile's chains, one instance at a time
+  for (int64_t c0 = tile0; c0 < tile1;) {
+    const int inst = chain_instance(a.p, c0);
+    int64_t c1 = inst + 1 < a.p.num_instances ? a.p.chain_off[inst + 1]
+                                              : (int64_t)a.p.num_chains;
+    c1 = c1 < tile1 ? (c1 > c0 ? c1 : c0 + 1) : tile1;
+    if (is_sparse_inst(a.p, inst)) {  // k_fields_csr's
+      c0 = c1;
+      continue;
+    }
+    const int n = a.p.n[inst], ld = a.p.ld[inst];
+    const float* J = a.p.J + a.p.j_off[inst];
+    const float* h = a.p.h + a.p.h_off[inst];
+    const bool vec_in =
+        ld % 4 == 0 && reinterpret_cast<uintptr_t>(J) % 16 == 0;
+    const int nt = (n + 31) >> 5;
+    const int64_t cw = c0 + 8 * wg;  // this warp's first chain
+    float2 ep[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g) ep[g] = make_float2(0.0f, 0.0f);
+
+    for (int base = rank * T::W; base < n; base += csize * T::W) {
+      auto stage = [&](int t, int buf) {  // rows 32 t ... of J
+        float* dst = jt + buf * (32 * T::W);
+        if (vec_in) {
+          for (int e = tid; e < 32 * T::W / 4; e += blockDim.x) {
+            const int r = e / (T::W / 4), q = 4 * (e % (T::W / 4));
+            const int row = 32 * t + r, col = base + q;
+            const int left = row < n ? n - col : 0;
+            const int bytes = left >= 4 ? 16 : left > 0 ? 4 * left : 0;
+            cp_async_zfill16(dst + r * T::W + q,
+                             bytes ? J + (int64_t)row * ld + col : J, bytes);
+          }
+        } else {
+          for (int e = tid; e < 32 * T::W; e += blockDim.x) {
+            const int r = e / T::W, q = e % T::W;
+            const int row = 32 * t + r, col = base + q;
+            const bool in = row < n && col < n;
+            cp_async_zfill4(dst + r * T::W + q,
+                            in ? J + (int64_t)row * ld + col : J, in ? 4 : 0);
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      // word t of this thread's chain; its multipliers, [row][chain]
+      constexpr int RPT = T::CH / 8;  // rows per thread: 32 CH / 256
+      const int mc = tid % T::CH, mr = (tid / T::CH) * RPT;
+      auto word = [&](int t) {
+        return c0 + mc < c1 ? a.s.spins[(c0 + mc) * a.p.words + t] : 0u;
+      };
+      auto put_mult = [&](uint32_t w, int buf) {
+#pragma unroll
+        for (int r = 0; r < RPT; ++r)
+          mt[buf * (32 * T::CH) + (mr + r) * T::CH + mc] =
+              ((w >> (mr + r)) & 1u) ? 1.0f : (ising ? -1.0f : 0.0f);
+      };
+      stage(0, 0);
+      put_mult(word(0), 0);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+
+      float2 F[8][TC];
+#pragma unroll
+      for (int g = 0; g < 8; ++g)
+#pragma unroll
+        for (int k = 0; k < TC; ++k) F[g][k] = make_float2(0.0f, 0.0f);
+      for (int t = 0; t < nt; ++t) {
+        const int buf = t & 1;
+        uint32_t wn = 0u;
+        if (t + 1 < nt) {
+          stage(t + 1, buf ^ 1);
+          wn = word(t + 1);
+        }
+        float part[8][TC];
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+#pragma unroll
+          for (int k = 0; k < TC; ++k) part[g][k] = 0.0f;
+        const float* jr = jt + buf * (32 * T::W) + (wc * 32 + lane) * TC;
+        const float* mr8 = mt + buf * (32 * T::CH) + 8 * wg;
+        // rows past n are zero in the tile: they add +-0
+#pragma unroll 4
+        for (int r = 0; r < 32; ++r) {
+          float v[TC];
+          if constexpr (TC == 4) {
+            const float4 x = *reinterpret_cast<const float4*>(jr + r * T::W);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+          } else {
+#pragma unroll
+            for (int k = 0; k < TC; ++k) v[k] = jr[r * T::W + k];
+          }
+          const float4 m0 =
+              *reinterpret_cast<const float4*>(mr8 + r * T::CH);
+          const float4 m1 =
+              *reinterpret_cast<const float4*>(mr8 + r * T::CH + 4);
+          const float m[8] = {m0.x, m0.y, m0.z, m0.w,
+                              m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+#pragma unroll
+            for (int k = 0; k < TC; ++k)
+              part[g][k] = fmaf(m[g], v[k], part[g][k]);
+        }
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+#pragma unroll
+          for (int k = 0; k < TC; ++k) pair_add(F[g][k], part[g][k]);
+        if (t + 1 < nt) {
+          put_mult(wn, buf ^ 1);
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+      }
+
+      // fields out, energy terms s (F / 2 + h)
+      const int col0 = base + (wc * 32 + lane) * TC;
+      float hc[TC];
+#pragma unroll
+      for (int k = 0; k < TC; ++k) hc[k] = col0 + k < n ? h[col0 + k] : 0.0f;
+#pragma unroll
+      for (int g = 0; g < 8; ++g) {
+        const int64_t c = cw + g;
+        if (c >= c1 || col0 >= n) continue;
+        const uint32_t* sw = a.s.spins + c * a.p.words;
+        const uint32_t wv = sw[col0 >> 5];  // TC divides 32: one word
+        float H[TC];
+#pragma unroll
+        for (int k = 0; k < TC; ++k) {
+          const float hi = F[g][k].x, lo = F[g][k].y;
+          float e1, e2, e3;
+          const float s1 = two_sum(hi, hc[k], e1);
+          const float t1 = two_sum(e1, lo, e2);
+          const float r1 = two_sum(s1, t1, e3);
+          H[k] = r1 + (e3 + e2);
+          const float half = 0.5f * hi;
+          const bool up = (wv >> ((col0 + k) & 31)) & 1u;
+          const float sg = up ? 1.0f : (ising ? -1.0f : 0.0f);
+          if (fabsf(hi) < INFINITY && fabsf(s1) < INFINITY) {
+            const float s2 = two_sum(half, hc[k], e1);
+            pair_add(ep[g], sg * s2);
+            ep[g].y += sg * (e1 + 0.5f * lo);
+          } else if (col0 + k < n) {
+            H[k] = (float)(field_f64(J, ld, n, sw, ising, col0 + k) +
+                           (double)hc[k]);
+            ep[g].x = __int_as_float(0x7fc00000);  // energy in f64 below
+          }
+        }
+        float* out = a.fields + c * a.field_ld + col0;
+        if (vec_out && col0 + TC <= n) {
+          if constexpr (TC == 4)
+            *reinterpret_cast<float4*>(out) =
+                make_float4(H[0], H[1], H[2], H[3]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < TC; ++k)
+            if (col0 + k < n) out[k] = H[k];
+        }
+      }
+    }  // column passes
+
+    if (a.set_energies) {
+      // lane sums of the pairs: three halving steps leave chain 4 b4 + 2 b3
+      // + b2 (bits of the lane) in every lane, two more finish the sum
+#pragma unroll
+      for (int o = 4; o; o >>= 1) {
+        const bool up = lane & (4 * o);
+#pragma unroll
+        for (int g = 0; g < o; ++g) {
+          const float2 mine = up ? ep[g + o] : ep[g];
+          const float2 give = up ? ep[g] : ep[g + o];
+          ep[g] = mine;
+          const float gx = __shfl_xor_sync(0xffffffffu, give.x, 4 * o);
+          const float gy = __shfl_xor_sync(0xffffffffu, give.y, 4 * o);
+          pair_add(ep[g], gx);
+          ep[g].y += gy;
+        }
+      }
+#pragma unroll
+      for (int o = 2; o; o >>= 1) {
+        const float gx = __shfl_xor_sync(0xffffffffu, ep[0].x, o);
+        const float gy = __shfl_xor_sync(0xffffffffu, ep[0].y, o);
+        pair_add(ep[0], gx);
+        ep[0].y += gy;
+      }
+      if ((lane & 3) == 0) es[wc * T::CH + 8 * wg + (lane >> 2)] = ep[0];
+      if (csize > 1) cl.sync(); else __syncthreads();
+      if (rank == 0 && tid < T::CH && c0 + tid < c1) {
+        double t = 0.0;
+        bool fin = true;
+        for (int r = 0; r < csize; ++r) {
+          const float2* er = csize > 1 ? cl.map_shared_rank(es, r) : es;
+          for (int w = 0; w < CG; ++w) {
+            const float2 v = er[w * T::CH + tid];
+            fin = fin && fabsf(v.x) < INFINITY;
+            t += (double)v.x + (double)v.y;
+          }
+        }
+        if (!fin) {
+          const uint32_t* sw = a.s.spins + (c0 + tid) * a.p.words;
+          t = 0.0;
+          for (int col = 0; col < n; ++col) {
+            const double si = ((sw[col >> 5] >> (col & 31)) & 1u)
+                                  ? 1.0 : (ising ? -1.0 : 0.0);
+            t += si * (0.5 * field_f64(J, ld, n, sw, ising, col) +
+                       (double)h[col]);
+          }
+        }
+        a.s.energies[c0 + tid] = (float)t;
+      }
+      if (csize > 1) cl.sync(); else __syncthreads();
+    }
+    c0 = c1;
+  }
+}
+
+template <int TC, int CG>
+static cudaError_t launch_fields_t(const PrepArgs& a, int csize,
+                                   cudaStream_t st) {
+  using T = FieldTile<TC, CG>;
+  static bool attr[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(
+        k_fields<TC, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (int)T::BYTES);
+    if (e != cudaSuccess) return e;
+    attr[dev] = true;
+  }
+  const int64_t tiles = ((int64_t)a.p.num_chains + T::CH - 1) / T::CH;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * csize));
+  cfg.blockDim = dim3(32 * kFieldWarps);
+  cfg.dynamicSmemBytes = T::BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)csize;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_fields<TC, CG>, a);
+}
+
+// The tile by size: 256 columns x 32 chains (4 columns a lane) when that
+// still gives every SM work; up to 128 columns, 64 chains; up to 32 columns,
+// one column a lane.  Few chains, or few per instance (a tile's chains are
+// done one instance after another), take 8 chains x 256 columns, the columns
+// split over a cluster.
+static cudaError_t launch_fields(const PrepArgs& a, cudaStream_t st) {
+  const int64_t chains = a.p.num_chains;
+  const int64_t per = chains / (a.p.num_instances > 0 ? a.p.num_instances : 1);
+  const int n = a.p.max_n;
+  constexpr int64_t kFill = 2 * 152;  // CTAs that keep the GPU busy
+  if (per >= 64 && n <= 32 && chains / 64 >= kFill)
+    return launch_fields_t<1, 1>(a, 1, st);
+  if (per >= 64 && n <= 128 && chains / 64 >= kFill)
+    return launch_fields_t<4, 1>(a, 1, st);
+  const int passes = (n + 255) / 256;
+  if (per >= 32 && chains / 32 * passes >= kFill) {
+    int cs = 1;
+    while (cs < 8 && cs < passes && chains / 32 * cs < kFill) cs *= 2;
+    return launch_fields_t<4, 2>(a, cs, st);
+  }
+  int cs = 1;
+  while (cs < 8 && cs < passes && (chains + 7) / 8 * cs < kFill) cs *= 2;
+  return launch_fields_t<1, 8>(a, cs, st);
 }
 
 // CTA per read, thread per replica: the slot betas and the initial best.
@@ -177,10 +506,13 @@ __global__ void k_read_init(const PrepArgs a) {
 }
 
 void launch_prepare(const PrepArgs& a, cudaStream_t st) {
-  if (a.p.num_chains > 0) {
-    int warps = (a.p.max_n + 255) / 256;
-    warps = warps < 1 ? 1 : warps > kFieldWarps ? kFieldWarps : warps;
-    k_fields<<<(unsigned)a.p.num_chains, warps * 32, 0, st>>>(a);
+  if (a.p.num_chains > 0 && a.p.num_instances > 0) {
+    launch_fields(a, st);
+    if (a.p.csr_row_off) {
+      int warps = (a.p.max_n + 255) / 256;
+      warps = warps < 1 ? 1 : warps > kFieldWarps ? kFieldWarps : warps;
+      k_fields_csr<<<(unsigned)a.p.num_chains, warps * 32, 0, st>>>(a);
+    }
   }
   if (a.p.num_reads > 0)
     k_read_init<<<(unsigned)a.p.num_reads, 128, 0, st>>>(a);
