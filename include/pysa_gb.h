@@ -145,7 +145,11 @@ typedef struct {
   int32_t field_ld;       /* row stride of fields (>= 32 * ceil(max_n/32),
                              a multiple of 4; fields 16-byte aligned) */
   int32_t perm_slots;     /* visiting orders held (sweeps per batch) */
-  int32_t *perm;          /* [perm_slots, num_instances, max_n] */
+  int32_t *perm;          /* [perm_slots, num_instances, max_n] visiting
+                             orders; sweeps write the level schedule of
+                             sparse instances there in either order (NULL
+                             is accepted in sequential order: such
+                             instances then sweep more slowly) */
   float *packed_j;        /* couplings in the sweep kernel's row layout */
   int64_t packed_j_elems; /* capacity of packed_j */
   int32_t *items;         /* [num_items, 8] work list of the sweep kernel */
@@ -198,7 +202,7 @@ typedef struct {
    * group, padding entries with value 0 */
   int32_t csr_width;
   int32_t csr_chains;     /* host, from pysa_gb_setup: chains per work item
-                             (128, or 64 / 32 while that leaves SMs idle) */
+                             (32) */
   /* host, from pysa_gb_setup: work items of the wide-instance sweep (dense
    * instances with n > 4096: fields in this workspace's fields array, J
    * read in place, so j_off and ld of those instances must be multiples

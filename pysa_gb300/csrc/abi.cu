@@ -279,30 +279,19 @@ int pysa_gb_setup(const pysa_gb_problems* p, const pysa_gb_host_tables* host,
     }
     ws->variant_count[v] = (int32_t)items.size() - ws->variant_start[v];
   }
-  // sparse instances: up to 128 chains per item of the sparse-row sweep,
-  // fewer while the items would leave SMs idle
+  // sparse instances: 32 chains per item of the sparse-row sweep
   ws->csr_item_start = (int32_t)items.size();
-  int cpb = kCsrChains;
-  {
-    int64_t sparse_chains = 0;
-    for (int i = 0; i < p->num_instances; ++i)
-      if (is_sparse(host, i))
-        sparse_chains += (int64_t)replicas_host[i] * reads_host[i];
-    const int sms = sm_count();
-    while (cpb > 32 && (sparse_chains + cpb - 1) / cpb < sms) cpb /= 2;
-  }
-  // the sparse-row sweep keeps every chain's spin words (and, in random
-  // order, the visiting order and a record slab) in shared memory
+  const int cpb = kCsrChains;
+  // the sparse-row sweep keeps every chain's spin words, the level schedule
+  // and (in random order) the visiting order in shared memory; the bound is
+  // n <= 26 752
   {
     const size_t words = (size_t)(p->max_n + 31) / 32;
-    auto smem = [&](int ch) {
-      return words * ch * 4 + (size_t)p->max_n * 4 + 17408 + 1024;
-    };
+    const size_t smem = words * 32 * 4 + (size_t)p->max_n * 4 + 17408 + 1024;
     bool any_sparse = false;
     for (int i = 0; i < p->num_instances; ++i)
       any_sparse |= is_sparse(host, i);
-    while (cpb > 32 && smem(cpb) > 232448) cpb /= 2;
-    if (any_sparse && smem(cpb) > 232448)
+    if (any_sparse && smem > 232448)
       return fail(PYSA_GB_ERR_SIZE,
                   "sparse instances: n too large for the sparse-row sweep's "
                   "shared memory at 32 chains per CTA");
@@ -775,6 +764,22 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
     }
     return PYSA_GB_OK;
   }
+  CsrArgs ca;
+  ca.p = *p;
+  ca.s = *s;
+  ca.perm = ws->perm_slots > 0 ? ws->perm : nullptr;
+  ca.perm_slots = a.perm_slots;
+  ca.num_items = ws->csr_item_count;
+  ca.items = reinterpret_cast<const SweepItem*>(ws->items) +
+             ws->csr_item_start;
+  ca.seed = o->seed;
+  ca.width = ws->csr_width;
+  ca.pad_ = 0;
+  for (int r = 0; r < 10; ++r) {
+    ca.round_keys[2 * r] = (uint32_t)o->seed + (uint32_t)r * 0x9E3779B9u;
+    ca.round_keys[2 * r + 1] =
+        (uint32_t)(o->seed >> 32) + (uint32_t)r * 0xBB67AE85u;
+  }
   for (int sw = 0; sw < num_sweeps; ++sw) {
     if (use_tc && (phases & 1)) {
       if (random) {
@@ -796,18 +801,11 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       if (e != cudaSuccess) return cuda_fail(e, "sweep launch");
     }
     if ((phases & 1) && ws->csr_item_count > 0) {
-      CsrArgs ca;
-      ca.p = *p;
-      ca.s = *s;
-      ca.perm = ws->perm;
-      ca.perm_slots = a.perm_slots;
-      ca.num_items = ws->csr_item_count;
-      ca.items = reinterpret_cast<const SweepItem*>(ws->items) +
-                 ws->csr_item_start;
-      ca.seed = o->seed;
-      ca.width = ws->csr_width;
-      ca.chains = ws->csr_chains > 0 ? ws->csr_chains : kCsrChains;
-      cudaError_t e = launch_csr(ca, random, st);
+      // the level schedule: of every sweep's order in random order, once
+      // per call in sequential order
+      cudaError_t e = cudaSuccess;
+      if (random || sw == 0) e = launch_csr_schedule(ca, random, st);
+      if (e == cudaSuccess) e = launch_csr(ca, random, st);
       if (e != cudaSuccess) return cuda_fail(e, "sparse sweep launch");
     }
     if ((phases & 1) && ws->wide_item_count > 0) {

@@ -4,290 +4,763 @@
 // Same sweep as pysa/simulation.py:60-76 (sequential) / :41-57 (random
 // order) with the rule of pysa/ising.py:40-63 / pysa/qubo.py:40-63, but the
 // field of spin i is recomputed from the nonzero couplings of row i instead
-// of a dense dot, so an attempt costs O(degree).  One thread per chain; the
-// CTA's 128 chains keep their spins bit-packed in shared memory ([word]
-// [chain], so the threads' words are consecutive); all of them visit spin i
-// together, so the row's entries are the same addresses for every thread
-// (broadcast loads through L1).
+// of a dense dot, so an attempt costs O(degree).
+//
+// A CTA holds 32 chains (lane = chain); shared memory holds their spins as
+// one word per spin, bit = chain, so a warp reads a neighbour's spins with
+// one broadcast load and its own chain's with a shift by the lane.  The
+// visiting positions are cut into quads of four (one Philox draw each), and
+// the quads into levels: a quad's level is one more than the largest level of
+// the earlier quads that read its spins or hold spins it reads.  Quads of
+// one level do not see each other's flips, so the CTA's warps decide them at
+// the same time, a barrier apart from the next level, and every attempt reads
+// exactly the spins it reads when the positions are visited one by one.  A
+// quad is decided in order by one warp; its records and random thresholds
+// are fetched before the barrier.  (Where quads tie unrelated positions
+// together, as at the row ends of a lattice whose side is no multiple of
+// four, the schedule cuts them into shorter units; see k_csr_schedule.)
+//
+// Bound by instruction issue and, per level, by the latency of one quad's four
+// dependent attempts.  Measured against one thread per chain visiting the
+// positions one by one (times per sweep with the exchange): 64 x 64 lattice,
+// 4000 chains 1.44 -> 0.13 ms in visiting order (79 levels), 1.66 -> 0.44 ms
+// in random order (most of the rest makes the orders); 100 x 100, 2000 chains
+// 3.7 -> 0.39 ms; 33 x 33, 16000 chains 0.43 -> 0.19 ms.
 //
 // Row layout: the entries of row i are grouped by column % 8 (ascending
 // column inside a group) and rows[9 i + k] .. rows[9 i + k + 1] delimit group
 // k; or, when every row has at most 32 entries, each row is a fixed record
 // of D = 4, 8, 16 or 32 entries in that order (bit 31 of the column marks
 // the last entry of a group, padding entries have value 0), read with
-// vector loads all at once.  The field is summed as eight partial sums, one per group, added in
-// group order, then h_i: the fixed-order f32 dot of the oracle with its zero
-// terms left out (adding a zero product changes no partial sum), so
-// trajectories equal the oracle's for any couplings, not only integer ones.
+// vector loads all at once.  The field is summed as eight partial sums, one
+// per group, added in group order, then h_i: the fixed-order f32 dot of the
+// oracle with its zero terms left out (adding a zero product changes no
+// partial sum), so trajectories equal the oracle's for any couplings, not
+// only integer ones.
+#include <type_traits>
+
 #include "common.cuh"
 #include "csr_api.h"
 #include "sweep_plain.cuh"
 
 namespace pysa_gb {
 
-// Asynchronous global -> shared copies (no register staging).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   smem_addr(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
-                   smem_addr(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+// --------------------------------------------------------------- schedule
+// The level schedule of one visiting order lives in the high halves of the
+// order's row of the visiting-order workspace (spins are below 2^16).  With
+// nu units in nl levels: entry k < nu the k-th unit by (level, position),
+// entries nu ... nu + nl the levels' first places in that list, and the last
+// three entries of the row's first n: whether field sums are exact in any
+// order, nu, nl.  A unit is quad q, or (when nu > quads) q << 4 | first
+// position in it << 2 | positions - 1.  That takes nu + nl + 4 <= n entries,
+// which quads fit for n >= 10; below that, and where there is no such
+// workspace, every quad is a level of its own.
+constexpr int kSchedMinN = 10;
+constexpr int kSchedThreads = 512;
+// Widest instance whose quads may be cut (shared memory, 16 bits per unit).
+constexpr int kSchedCutN = 8192;
+
+__host__ __device__ constexpr int csr_quads(int n) { return (n + 3) >> 2; }
+
+// Schedule entries (units, and first places of the levels) the sweep holds:
+// at most n - 2 when quads may be cut, else two per quad and one.
+__host__ __device__ constexpr int sched_cap(int n) {
+  const int cut = (n < kSchedCutN ? n : kSchedCutN) + 1;
+  const int whole = 2 * csr_quads(n) + 1;
+  return cut > whole ? cut : whole;
 }
 
-// Fixed records are staged 32 visiting positions at a time into a double
-// buffer of shared memory, one row per thread of the first warp, while the
-// previous 32 are decided: [D columns][D values][h_i][pad] per row.
-template <int D>
-struct RecSlab {
-  static constexpr int STRIDE = 2 * D + 4;  // floats per staged row
-  static constexpr size_t BYTES = D > 0 ? (size_t)2 * 32 * STRIDE * 4 : 0;
-};
+// Shared memory of k_csr_schedule for up to nu units of n positions.
+__host__ __device__ constexpr size_t sched_bytes(int nu, int n, bool random,
+                                                 bool cut) {
+  return 4 * ((size_t)nu + 1) + 4 * (size_t)nu + 2 * (size_t)nu +
+         (random ? 2 * (size_t)n : 0) +
+         (cut ? 2 * (size_t)n + 2 * ((size_t)nu + 1) : 0);
+}
 
-// One staged fixed record in registers (all lanes read the same row of the
-// slab: broadcast loads).
-template <int D>
-struct Rec {
-  int32_t cols[D];
-  float vals[D];
-  float h;
-  __device__ __forceinline__ void load(const float* rec) {
-#pragma unroll
-    for (int q = 0; q < D / 4; ++q) {
-      const int4 c4 = reinterpret_cast<const int4*>(rec)[q];
-      const float4 v4 = reinterpret_cast<const float4*>(rec + D)[q];
-      cols[4 * q + 0] = c4.x; cols[4 * q + 1] = c4.y;
-      cols[4 * q + 2] = c4.z; cols[4 * q + 3] = c4.w;
-      vals[4 * q + 0] = v4.x; vals[4 * q + 1] = v4.y;
-      vals[4 * q + 2] = v4.z; vals[4 * q + 3] = v4.w;
+// CTA per instance.  Units are levelled 512 at a time (earlier ones are
+// final), the levels of a chunk raised until none changes; then a counting
+// sort, stable in the position.  When the quads give fewer than 8 per level,
+// they are cut between positions that do not touch (neither reads the
+// other's spin) and levelled again; the cut schedule is kept when it has
+// less than two thirds of the levels.
+template <bool RANDOM>
+__global__ void __launch_bounds__(kSchedThreads)
+    k_csr_schedule(const CsrArgs a) {
+  extern __shared__ __align__(16) unsigned char ssm[];
+  __shared__ int max_level;
+  __shared__ int warp_sum_s[kSchedThreads / 32];
+  const int inst = blockIdx.x;
+  if (a.p.csr_row_off[inst] < 0) return;  // dense
+  const int n = a.p.n[inst], nq = csr_quads(n);
+  if (n < kSchedMinN) return;
+  const uint32_t sweep = (uint32_t)(*a.s.sweep_counter);
+  int32_t* row =
+      a.perm + ((int64_t)(RANDOM ? sweep % (uint32_t)a.perm_slots : 0u) *
+                    a.p.num_instances + inst) * (int64_t)a.p.max_n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int32_t* rows =
+      a.width > 0 ? nullptr : a.p.csr_rows + a.p.csr_row_off[inst] * 9;
+  const int32_t* colp = a.p.csr_col + a.p.csr_ent_off[inst];
+  const float* valp = a.p.csr_val + a.p.csr_ent_off[inst];
+  auto entries = [&](int i, int64_t& e, int64_t& e1) {
+    e = (int64_t)a.width * i;
+    e1 = e + a.width;
+    if (a.width == 0) {
+      e = rows[(int64_t)i * 9];
+      e1 = rows[(int64_t)i * 9 + 8];
     }
-    h = rec[2 * D];
+  };
+  auto column = [&](int64_t e) { return __ldg(colp + e) & 0x7fffffff; };
+  // positions of the spins, and the uncut/cut units' tables behind it
+  uint16_t* inv = reinterpret_cast<uint16_t*>(ssm);  // [n], random
+  unsigned char* tab = ssm + (RANDOM ? 2 * (((size_t)n + 1) & ~1ull) : 0);
+  bool odd = false;  // a coupling that is no integer below 2^18
+  for (int t = tid; t < n; t += blockDim.x) {
+    if (RANDOM)
+      inv[row[t] & 0xFFFF] = (uint16_t)t;
+    else
+      row[t] = t;
+    if (a.width > 0)
+      for (int64_t e = (int64_t)a.width * t, e1 = e + a.width; e < e1; ++e) {
+        const float v = __ldg(valp + e);
+        odd = odd || !(fabsf(v) <= 262144.0f && v == rintf(v));
+      }
   }
-  // field sum over the current spins; a group's partial sum joins the
-  // total at the entry flagged last in it
-  __device__ __forceinline__ float dot(const uint32_t* my, int CH,
-                                       bool ising) const {
-    uint32_t words[D];
+  // up to 32 such couplings add up without rounding, whatever the order
+  const bool any_order = !__syncthreads_or(odd) && a.width > 0;
+  auto spin_at = [&](int t) { return RANDOM ? row[t] & 0xFFFF : t; };
+  auto pos_of = [&](int i) { return RANDOM ? (int)inv[i] : i; };
+
+  int best_nl = 0;
+  for (int cut = 0; cut < 2; ++cut) {
+    int nu = nq;
+    uint16_t *uid = nullptr, *first = nullptr;
+    unsigned char* mem = tab;
+    if (cut) {
+      // unit of every position: a running count of the unit starts
+      uid = reinterpret_cast<uint16_t*>(mem);                    // [n]
+      mem += 2 * (((size_t)n + 1) & ~1ull);
+      int carry = 0;
+      for (int t0 = 0; t0 < n; t0 += blockDim.x) {
+        const int t = t0 + tid;
+        int start = 0;
+        if (t < n) {
+          start = 1;
+          if (t & 3) {
+            const int i = spin_at(t), j = spin_at(t - 1);
+            int64_t e, e1;
+            for (entries(i, e, e1); e < e1; ++e)
+              if (column(e) == j) start = 0;
+            for (entries(j, e, e1); e < e1; ++e)
+              if (column(e) == i) start = 0;
+          }
+        }
+        int v = start;
 #pragma unroll
-    for (int e = 0; e < D; ++e) {
-      const int c = cols[e] & 0x7fffffff;
-      words[e] = my[(c >> 5) * CH];
+        for (int o = 1; o < 32; o <<= 1) {
+          const int up = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += up;
+        }
+        if (lane == 31) warp_sum_s[warp] = v;
+        __syncthreads();
+        int before = carry, all = 0;
+        for (int w = 0; w < kSchedThreads / 32; ++w) {
+          if (w < warp) before += warp_sum_s[w];
+          all += warp_sum_s[w];
+        }
+        if (t < n) uid[t] = (uint16_t)(before + v - 1);
+        carry += all;
+        __syncthreads();
+      }
+      nu = carry;
+      first = reinterpret_cast<uint16_t*>(mem);                  // [nu + 1]
+      mem += 2 * (((size_t)nu + 2) & ~1ull);
+      for (int t = tid; t < n; t += blockDim.x)
+        if (t == 0 || uid[t] != uid[t - 1]) first[uid[t]] = (uint16_t)t;
+      if (tid == 0) first[nu] = (uint16_t)n;
     }
-    float sum = 0.0f, part = 0.0f;
-#pragma unroll
-    for (int e = 0; e < D; ++e) {
-      const int c = cols[e] & 0x7fffffff;
-      const bool bit = (words[e] >> (c & 31)) & 1u;
-      if (ising)
-        part += bit ? vals[e] : -vals[e];
-      else if (bit)
-        part += vals[e];
-      if (cols[e] < 0) {  // last entry of its group
-        sum += part;
-        part = 0.0f;
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(mem);            // [nu + 1]
+    volatile int32_t* lev =
+        reinterpret_cast<volatile int32_t*>(cnt + nu + 1);       // [nu]
+    uint16_t* order =
+        reinterpret_cast<uint16_t*>(cnt + 2 * nu + 1);           // [nu]
+    auto unit_of = [&](int t) { return cut ? (int)uid[t] : t >> 2; };
+    if (tid == 0) max_level = 0;
+    for (int u = tid; u < nu; u += blockDim.x) lev[u] = 0;
+    for (int u = tid; u <= nu; u += blockDim.x) cnt[u] = 0u;
+    __syncthreads();
+    for (int u0 = 0; u0 < nu; u0 += blockDim.x) {
+      const int u = u0 + tid;
+      int tb = 0, te = 0;
+      if (u < nu) {
+        tb = cut ? (int)first[u] : 4 * u;
+        te = cut ? (int)first[u + 1] : (4 * u + 4 < n ? 4 * u + 4 : n);
+      }
+      for (;;) {
+        bool up = false;
+        int m = 0;
+        for (int t = tb; t < te; ++t) {
+          int64_t e, e1;
+          for (entries(spin_at(t), e, e1); e < e1; ++e) {
+            const int uc = unit_of(pos_of(column(e)));
+            if (uc < u) {
+              m = max(m, lev[uc] + 1);
+            } else if (uc > u && lev[uc] <= lev[u]) {
+              // a later unit may flip a spin that this one reads: the rows
+              // name it also where the other row lacks the entry
+              atomicMax(const_cast<int32_t*>(lev) + uc, lev[u] + 1);
+              up = true;
+            }
+          }
+        }
+        if (u < nu && m > lev[u]) {
+          atomicMax(const_cast<int32_t*>(lev) + u, m);
+          up = true;
+        }
+        if (!__syncthreads_or(up)) break;
       }
     }
-    return sum;
+    for (int u = tid; u < nu; u += blockDim.x) {
+      atomicAdd(&cnt[lev[u] + 1], 1u);
+      atomicMax(&max_level, lev[u]);
+    }
+    __syncthreads();
+    const int nl = max_level + 1;
+    // the quads' schedule is already written when a cut one is tried
+    const bool keep = !cut || (3 * nl < 2 * best_nl && nu + nl + 4 <= n);
+    if (!keep) return;  // uniform
+    best_nl = nl;
+    if (tid < 32) {
+      // cnt[l] = first place of level l; cnt[nl] = nu
+      uint32_t carry = 0u;
+      for (int l0 = 0; l0 <= nl; l0 += 32) {
+        uint32_t v = l0 + lane <= nl ? cnt[l0 + lane] : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t up = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += up;
+        }
+        v += carry;
+        if (l0 + lane <= nl) cnt[l0 + lane] = v;
+        carry = __shfl_sync(0xffffffffu, v, 31);
+      }
+    }
+    __syncthreads();
+    auto put_high = [&](int k, uint32_t v) {
+      row[k] = (row[k] & 0xFFFF) | (int32_t)(v << 16);
+    };
+    for (int l = tid; l <= nl; l += blockDim.x) put_high(nu + l, cnt[l]);
+    __syncthreads();
+    if (tid < 32) {
+      for (int u0 = 0; u0 < nu; u0 += 32) {
+        const int u = u0 + lane;
+        const uint32_t l = u < nu ? (uint32_t)lev[u] : 0xFFFFFFFFu;
+        const uint32_t same = __match_any_sync(0xffffffffu, l);
+        const uint32_t base = u < nu ? cnt[l] : 0u;
+        __syncwarp();
+        if (u < nu) {
+          order[base + __popc(same & ((1u << lane) - 1u))] = (uint16_t)u;
+          if ((same >> lane) == 1u) cnt[l] = base + __popc(same);
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    for (int k = tid; k < nu; k += blockDim.x) {
+      const int u = order[k];
+      uint32_t code = (uint32_t)u;
+      if (cut) {
+        const uint32_t t = first[u], len = first[u + 1] - t;
+        code = ((t >> 2) << 4) | ((t & 3u) << 2) | (len - 1u);
+      }
+      put_high(k, code);
+    }
+    if (tid == 0) {
+      put_high(n - 3, any_order ? 1u : 0u);
+      put_high(n - 2, (uint32_t)nu);
+      put_high(n - 1, (uint32_t)nl);
+    }
+    if (n > kSchedCutN || nq >= 8 * nl) return;  // wide enough (uniform)
+    __syncthreads();
   }
+}
+
+// ------------------------------------------------------------------ sweep
+// A quad's four records in the warp's shared memory, each
+//   [D entries][D values][h_i][own][pad],
+// an entry being the byte offset of its column's spin word (bit 31: end of a
+// group, left out when the sums are exact in any order), own that of the
+// visited spin.
+template <int D>
+struct QuadSlab {
+  static constexpr int STRIDE = 2 * D + 4;  // words per record
+  static constexpr int QUAD = 4 * STRIDE;   // words per buffer
+  // 16-byte pieces of columns and values per record, and per lane and quad
+  static constexpr int PIECES = D / 2;
+  static constexpr int PER_LANE = (4 * PIECES + 31) / 32;
 };
 
-template <bool RANDOM, int D>
-__global__ void __launch_bounds__(kCsrChains) k_sweep_csr(const CsrArgs a) {
-  const int CH = blockDim.x;  // chains per CTA = the spin words' stride
-  extern __shared__ __align__(16) uint32_t smem_u[];
+// Philox4x32-10 with the ten round keys in kernel parameters (constant
+// operands of the rounds' logic instructions): draws 4 q .. 4 q + 3 of the
+// sweep stream of chain `b`.
+__device__ __forceinline__ void draw4_keys(const CsrArgs& a, uint32_t inst,
+                                           uint32_t sweep, uint32_t b,
+                                           uint32_t q, uint32_t out[4]) {
+  uint32_t c0 = q, c1 = sweep, c2 = b, c3 = (inst << 4) | TAG_SWEEP;
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c0;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
+    c0 = (uint32_t)(p1 >> 32) ^ c1 ^ a.round_keys[2 * r];
+    c1 = (uint32_t)p1;
+    c2 = (uint32_t)(p0 >> 32) ^ c3 ^ a.round_keys[2 * r + 1];
+    c3 = (uint32_t)p0;
+  }
+  out[0] = c0;
+  out[1] = c1;
+  out[2] = c2;
+  out[3] = c3;
+}
+
+// 32 x 32 bit transpose over a warp: lane l's bit b becomes lane b's bit l.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t v, int lane) {
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t m = s == 16  ? 0x0000FFFFu
+                       : s == 8 ? 0x00FF00FFu
+                       : s == 4 ? 0x0F0F0F0Fu
+                       : s == 2 ? 0x33333333u
+                                : 0x55555555u;
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, v, s);
+    v = (lane & s) ? ((o >> s) & m) | (v & ~m) : (v & m) | ((o << s) & ~m);
+  }
+  return v;
+}
+
+// log2 of a uniform (x + 1/2) 2^-32, approximate: never subnormal, so the
+// flush-to-zero form is the same function.
+__device__ __forceinline__ float log2_uniform(uint32_t x) {
+  float l;
+  asm("lg2.approx.ftz.f32 %0, %1;"
+      : "=f"(l)
+      : "f"(__uint2float_rn(x) * 0x1p-32f + 0x1p-33f));
+  return l;
+}
+
+template <bool RANDOM, bool ISING, int D>
+__global__ void __launch_bounds__(32 * kCsrWarps, 1)
+    k_sweep_csr(const CsrArgs a) {
+  using Q = QuadSlab<D>;
+  extern __shared__ __align__(128) uint32_t smem_u[];
   const SweepItem item = a.items[blockIdx.x];
   const int inst = item.inst;
-  const int n = a.p.n[inst];
+  const int n = a.p.n[inst], nq = csr_quads(n);
   const int words = (n + 31) >> 5;
-  uint32_t* spin_s = smem_u;  // [words][CH]
-  float* slab = reinterpret_cast<float*>(smem_u + words * CH);  // RecSlab<D>
-  int32_t* perm_s =
-      reinterpret_cast<int32_t*>(smem_u + words * CH + RecSlab<D>::BYTES / 4);
-  __shared__ uint8_t imp_s[kCsrChains];
-  const int tid = threadIdx.x;
-  const bool valid = tid < item.nchains;
-  const int64_t chain = item.chain0 + tid;
-  const bool ising = a.p.problem_type == PYSA_GB_ISING;
+  const int W = blockDim.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t* spin_s = smem_u;                                  // [32 words]
+  uint32_t* slab = smem_u + words * 32 + warp * 2 * Q::QUAD;  // [W][2][QUAD]
+  float2* de_s = reinterpret_cast<float2*>(
+      smem_u + words * 32 + W * 2 * Q::QUAD);                 // [W][32]
+  uint16_t* sched = reinterpret_cast<uint16_t*>(de_s + W * 32);  // [cap]
+  uint16_t* perm_s = sched + sched_cap(n);                    // [n], random
+  __shared__ uint8_t imp_s[32];
+  const bool valid = lane < item.nchains;
+  const int64_t chain = item.chain0 + lane;
   const uint32_t sweep = (uint32_t)(*a.s.sweep_counter);
 
-  // spins in, coalesced over (chain, word)
-  for (int idx = tid; idx < CH * words; idx += blockDim.x) {
-    const int c = idx / words, w = idx - c * words;
-    spin_s[w * CH + c] =
-        c < item.nchains
-            ? a.s.spins[(item.chain0 + c) * (int64_t)a.p.words + w]
-            : 0u;
+  // spins in, each word's 32 spins x 32 chains transposed
+#pragma unroll 4
+  for (int w = warp; w < words; w += W)
+    spin_s[w * 32 + lane] = warp_transpose(
+        valid ? a.s.spins[chain * (int64_t)a.p.words + w] : 0u, lane);
+  const int32_t* row =
+      a.perm + ((int64_t)(RANDOM ? sweep % (uint32_t)a.perm_slots : 0u) *
+                    a.p.num_instances + inst) * (int64_t)a.p.max_n;
+  int nu = nq, nl = nq;
+  bool any_order = false;
+  if (a.perm && n >= kSchedMinN) {
+    any_order = ((uint32_t)row[n - 3] >> 16) != 0u;
+    nu = (int)((uint32_t)row[n - 2] >> 16);
+    nl = (int)((uint32_t)row[n - 1] >> 16);
+#pragma unroll 2
+    for (int k = tid; k <= nu + nl; k += blockDim.x)
+      sched[k] = (uint16_t)((uint32_t)row[k] >> 16);
+  } else {  // every quad a level of its own
+    for (int k = tid; k <= 2 * nq; k += blockDim.x)
+      sched[k] = (uint16_t)(k < nq ? k : k - nq);
   }
-  if (RANDOM) {
-    const int32_t* perm_g =
-        a.perm + ((int64_t)(sweep % (uint32_t)a.perm_slots) *
-                      a.p.num_instances + inst) * (int64_t)a.p.max_n;
-    for (int t = tid; t < n; t += blockDim.x) perm_s[t] = perm_g[t];
-  }
+  const bool cut = nu != nq;  // units are parts of quads
+  if (RANDOM)
+    for (int t = tid; t < n; t += blockDim.x)
+      perm_s[t] = (uint16_t)(row[t] & 0xFFFF);
   __syncthreads();
 
   const float beta = valid ? a.s.chain_beta[chain] : 0.0f;
   const uint32_t cl = (uint32_t)(chain - a.p.chain_off[inst]);
-  const uint64_t seed_c =
-      valid ? chain_seed(a.seed, a.s.stream_key, chain) : a.seed;
   const int32_t* rows =
       D > 0 ? nullptr : a.p.csr_rows + a.p.csr_row_off[inst] * 9;
   const int32_t* colp = a.p.csr_col + a.p.csr_ent_off[inst];
   const float* valp = a.p.csr_val + a.p.csr_ent_off[inst];
   const float* h = a.p.h + a.p.h_off[inst];
-  uint32_t* my = spin_s + tid;
-  double dE = 0.0;
+  // Decisions in field units: with x = +-field signed so that dn = scale x, a
+  // flip is accepted when x >= th and rejected when x < tl; th and tl bracket
+  // log(u) / (beta scale) by a band of the f32 logarithm, 3e-5 +
+  // 1e-6 |log u| (over three times its error and the thresholds' roundings),
+  // and in between the exact rule decides.  log u < 0, so both are linear in
+  // log2 u: tl = tl1 log2 u + tl0, th = min(th1 log2 u + th0, 0).  beta <= 0
+  // accepts every finite x; a beta too small to invert, or NaN, leaves every
+  // x < 0 to the exact rule.
+  constexpr float kScale = ISING ? 2.0f : 1.0f;
+  constexpr float kLn2 = 0.69314718056f;
+  const bool plain_beta = beta >= 1e-30f;
+  const float invb = 1.0f / (beta * kScale);
+  const float tl1 = plain_beta ? kLn2 * 1.000001f * invb : 0.0f;
+  const float tl0 = plain_beta ? -3e-5f * invb : -INFINITY;
+  const float th1 = plain_beta ? kLn2 * 0.999999f * invb : 0.0f;
+  const float th0 = plain_beta ? 3e-5f * invb
+                    : beta <= 0.0f ? -3.4028234e38f : 0.0f;
+  // energy change in field units: an exact f32 pair, no f64 in the loop
+  float2 dE = make_float2(0.0f, 0.0f);
 
-  // rows of visiting positions 32 b .. 32 b + 31 into slab buffer b & 1
-  auto stage = [&](int b) {
+  auto spin_at = [&](int t) { return RANDOM ? (int)perm_s[t] : t; };
+  // records of quad q: 16-byte pieces and h into registers ...
+  uint4 rg[Q::PER_LANE > 0 ? Q::PER_LANE : 1];
+  float rh = 0.0f;
+  // the lane's first piece: record pr, columns 4 pk ... or values past them
+  const int pr = D > 0 ? lane / (D > 0 ? Q::PIECES : 1) : 0;
+  const int pk = D > 0 ? lane % (D > 0 ? Q::PIECES : 1) : 0;
+  const bool pcol = 4 * pk < D;
+  const uint4* psrc = reinterpret_cast<const uint4*>(
+      pcol ? (const void*)(colp + 4 * pk) : (const void*)(valp + 4 * pk - D));
+  constexpr int REC_STEP = D > 0 ? 32 / (Q::PIECES > 0 ? Q::PIECES : 1) : 1;
+  auto fetch = [&](int q) {
     if constexpr (D > 0) {
-      const int t = 32 * b + tid;
-      if (tid < 32 && t < n) {
-        const int i = RANDOM ? perm_s[t] : t;
-        float* dst = slab + ((b & 1) * 32 + tid) * RecSlab<D>::STRIDE;
 #pragma unroll
-        for (int q = 0; q < D / 4; ++q) {
-          cp_async16(dst + 4 * q, colp + (int64_t)i * D + 4 * q);
-          cp_async16(dst + D + 4 * q, valp + (int64_t)i * D + 4 * q);
-        }
-        cp_async4(dst + 2 * D, h + i);
+      for (int e = 0; e < Q::PER_LANE; ++e) {
+        const int r = pr + e * REC_STEP, t = 4 * q + r;
+        if (r < 4 && t < n) rg[e] = __ldg(psrc + spin_at(t) * (D / 4));
       }
-      cp_async_commit();
+      if (lane < 4 && 4 * q + lane < n) rh = __ldg(h + spin_at(4 * q + lane));
     }
   };
-  stage(0);
-  if constexpr (D > 0) {
-    cp_async_wait_all();
-    __syncthreads();
-  }
-  const int nb = (n + 31) >> 5;
-  for (int b = 0; b < nb; ++b) {
-    if (b + 1 < nb) stage(b + 1);
-    for (int t0 = 32 * b; t0 < n && t0 < 32 * b + 32; t0 += 4) {
-      uint32_t rnd[4];
-      draw4(seed_c, TAG_SWEEP, (uint32_t)inst, sweep, cl,
-            (uint32_t)(t0 >> 2), rnd);
-      // short records: all four up front, ahead of the flips' shared
-      // stores; long ones one at a time (registers)
-      constexpr bool kHoist = D > 0 && D <= 8;
-      Rec<(D > 0 ? D : 4)> recs[kHoist ? 4 : 1];
-      if constexpr (kHoist) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          recs[q].load(slab + ((b & 1) * 32 + ((t0 + q) & 31)) *
-                                  RecSlab<D>::STRIDE);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int t = t0 + q;
-        if (t >= n) break;
-        const int i = RANDOM ? perm_s[t] : t;
-        float sum = 0.0f, hi;
-        if constexpr (D > 0) {
-          auto& r = recs[kHoist ? q : 0];
-          if constexpr (!kHoist)
-            r.load(slab + ((b & 1) * 32 + (t & 31)) * RecSlab<D>::STRIDE);
-          sum = r.dot(my, CH, ising);
-          hi = r.h;
-        } else {
-          const int32_t* r9 = rows + (int64_t)i * 9;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            float part = 0.0f;
-            const int e1 = __ldg(r9 + k + 1);
-            for (int e = __ldg(r9 + k); e < e1; ++e) {
-              const int col = __ldg(colp + e);
-              const float v = __ldg(valp + e);
-              const bool bit = (my[(col >> 5) * CH] >> (col & 31)) & 1u;
-              if (ising)
-                part += bit ? v : -v;
-              else if (bit)
-                part += v;
-            }
-            sum += part;
-          }
-          hi = __ldg(h + i);
-        }
-        const float field = sum + hi;
-        const uint32_t wi = my[(i >> 5) * CH];
-        const bool sbit = (wi >> (i & 31)) & 1u;
-        const float dn = ising ? (sbit ? 2.0f * field : -2.0f * field)
-                               : (sbit ? field : -field);
-        if (valid && metropolis_accept(dn, beta, rnd[q])) {
-          my[(i >> 5) * CH] = wi ^ (1u << (i & 31));
-          dE -= (double)dn;  // the sweep's energy change, summed in f64
-        }
-      }
-    }
+  // ... and from there into slab buffer b: columns become byte offsets of
+  // spin words (times 4; bit 31 kept unless the sums need no groups)
+  const uint32_t mul = pcol ? 4u : 1u;
+  const uint32_t keep = pcol && !any_order ? 0x80000000u : 0u;
+  auto put = [&](int q, int b) {
     if constexpr (D > 0) {
-      cp_async_wait_all();
-      __syncthreads();  // buffer b & 1 free, b + 1 landed
+      uint32_t* s = slab + b * Q::QUAD;
+#pragma unroll
+      for (int e = 0; e < Q::PER_LANE; ++e) {
+        const int r = pr + e * REC_STEP;
+        uint4 v = rg[e];
+        v.x = v.x * mul | (v.x & keep);
+        v.y = v.y * mul | (v.y & keep);
+        v.z = v.z * mul | (v.z & keep);
+        v.w = v.w * mul | (v.w & keep);
+        if (r < 4)
+          *reinterpret_cast<uint4*>(s + r * Q::STRIDE + 4 * pk) = v;
+      }
+      if (lane < 4)
+        *reinterpret_cast<uint2*>(s + lane * Q::STRIDE + 2 * D) = make_uint2(
+            __float_as_uint(rh),
+            4 * q + lane < n ? 4u * (uint32_t)spin_at(4 * q + lane) : 0u);
+      __syncwarp();
     }
+  };
+  float tl[4], th[4];
+  auto thresholds = [&](int q) {
+    uint32_t x[4];
+    if (a.s.stream_key)
+      draw4(chain_seed(a.seed, valid ? a.s.stream_key : nullptr, chain),
+            TAG_SWEEP, (uint32_t)inst, sweep, cl, (uint32_t)q, x);
+    else
+      draw4_keys(a, (uint32_t)inst, sweep, cl, (uint32_t)q, x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float l2 = log2_uniform(x[k]);
+      tl[k] = fmaf(tl1, l2, tl0);
+      th[k] = fminf(fmaf(th1, l2, th0), 0.0f);
+    }
+  };
+  auto word_at = [&](uint32_t off) {
+    return reinterpret_cast<uint32_t*>(
+        reinterpret_cast<unsigned char*>(spin_s) + off);
+  };
+  // a product by a lane constant (the multiply-add pipe; the logic pipe, at
+  // half its rate, is the busier one) brings this lane's spin to the sign bit
+  const uint32_t to_sign = 0x80000000u >> lane;
+  // value of an entry with its spin's sign (Ising), or masked by the spin
+  // (QUBO: adding +0 changes no partial sum)
+  auto signed_value = [&](uint32_t off, float v) {
+    const uint32_t s = *word_at(off) * to_sign;
+    return __uint_as_float(ISING
+                               ? __float_as_uint(v) ^ (~s & 0x80000000u)
+                               : __float_as_uint(v) &
+                                     (uint32_t)((int32_t)s >> 31));
+  };
+  // decides position k of a quad, field f, spin at byte offset `own`.  The
+  // fast rule only notes a decision inside the band (`ask`); EXACT decides
+  // such a one with the exact rule.
+  bool ask = false;
+  auto attempt = [&](auto exact_t, int q, int k, float tlk, float thk,
+                     uint32_t own, float f) {
+    uint32_t* wp = word_at(own);
+    const uint32_t w = *wp;
+    const float x = __uint_as_float(__float_as_uint(f) ^
+                                    (~(w * to_sign) & 0x80000000u));
+    bool acc = x >= thk && valid;
+    const bool in = valid && !(x >= thk) && !(x < tlk);
+    if constexpr (decltype(exact_t)::value) {
+      if (in)
+        acc = accept_slow_redraw(
+            kScale * x, beta, chain_seed(a.seed, a.s.stream_key, chain),
+            (uint32_t)inst, sweep, cl, (uint32_t)(4 * q + k));
+      __syncwarp();
+    } else {
+      ask = ask || in;
+    }
+    const uint32_t flips = __ballot_sync(0xffffffffu, acc);
+    if (lane == 0) *wp = w ^ flips;
+    const float y = acc ? x : 0.0f;
+    const float t1 = dE.x - y;
+    const float bb = t1 - dE.x;
+    dE.y += (dE.x - (t1 - bb)) - (y + bb);
+    dE.x = t1;
+    __syncwarp();  // the flips seen by every lane
+    return w;
+  };
+  // position k of quad q, records in slab buffer b; returns the spin word
+  // before it
+  auto decide = [&](auto any_order_t, auto exact_t, int q, int b, int k,
+                    float tlk, float thk) {
+    if constexpr (D > 0) {
+      const uint32_t* rec = slab + b * Q::QUAD + k * Q::STRIDE;
+      float sum = 0.0f, part = 0.0f;
+#pragma unroll
+      for (int e4 = 0; e4 < D / 4; ++e4) {
+        const uint4 c4 = reinterpret_cast<const uint4*>(rec)[e4];
+        const float4 v4 = reinterpret_cast<const float4*>(rec + D)[e4];
+        const uint32_t cs[4] = {c4.x, c4.y, c4.z, c4.w};
+        const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if constexpr (decltype(any_order_t)::value) {
+            sum += signed_value(cs[e], vs[e]);
+          } else {
+            part += signed_value(cs[e] & 0x7fffffffu, vs[e]);
+            const bool last = (int32_t)cs[e] < 0;  // end of its group
+            sum = last ? sum + part : sum;
+            part = last ? 0.0f : part;
+          }
+        }
+      }
+      const uint2 ho = *reinterpret_cast<const uint2*>(rec + 2 * D);
+      return attempt(exact_t, q, k, tlk, thk, ho.y,
+                     sum + __uint_as_float(ho.x));
+    } else {
+      const int i = spin_at(4 * q + k);
+      const int32_t* r9 = rows + (int64_t)i * 9;
+      float sum = 0.0f;
+#pragma unroll
+      for (int g = 0; g < 8; ++g) {
+        float part = 0.0f;
+        const int e1 = __ldg(r9 + g + 1);
+        for (int e = __ldg(r9 + g); e < e1; ++e)
+          part += signed_value(4u * (uint32_t)__ldg(colp + e),
+                               __ldg(valp + e));
+        sum += part;
+      }
+      return attempt(exact_t, q, k, tlk, thk, 4u * (uint32_t)i,
+                     sum + __ldg(h + i));
+    }
+  };
+  auto pick = [&](const float (&v)[4], int k) {
+    return k < 2 ? (k ? v[1] : v[0]) : (k == 2 ? v[2] : v[3]);
+  };
+
+  // Two groups of warps take the levels in turn: while one decides a level,
+  // the other fetches and draws for the next.  This warp's units: places
+  // first(l) + its number in the group, + the group's size, ... of every
+  // other level.
+  const int WG = W >> 1, wi = warp % WG;
+  const int qshift = cut ? 4 : 0;
+  const uint16_t* first = sched + nu;
+  auto sweep_all = [&](auto any_order_t) {
+    int l = warp / WG - 2, place = 0, end = 0;
+    // on to this warp's next unit
+    auto settle = [&]() {
+      place += WG;
+      while (place >= end) {
+        l += 2;
+        if (l >= nl) return;
+        place = (int)first[l] + wi;
+        end = (int)first[l + 1];
+      }
+    };
+    settle();
+    int unit = 0, b = 0;
+    if (l < nl) {
+      unit = sched[place];
+      fetch(unit >> qshift);
+      thresholds(unit >> qshift);
+      put(unit >> qshift, 0);
+    }
+    int done = 0;  // barriers passed: one before every level but the first
+    while (l < nl) {
+      const int lv = l, u = unit, q = u >> qshift;
+      settle();
+      if (l < nl) {
+        unit = sched[place];
+        fetch(unit >> qshift);
+      }
+      for (; done < lv; ++done) __syncthreads();
+      int k0 = cut ? (u >> 2) & 3 : 0;
+      const int left = n - 4 * q;
+      const int k1 = cut ? k0 + (u & 3) + 1 : left < 4 ? left : 4;
+      if (k1 - k0 == 4) {
+        // the fast rule for all four; where a lane's decision needed the
+        // exact one, the quad is undone and decided again below
+        const float2 dE0 = dE;
+        uint32_t w0[4];
+        ask = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          w0[k] = decide(any_order_t, std::false_type{}, q, b, k, tl[k],
+                         th[k]);
+        if (!__any_sync(0xffffffffu, ask)) {
+          k0 = k1;
+        } else {
+          if (lane == 0) {
+#pragma unroll
+            for (int k = 3; k >= 0; --k) spin_s[spin_at(4 * q + k)] = w0[k];
+          }
+          __syncwarp();
+          dE = dE0;
+        }
+      }
+#pragma unroll 1
+      for (int k = k0; k < k1; ++k)
+        decide(any_order_t, std::true_type{}, q, b, k, pick(tl, k),
+               pick(th, k));
+      if (l != lv && lv + 1 < nl) {  // this warp is through with the level
+        ++done;
+        __syncthreads();
+      }
+      b ^= 1;
+      if (l < nl) {
+        thresholds(unit >> qshift);
+        put(unit >> qshift, b);
+      }
+    }
+    for (; done < nl; ++done) __syncthreads();
+  };
+  if constexpr (D > 0) {
+    if (any_order)
+      sweep_all(std::true_type{});
+    else
+      sweep_all(std::false_type{});
+  } else {
+    sweep_all(std::false_type{});
   }
 
   // energies and the per-chain best (strict <, pysa/simulation.py:150-171)
-  bool improved = false;
-  if (valid) {
-    const float e_new = (float)((double)a.s.energies[chain] + dE);
-    a.s.energies[chain] = e_new;
-    if (e_new < a.s.best_energy[chain]) {
-      improved = true;
-      a.s.best_energy[chain] = e_new;
-      a.s.best_sweep[chain] = (int32_t)sweep;
-    }
-  }
-  imp_s[tid] = improved ? 1 : 0;
+  de_s[warp * 32 + lane] = dE;
   __syncthreads();
-  for (int idx = tid; idx < item.nchains * words; idx += blockDim.x) {
-    const int c = idx / words, w = idx - c * words;
-    const uint32_t v = spin_s[w * CH + c];
-    const int64_t off = (item.chain0 + c) * (int64_t)a.p.words + w;
-    a.s.spins[off] = v;
-    if (imp_s[c]) a.s.best_spins[off] = v;
+  if (warp == 0) {
+    bool improved = false;
+    if (valid) {
+      double d = 0.0;
+      for (int w = 0; w < W; ++w) {
+        const float2 v = de_s[w * 32 + lane];
+        d += fabsf(v.x) < INFINITY ? (double)v.x + (double)v.y : (double)v.x;
+      }
+      const float e_new =
+          (float)((double)a.s.energies[chain] + (double)kScale * d);
+      a.s.energies[chain] = e_new;
+      if (e_new < a.s.best_energy[chain]) {
+        improved = true;
+        a.s.best_energy[chain] = e_new;
+        a.s.best_sweep[chain] = (int32_t)sweep;
+      }
+    }
+    imp_s[lane] = improved ? 1 : 0;
+  }
+  __syncthreads();
+  const bool keep_best = imp_s[lane] != 0;
+#pragma unroll 4
+  for (int w = warp; w < words; w += W) {
+    const uint32_t v = warp_transpose(spin_s[w * 32 + lane], lane);
+    const int64_t off = chain * (int64_t)a.p.words + w;
+    if (valid) {
+      a.s.spins[off] = v;
+      if (keep_best) a.s.best_spins[off] = v;
+    }
   }
 }
 
-template <bool RANDOM, int D>
-static cudaError_t launch_csr_t(const CsrArgs& a, size_t base,
-                                cudaStream_t st) {
-  const size_t smem = base + RecSlab<D>::BYTES;
+template <bool RANDOM, bool ISING, int D>
+static cudaError_t launch_csr_t(const CsrArgs& a, cudaStream_t st) {
+  const int n = a.p.max_n;
+  // a level holds a few to a few dozen units, more of them the wider the
+  // instance; two groups of warps share the levels
+  int W = n <= 512 ? 8 : n <= 2048 ? 16 : kCsrWarps;
+  auto bytes = [&](int w) {
+    return (size_t)((n + 31) / 32) * 128 +
+           (size_t)w * (2 * QuadSlab<D>::QUAD * 4 + 256) +
+           2 * (size_t)sched_cap(n) + (RANDOM ? 2 * (size_t)n : 0);
+  };
+  while (W > 2 && bytes(W) > 232448 - 256) W /= 2;
+  const size_t smem = bytes(W);
   cudaError_t e = cudaFuncSetAttribute(
-      k_sweep_csr<RANDOM, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      k_sweep_csr<RANDOM, ISING, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
       (int)smem);
   if (e != cudaSuccess) return e;
-  k_sweep_csr<RANDOM, D><<<a.num_items, a.chains, smem, st>>>(a);
+  k_sweep_csr<RANDOM, ISING, D><<<a.num_items, 32 * W, smem, st>>>(a);
   return cudaGetLastError();
 }
 
-template <bool RANDOM>
-static cudaError_t launch_csr_w(const CsrArgs& a, size_t smem,
-                                cudaStream_t st) {
+template <bool RANDOM, bool ISING>
+static cudaError_t launch_csr_w(const CsrArgs& a, cudaStream_t st) {
   switch (a.width) {
-    case 4: return launch_csr_t<RANDOM, 4>(a, smem, st);
-    case 8: return launch_csr_t<RANDOM, 8>(a, smem, st);
-    case 16: return launch_csr_t<RANDOM, 16>(a, smem, st);
-    case 32: return launch_csr_t<RANDOM, 32>(a, smem, st);
-    default: return launch_csr_t<RANDOM, 0>(a, smem, st);
+    case 4: return launch_csr_t<RANDOM, ISING, 4>(a, st);
+    case 8: return launch_csr_t<RANDOM, ISING, 8>(a, st);
+    case 16: return launch_csr_t<RANDOM, ISING, 16>(a, st);
+    case 32: return launch_csr_t<RANDOM, ISING, 32>(a, st);
+    default: return launch_csr_t<RANDOM, ISING, 0>(a, st);
   }
+}
+
+cudaError_t launch_csr_schedule(const CsrArgs& a, bool random,
+                                cudaStream_t st) {
+  if (a.num_items <= 0 || !a.perm) return cudaSuccess;
+  // the larger of all quads and, up to kSchedCutN, as many units as spins
+  const int n = a.p.max_n, nc = n < kSchedCutN ? n : kSchedCutN;
+  const size_t whole = sched_bytes(csr_quads(n), n, random, false);
+  const size_t parts = sched_bytes(nc, nc, random, true);
+  const size_t smem = (whole > parts ? whole : parts) + 16;
+  const void* f = random ? (const void*)k_csr_schedule<true>
+                         : (const void*)k_csr_schedule<false>;
+  cudaError_t e = cudaFuncSetAttribute(
+      f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if (random)
+    k_csr_schedule<true><<<a.p.num_instances, kSchedThreads, smem, st>>>(a);
+  else
+    k_csr_schedule<false><<<a.p.num_instances, kSchedThreads, smem, st>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_csr(const CsrArgs& a, bool random, cudaStream_t st) {
   if (a.num_items <= 0) return cudaSuccess;
-  const int words = (a.p.max_n + 31) / 32;
-  const size_t base = (size_t)words * a.chains * 4 +
-                      (random ? (size_t)a.p.max_n * 4 : 0);
-  return random ? launch_csr_w<true>(a, base, st)
-                : launch_csr_w<false>(a, base, st);
+  const bool ising = a.p.problem_type == PYSA_GB_ISING;
+  if (random)
+    return ising ? launch_csr_w<true, true>(a, st)
+                 : launch_csr_w<true, false>(a, st);
+  return ising ? launch_csr_w<false, true>(a, st)
+               : launch_csr_w<false, false>(a, st);
 }
 
 }  // namespace pysa_gb
