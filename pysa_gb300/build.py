@@ -25,7 +25,7 @@ if os.environ.get("PYSA_GB_TRACE") == "1":  # timeline stamps (diagnostics)
 
 SOURCES = ["abi.cu", "kernels_aux.cu", "plain_small.cu", "plain_large.cu",
            "ais.cu", "sweep_tc.cu", "sweep_tc_e8.cu", "sweep_csr.cu",
-           "sweep_wide.cu", "noalloc.cu",
+           "sweep_wide.cu", "sweep_small.cu", "noalloc.cu",
            "gemm_tc.cu", "mlp.cu"]
 
 

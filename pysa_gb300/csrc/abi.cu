@@ -8,6 +8,7 @@
 
 #include "ais_api.h"
 #include "csr_api.h"
+#include "small_api.h"
 #include "tc_api.h"
 #include "wide_api.h"
 #include "aux.cuh"
@@ -72,6 +73,10 @@ static int cuda_fail(cudaError_t e, const char* where) {
 
 // Default for the most sweeps one fused tensor-core launch covers.
 constexpr int kMaxFusedSweeps = 128;
+
+// Most sweeps of one launch of the resident small sweep (about a
+// millisecond each thousand).
+constexpr int kMaxSmallSweeps = 4096;
 
 // Streaming multiprocessors of the current device (cached per device).
 static inline bool is_sparse(const pysa_gb_host_tables* h, int i) {
@@ -666,6 +671,8 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
   ta.recompute_every = o->recompute_every;
   ta.use_pt = o->use_pt;
   ta.exchange_every = o->exchange_every;
+  ta.log_omega_stride = 0;  // fused launches only
+  ta.pad_ = 0;
   ta.unit_wait_ns = g_unit_wait_ns;
   ta.decision_mode = g_decision_mode;
   ta.round_limit = g_round_limit;
@@ -685,8 +692,15 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
                       : sm_count();
   const int folds[3] = {1, 2, 4};
   int last_v = -1;
-  for (int v = 0; v < 3; ++v)
+  for (int v = 0; use_tc && v < 3; ++v)
     if (ws->tc_variant_count[v] > 0) last_v = v;
+  // dense instances left to the CUDA cores: the smallest (the variants of n
+  // <= 64) sweep resident on an SM, any number of sweeps per launch
+  bool small_live = false, wider_live = false;
+  for (int v = 0; v < kNumPlainVariants; ++v)
+    if (ws->variant_count[v] > 0 && ((plain_mask >> v) & 1))
+      (32 * plain_variant(v).nc <= kSmallMaxN ? small_live : wider_live) =
+          true;
   // Fused launches over items of one size split the launch's item-sweeps
   // evenly over the CTAs (wrap-around units) unless the caller fixed the
   // unit length.
@@ -710,19 +724,21 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       ta.unit_sweeps = ta.wrap ? ku * units : ku;
       ta.units_per_item = ta.wrap ? 1 : units;
       ta.fuse_exchange = fuse;
-      ta.advance_counter = fuse && v == last_v;
+      ta.advance_counter = fuse && v == last_v && !small_live;
+      ta.log_omega_stride = fuse ? o->log_omega_stride : 0;
       e = launch_tc(ta, folds[v], random, sms, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc sweep launch");
     }
     return PYSA_GB_OK;
   };
-  // Fused: every instance on the tensor cores, exchange inside the kernel
-  // (or none), no log-omega; several sweeps per launch with the fields
-  // resident in tensor memory.
-  const bool fused = use_tc && phases == 3 && ws->plain_live == 0 &&
-                     ws->csr_item_count == 0 && ws->wide_item_count == 0 &&
-                     o->log_omega_stride == 0 &&
-                     (!o->use_pt || ws->tc_fusable) && ws->tc_sched;
+  // Fused: every instance either on the tensor cores with whole reads per
+  // CTA (or nothing to do between sweeps), or small enough to stay on an SM;
+  // exchange and log-omega inside the kernels, several sweeps per launch.
+  const bool between = o->use_pt || o->log_omega_stride > 0;
+  const bool fused = phases == 3 && !wider_live && ws->csr_item_count == 0 &&
+                     ws->wide_item_count == 0 && (last_v >= 0 || small_live) &&
+                     (last_v < 0 ||
+                      ((!between || ws->tc_fusable) && ws->tc_sched));
   // random order on the tensor cores: visiting orders of the next `cnt`
   // sweeps, and the tiles repacked in those orders
   auto rand_prepare = [&](int cnt) -> int {
@@ -737,7 +753,8 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
     const int ku_pref = ws->tc_unit_sweeps > 0 ? ws->tc_unit_sweeps : 8;
     int per_launch =
         ws->tc_launch_sweeps > 0 ? ws->tc_launch_sweeps : kMaxFusedSweeps;
-    if (random && per_launch > ws->tc_rand_slots)
+    if (last_v < 0) per_launch = kMaxSmallSweeps;
+    if (last_v >= 0 && random && per_launch > ws->tc_rand_slots)
       per_launch = ws->tc_rand_slots;
     // items of the largest fold: its launch sets the number of unit waves
     int items = 1;
@@ -749,17 +766,38 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
     int remaining = num_sweeps;
     while (remaining > 0) {
       int chunk = remaining < per_launch ? remaining : per_launch;
-      const int ku = ws->tc_unit_sweeps > 0
+      const int ku = last_v < 0 ? chunk
+                     : ws->tc_unit_sweeps > 0
                          ? (chunk < ku_pref ? chunk : ku_pref)
                      : all_wrap ? chunk
                                 : tc_unit_for(chunk, ku_pref, items, sms);
       chunk = chunk / ku * ku;
-      if (random) {
-        const int rc = rand_prepare(chunk);
+      if (last_v >= 0) {
+        if (random) {
+          const int rc = rand_prepare(chunk);
+          if (rc != PYSA_GB_OK) return rc;
+        }
+        const int rc = tc_launches(ku, chunk / ku, 1);
         if (rc != PYSA_GB_OK) return rc;
       }
-      const int rc = tc_launches(ku, chunk / ku, 1);
-      if (rc != PYSA_GB_OK) return rc;
+      if (small_live) {
+        SmallArgs sa;
+        sa.p = *p;
+        sa.s = *s;
+        sa.fields = ws->fields;
+        sa.field_ld = ws->field_ld;
+        sa.cap = 0;
+        sa.seed = o->seed;
+        sa.num_sweeps = chunk;
+        sa.use_pt = o->use_pt;
+        sa.exchange_every = o->exchange_every;
+        sa.log_omega_stride = o->log_omega_stride;
+        sa.advance = 1;
+        sa.pad_ = 0;
+        sa.skip_inst = a.skip_inst;
+        cudaError_t e = launch_small(sa, random, st);
+        if (e != cudaSuccess) return cuda_fail(e, "small sweep launch");
+      }
       remaining -= chunk;
     }
     return PYSA_GB_OK;

@@ -151,6 +151,42 @@ __device__ __forceinline__ bool metropolis_accept_lf(
   return accept_slow_redraw(dn, beta, seed, inst, sweep, chain, step);
 }
 
+// log2 of a uniform (x + 1/2) 2^-32, approximate: never subnormal, so the
+// flush-to-zero form is the same function.
+__device__ __forceinline__ float log2_uniform(uint32_t x) {
+  float l;
+  asm("lg2.approx.ftz.f32 %0, %1;"
+      : "=f"(l)
+      : "f"(__uint2float_rn(x) * 0x1p-32f + 0x1p-33f));
+  return l;
+}
+
+// Random thresholds of a chain's decisions in field units: with x = +-field
+// signed so that dn = scale x, a flip is accepted when x >= th and rejected
+// when x < tl; th and tl bracket log(u) / (beta scale) by a band of the f32
+// logarithm, 3e-5 + 1e-6 |log u| (over three times its error and the
+// thresholds' roundings), and in between the exact rule decides.  log u < 0,
+// so both are linear in log2 u: tl = tl1 log2 u + tl0, th = min(th1 log2 u +
+// th0, 0).  beta <= 0 accepts every finite x; a beta too small to invert, or
+// NaN, leaves every x < 0 to the exact rule.
+struct FieldThreshold {
+  float tl1, tl0, th1, th0;
+  __device__ __forceinline__ FieldThreshold(float beta, float scale) {
+    constexpr float kLn2 = 0.69314718056f;
+    const bool plain = beta >= 1e-30f;
+    const float inv = 1.0f / (beta * scale);
+    tl1 = plain ? kLn2 * 1.000001f * inv : 0.0f;
+    tl0 = plain ? -3e-5f * inv : -INFINITY;
+    th1 = plain ? kLn2 * 0.999999f * inv : 0.0f;
+    th0 = plain ? 3e-5f * inv : beta <= 0.0f ? -3.4028234e38f : 0.0f;
+  }
+  __device__ __forceinline__ void at(uint32_t x, float& tl, float& th) const {
+    const float l2 = log2_uniform(x);
+    tl = fmaf(tl1, l2, tl0);
+    th = fminf(fmaf(th1, l2, th0), 0.0f);
+  }
+};
+
 // Same rule on a precomputed f64 threshold (AIS form: full >= 0 accepts).
 __device__ __forceinline__ bool accept_full(double full, uint32_t x) {
   if (full >= 0.0) return true;

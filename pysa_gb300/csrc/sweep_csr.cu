@@ -338,16 +338,6 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t v, int lane) {
   return v;
 }
 
-// log2 of a uniform (x + 1/2) 2^-32, approximate: never subnormal, so the
-// flush-to-zero form is the same function.
-__device__ __forceinline__ float log2_uniform(uint32_t x) {
-  float l;
-  asm("lg2.approx.ftz.f32 %0, %1;"
-      : "=f"(l)
-      : "f"(__uint2float_rn(x) * 0x1p-32f + 0x1p-33f));
-  return l;
-}
-
 template <bool RANDOM, bool ISING, int D>
 __global__ void __launch_bounds__(32 * kCsrWarps, 1)
     k_sweep_csr(const CsrArgs a) {
@@ -404,23 +394,8 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
   const int32_t* colp = a.p.csr_col + a.p.csr_ent_off[inst];
   const float* valp = a.p.csr_val + a.p.csr_ent_off[inst];
   const float* h = a.p.h + a.p.h_off[inst];
-  // Decisions in field units: with x = +-field signed so that dn = scale x, a
-  // flip is accepted when x >= th and rejected when x < tl; th and tl bracket
-  // log(u) / (beta scale) by a band of the f32 logarithm, 3e-5 +
-  // 1e-6 |log u| (over three times its error and the thresholds' roundings),
-  // and in between the exact rule decides.  log u < 0, so both are linear in
-  // log2 u: tl = tl1 log2 u + tl0, th = min(th1 log2 u + th0, 0).  beta <= 0
-  // accepts every finite x; a beta too small to invert, or NaN, leaves every
-  // x < 0 to the exact rule.
   constexpr float kScale = ISING ? 2.0f : 1.0f;
-  constexpr float kLn2 = 0.69314718056f;
-  const bool plain_beta = beta >= 1e-30f;
-  const float invb = 1.0f / (beta * kScale);
-  const float tl1 = plain_beta ? kLn2 * 1.000001f * invb : 0.0f;
-  const float tl0 = plain_beta ? -3e-5f * invb : -INFINITY;
-  const float th1 = plain_beta ? kLn2 * 0.999999f * invb : 0.0f;
-  const float th0 = plain_beta ? 3e-5f * invb
-                    : beta <= 0.0f ? -3.4028234e38f : 0.0f;
+  const FieldThreshold ft(beta, kScale);
   // energy change in field units: an exact f32 pair, no f64 in the loop
   float2 dE = make_float2(0.0f, 0.0f);
 
@@ -479,11 +454,7 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
     else
       draw4_keys(a, (uint32_t)inst, sweep, cl, (uint32_t)q, x);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float l2 = log2_uniform(x[k]);
-      tl[k] = fmaf(tl1, l2, tl0);
-      th[k] = fminf(fmaf(th1, l2, th0), 0.0f);
-    }
+    for (int k = 0; k < 4; ++k) ft.at(x[k], tl[k], th[k]);
   };
   auto word_at = [&](uint32_t off) {
     return reinterpret_cast<uint32_t*>(

@@ -376,6 +376,36 @@ __device__ __noinline__ void redo_subblock(const RedoCtx& x, uint32_t* wcur,
   *dEb = e;
 }
 
+// Log-omega of an item's reads (pysa/ais.py:79-112), a warp per read: terms
+// of the sorted ladder from f32 products, summed in f64.  E: the chains'
+// energies.  Out of line: it runs only with get_part_fun, and inlined it
+// would slow every sweep.
+static __device__ __noinline__ void item_log_omega(const TcArgs& a,
+                                                   const TcItem& item,
+                                                   const float* E,
+                                                   uint32_t sweep) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int inst = item.inst, R = a.p.replicas[inst];
+  const float* betas = a.p.ladder + a.p.ladder_off[inst];
+  const int32_t* sorted = a.p.ladder_sorted + a.p.ladder_off[inst];
+  const int64_t read0 =
+      a.p.read_off[inst] + (item.chain0 - a.p.chain_off[inst]) / R;
+  for (int r = warp; r < item.nchains / R; r += 4) {
+    const int32_t* B = a.s.beta_idx + item.chain0 + (int64_t)r * R;
+    double lw = 0.0;
+    for (int k = 1 + lane; k < R; k += 32) {
+      const int hi = sorted[k];
+      const float b = betas[hi];
+      const float old = k > 1 ? betas[sorted[k - 1]] : 0.0f;
+      const float e = E[r * R + __ldcg(B + hi)];
+      lw += (double)__fsub_rn(__fmul_rn(-b, e), __fmul_rn(-old, e));
+    }
+    lw = warp_sum(lw);
+    if (lane == 0)
+      a.s.log_omega[(read0 + r) * a.log_omega_stride + sweep] = lw;
+  }
+}
+
 // Work units.  Fixed units (a.wrap == 0): unit u is item u % num_items for
 // sweeps (u / num_items) * unit_sweeps ... + unit_sweeps - 1 of the launch,
 // taken from a queue in order.  Wrap-around units (a.wrap == 1, items of one
@@ -1714,6 +1744,9 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             __syncwarp();
           }
         }
+        // (a warp reads back the slot maps that it wrote above itself)
+        if (a.log_omega_stride > 0 && !*sh.abort)
+          item_log_omega(a, item, ex_E, sweep);
         named_sync_128();
       }  // sweeps
 

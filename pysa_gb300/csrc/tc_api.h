@@ -34,6 +34,8 @@ struct TcArgs {
   int32_t use_pt;
   int32_t advance_counter;  // 1: the last CTA advances the sweep counter
   int32_t exchange_every;   // <= 1: every sweep; k: after (s + 1) % k == 0
+  int32_t log_omega_stride; // > 0: log-omega of every sweep (fused)
+  int32_t pad_;
   uint64_t unit_wait_ns;  // bound of the wait for an item's previous unit
                           // (0: one second)
   int32_t decision_mode;  // 0 per-block choice, 1 block rounds, 2 sub-blocks
