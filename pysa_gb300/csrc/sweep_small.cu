@@ -14,16 +14,21 @@
 // the first one not certainly rejected is the next decision (the ones before
 // it are rejected as the one-by-one rule rejects them, having seen every
 // earlier flip), and an accepted flip corrects all fields with one row of
-// couplings.  A sweep thus takes its accepted flips + 1 rounds of about 100
-// cycles instead of n dependent attempts.  Field updates, energy sums and
-// draws are those of the plain sweep kernel, bit for bit.
+// couplings.  A sweep thus takes its accepted flips + 1 rounds instead of n
+// dependent attempts; a chain whose last sweep flipped many spins takes the
+// positions in turn.  Field updates, energy sums and draws are those of the
+// plain sweep kernel, bit for bit.
 //
 // One more warp works ahead: the next sweep's visiting order and this
-// sweep's exchange draws.
+// sweep's exchange draws.  While the reads are fewer than the SMs, a cluster
+// of up to 8 CTAs shares a read's chains; energies and new betas cross
+// through distributed shared memory.
 //
-// Measured (times per sweep with exchange): n = 60, 640 chains, log-omega
-// 62 -> 3.3 us; n = 24, 4 chains, random order 20 -> 1.2 us (three launches
-// per sweep before).
+// Measured (times per sweep with exchange): n = 60, 640 chains in 20 reads,
+// log-omega 62 -> 8 us (22 on one CTA per read in rounds alone); n = 24, 4
+// chains, random order 25 -> 2.5 us (three launches per sweep before).
+#include <cooperative_groups.h>
+
 #include "aux.cuh"
 #include "small_api.h"
 
@@ -32,6 +37,11 @@ namespace pysa_gb {
 namespace {
 
 constexpr int kMaxSmallWarps = 31;  // chains at a time; one more works ahead
+// A chain is swept position by position after a sweep that flipped more than
+// one spin in kDenseFlips (a round of the other form costs about as much as
+// five positions), in rounds otherwise.
+constexpr int kDenseFlips = 5;
+constexpr int64_t kSmallFill = 160;  // CTAs that give about every SM one
 
 // Shared memory of a CTA, in 4-byte words: fixed part, then per replica.
 struct SmallSmem {
@@ -40,9 +50,9 @@ struct SmallSmem {
   static constexpr int INV = PERM + 2 * 64;    // [2][64] positions of spins
   static constexpr int WORK = INV + 2 * 64;    // [2][64] helper scratch
   static constexpr int FIXED = WORK + 2 * 64;
-  static constexpr int PER = 64 + 2 + 14;      // words per replica
-  static size_t bytes(int cap) {
-    return 4 * ((size_t)FIXED + (size_t)PER * cap);
+  static constexpr int PER = 64 + 2 + 15;      // words per replica
+  static size_t bytes(int cap) {  // and a byte per replica of any read
+    return 4 * ((size_t)FIXED + (size_t)PER * cap) + kMaxReplicas;
   }
 };
 
@@ -98,8 +108,14 @@ __device__ void small_order(uint64_t seed, uint32_t inst, uint32_t sweep,
 template <bool RANDOM>
 __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
     k_sweep_small(const SmallArgs a) {
+  namespace cg = cooperative_groups;
   extern __shared__ __align__(16) uint32_t sm[];
-  const int64_t r = blockIdx.x;
+  cg::cluster_group cl = cg::this_cluster();
+  const int csize = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  auto sync_read = [&]() {  // every CTA of the read
+    if (csize > 1) cl.sync(); else __syncthreads();
+  };
+  const int64_t r = blockIdx.x / csize;
   const int inst = a.p.read_inst[r];
   const int n = a.p.n[inst];
   const bool mine = n <= kSmallMaxN &&
@@ -111,6 +127,11 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
     const int NW = (int)(blockDim.x >> 5) - 1;  // warps with chains
     const int R = a.p.replicas[inst];
     const bool fit = R <= a.cap;  // else the state stays in global memory
+    // this CTA's chains c0 ... c1 - 1 (all of them in rank 0 if they don't
+    // fit); the energies of all, the slot map and the exchange are rank 0's
+    const int Rc = fit ? (R + csize - 1) / csize : R;
+    const int c0 = rank * Rc < R ? rank * Rc : R;
+    const int c1 = c0 + Rc < R ? c0 + Rc : R;
     const int64_t lread = r - a.p.read_off[inst];
     const int64_t base = a.p.chain_off[inst] + lread * R;
     const int words = (n + 31) >> 5;
@@ -140,6 +161,8 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
     float2* X2 = reinterpret_cast<float2*>(per + 74 * cap);  // draw, log
     float2* E2 = reinterpret_cast<float2*>(per + 76 * cap);  // energy, dbeta
     int32_t* B2 = reinterpret_cast<int32_t*>(per + 78 * cap);
+    uint32_t* LT = per + 79 * cap;                           // reject below
+    uint8_t* dense = reinterpret_cast<uint8_t*>(per + 80 * cap);  // [R]
     auto Hc = [&](int c) {
       return fit ? Hs + 64 * c : a.fields + (base + c) * (int64_t)a.field_ld;
     };
@@ -156,7 +179,7 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
         J[e] = c < n ? Jg[(int64_t)i * ld + c] : 0.0f;
       }
       if (fit) {
-        for (int e = tid; e < R * 64; e += blockDim.x) {
+        for (int e = 64 * c0 + tid; e < 64 * c1; e += blockDim.x) {
           const int c = e >> 6, i = e & 63;
           Hs[e] = i < n ? a.fields[(base + c) * (int64_t)a.field_ld + i]
                         : 0.0f;
@@ -172,12 +195,13 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
           const_cast<float*>(Bt)[c] = betas[c];
         }
       }
+      for (int c = tid; c < R; c += blockDim.x) dense[c] = 1;
       if (RANDOM && warp == NW)
         small_order(a.seed, (uint32_t)inst, sweep0, n, lane, work_s,
                     work_s + 64, perm_s + 64 * (sweep0 & 1),
                     inv_s + 64 * (sweep0 & 1));
     }
-    __syncthreads();
+    sync_read();
 
     for (int s = 0; s < a.num_sweeps; ++s) {
       const uint32_t sweep = sweep0 + (uint32_t)s;
@@ -191,7 +215,7 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
         const bool in0 = lane < n, in1 = k1 < n;
         const int i0 = in0 ? (RANDOM ? perm[lane] : lane) : 0;
         const int i1 = in1 ? (RANDOM ? perm[k1] : k1) : 0;
-        for (int c = warp; c < R; c += NW) {
+        for (int c = c0 + warp; c < c1; c += NW) {
           float* H = Hc(c);
           uint32_t* S = Sc(c);
           float h0 = in0 ? H[i0] : 0.0f, h1 = in1 ? H[i1] : 0.0f;
@@ -234,6 +258,61 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
           uint32_t p0 = __ballot_sync(0xffffffffu, in0);
           uint32_t p1 = __ballot_sync(0xffffffffu, in1);
           float d0 = 0.0f, d1 = 0.0f;  // energy change, 32 positions each
+          const uint32_t B0 = S0, B1 = S1;  // spins before the sweep
+          // one decision: position js of half hf, signed field y.  The exact
+          // rule where the thresholds have no answer.
+          auto exact = [&](int t, float y) {
+            return accept_slow_redraw(scale * y, beta, seed, (uint32_t)inst,
+                                      sweep, cl, (uint32_t)t);
+          };
+          bool again = !dense[c];
+          if (!again) {
+            // Flips are common: the positions in turn.  Every row, threshold
+            // and the field values after a flip are ready before the
+            // decision, which selects: about 60 cycles a position.  No exact
+            // rule here: a decision that needs it (once in a few hundred
+            // sweeps) has the chain swept again in rounds.
+            uint32_t unsure = 0u, f0 = 0u, f1 = 0u;
+            auto turn = [&](int t, bool hf) {
+              const int js = t & 31;
+              const float* row = J + 64 * (RANDOM ? perm[t] : t);
+              const float r0 = row[i0], r1 = row[i1];
+              const float th = __shfl_sync(0xffffffffu, hf ? th1 : th0, js);
+              const float tl = __shfl_sync(0xffffffffu, hf ? tl1 : tl0, js);
+              const bool sb = (((hf ? S1 : S0) >> js) & 1u) != 0u;
+              const float d = sb ? -scale : scale;
+              const float v0 = fmaf(d, r0, h0), v1 = fmaf(d, r1, h1);
+              const float hv = __shfl_sync(0xffffffffu, hf ? h1 : h0, js);
+              const float y = sb ? hv : -hv;
+              const bool acc = y >= th;
+              unsure |= (!acc && !(y < tl)) ? 1u : 0u;
+              h0 = acc ? v0 : h0;
+              h1 = acc ? v1 : h1;
+              const float de = acc ? scale * y : 0.0f;
+              if (hf) {
+                f1 |= acc ? 1u << js : 0u;
+                d1 -= de;
+              } else {
+                f0 |= acc ? 1u << js : 0u;
+                d0 -= de;
+              }
+            };
+            const int na = n < 32 ? n : 32;
+#pragma unroll 4
+            for (int t = 0; t < na; ++t) turn(t, false);
+#pragma unroll 4
+            for (int t = 32; t < n; ++t) turn(t, true);
+            again = unsure != 0u;
+            if (again) {
+              h0 = in0 ? H[i0] : 0.0f;
+              h1 = in1 ? H[i1] : 0.0f;
+              d0 = d1 = 0.0f;
+            } else {
+              S0 ^= f0;
+              S1 ^= f1;
+            }
+          }
+          if (again) {
           for (;;) {
             const float y0 = __uint_as_float(__float_as_uint(h0) ^ g0);
             const float y1 = __uint_as_float(__float_as_uint(h1) ^ g1);
@@ -261,9 +340,7 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
                                  : js + (hf ? 32 : 0);
             bool acc = ((hf ? a1 : a0) & bit) != 0u;
             if (!acc)  // inside the band: the exact rule
-              acc = accept_slow_redraw(scale * y, beta, seed, (uint32_t)inst,
-                                       sweep, cl,
-                                       (uint32_t)(js + (hf ? 32 : 0)));
+              acc = exact(js + (hf ? 32 : 0), y);
             if (acc) {
               const bool sb = ((hf ? S1 : S0) & bit) != 0u;
               const float d = sb ? -scale : scale;
@@ -282,6 +359,7 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
               }
             }
           }
+          }
           if (in0) H[i0] = h0;
           if (in1) H[i1] = h1;
           uint32_t na = S0, nb = S1;
@@ -293,6 +371,7 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
                 0xffffffffu, in1 && (((q1 < 32 ? S0 : S1) >> (q1 & 31)) & 1u));
           }
           if (lane == 0) {
+            dense[c] = kDenseFlips * (__popc(S0 ^ B0) + __popc(S1 ^ B1)) > n;
             S[0] = na;
             if (words > 1) S[1] = nb;
             if (fit) {
@@ -305,11 +384,16 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
         }
       } else {
         // ---------------------------------------------------- work ahead
-        if (fit && xch)
+        if (fit && xch && rank == 0)
           for (int k = lane; k < R - 1; k += 32) {
             const uint32_t x = draw1(a.seed, TAG_PT, (uint32_t)inst, sweep,
                                      (uint32_t)lread, (uint32_t)k);
-            X2[k] = make_float2(__uint_as_float(x), log_uniform_f32(x));
+            // accept a pair at de >= .y, reject it below LT: log u and its
+            // band (pt_accept_lf); in between, the exact rule
+            const float lf = log_uniform_f32(x);
+            const float m = fmaf(2e-6f, fabsf(lf), 3.1e-5f);
+            X2[k] = make_float2(__uint_as_float(x), fminf(lf + m, 0.0f));
+            LT[k] = __float_as_uint(lf - m);
           }
         if (RANDOM && s + 1 < a.num_sweeps) {
           const uint32_t nx = (sweep + 1u) & 1u;
@@ -321,12 +405,13 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
 
       // ------------------------- energies, best states, exchange: warp 0
       if (warp == 0) {
-        for (int c = lane; c < R; c += 32) {
+        for (int c = c0 + lane; c < c1; c += 32) {
           float e = E[c];
           if (fit) {
             const float2 d = dE[c];
             e = (float)((double)e + ((double)d.x + (double)d.y));
             E[c] = e;
+            if (rank != 0) cl.map_shared_rank(E, 0)[c] = e;
           }
           // strict < (pysa/simulation.py:150-171)
           if (e < bestE[c]) {
@@ -339,6 +424,9 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
           }
         }
         __syncwarp();
+      }
+      if (csize > 1) cl.sync();  // the energies are in rank 0
+      if (warp == 0 && rank == 0) {
         if (xch && R > 1) {
           // pairs (R-1, R-2), (R-2, R-3), ... in order: only the replica
           // entering slot k1 carries from pair to pair, so every pair's
@@ -356,31 +444,57 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
           if (lane == 0) {
             int cb = B[R - 1];
             float ce = E[cb];
-            for (int k = 0; k < R - 1; ++k) {
-              int b2;
-              float2 e2, x2;
-              if (fit) {
-                b2 = B2[k];
-                e2 = E2[k];
-                x2 = X2[k];
-              } else {
-                const int t1 = R - k - 1, t2 = R - k - 2;
-                b2 = B[t2];
-                e2 = make_float2(E[b2], __fsub_rn(Bt[t1], Bt[t2]));
-                const uint32_t x = draw1(a.seed, TAG_PT, (uint32_t)inst,
-                                         sweep, (uint32_t)lread, (uint32_t)k);
-                x2 = make_float2(__uint_as_float(x), log_uniform_f32(x));
+            bool redo = !fit;
+            if (fit) {
+              // without the exact rule; a pair that needs it has the pass
+              // made again below
+              const int cb0 = cb;
+              const float ce0 = ce;
+              uint32_t unsure = 0u;
+#pragma unroll 4
+              for (int k = 0; k < R - 1; ++k) {
+                const int b2 = B2[k];
+                const float2 e2 = E2[k], x2 = X2[k];
+                const float de = __fmul_rn(__fsub_rn(ce, e2.x), e2.y);
+                const bool sw = de >= x2.y;
+                unsure |=
+                    (!sw && !(de < __uint_as_float(LT[k]))) ? 1u : 0u;
+                B[R - k - 1] = sw ? b2 : cb;  // final: no later pair
+                cb = sw ? cb : b2;
+                ce = sw ? ce : e2.x;
               }
-              const float de = __fmul_rn(__fsub_rn(ce, e2.x), e2.y);
-              const bool sw = pt_accept_lf(de, x2.y, __float_as_uint(x2.x));
-              B[R - k - 1] = sw ? b2 : cb;  // final: no later pair
-              cb = sw ? cb : b2;
-              ce = sw ? ce : e2.x;
+              if (unsure) {
+                for (int k = 0; k < R - 1; ++k) B[R - k - 2] = B2[k];
+                B[R - 1] = cb0;
+                cb = cb0;
+                ce = ce0;
+                redo = true;
+              }
+            }
+            if (redo) {
+              for (int k = 0; k < R - 1; ++k) {
+                const int t1 = R - k - 1, t2 = R - k - 2, b2 = B[t2];
+                const float e2 = E[b2];
+                const float de = __fmul_rn(__fsub_rn(ce, e2),
+                                           __fsub_rn(Bt[t1], Bt[t2]));
+                const bool sw = pt_accept(
+                    de, draw1(a.seed, TAG_PT, (uint32_t)inst, sweep,
+                              (uint32_t)lread, (uint32_t)k));
+                B[t1] = sw ? b2 : cb;
+                cb = sw ? cb : b2;
+                ce = sw ? ce : e2;
+              }
             }
             B[0] = cb;
           }
           __syncwarp();
-          for (int k = lane; k < R; k += 32) beta_c[B[k]] = Bt[k];
+          for (int k = lane; k < R; k += 32) {
+            const int c = B[k], own = csize > 1 ? c / Rc : 0;
+            if (own == 0)
+              beta_c[c] = Bt[k];
+            else
+              cl.map_shared_rank(beta_c, own)[c] = Bt[k];
+          }
         }
         if (a.log_omega_stride > 0) {
           // terms of the sorted ladder, f32 products, summed in f64
@@ -397,24 +511,25 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
             a.s.log_omega[r * a.log_omega_stride + sweep] = lw;
         }
       }
-      __syncthreads();
+      sync_read();
     }
 
     // ---- state out
     if (fit) {
-      for (int e = tid; e < R * 64; e += blockDim.x) {
+      for (int e = 64 * c0 + tid; e < 64 * c1; e += blockDim.x) {
         const int c = e >> 6, i = e & 63;
         if (i < n) a.fields[(base + c) * (int64_t)a.field_ld + i] = Hs[e];
       }
-      for (int c = tid; c < R; c += blockDim.x) {
+      for (int c = c0 + tid; c < c1; c += blockDim.x) {
         const int64_t g = base + c;
         a.s.spins[g * a.p.words] = Ss[2 * c];
         if (words > 1) a.s.spins[g * a.p.words + 1] = Ss[2 * c + 1];
         a.s.energies[g] = E[c];
-        a.s.beta_idx[g] = B[c];
         a.s.chain_beta[g] = beta_c[c];
         a.s.best_energy[g] = bestE[c];
       }
+      if (rank == 0)
+        for (int c = tid; c < R; c += blockDim.x) a.s.beta_idx[base + c] = B[c];
     }
   }
   __syncthreads();
@@ -436,19 +551,34 @@ cudaError_t launch_small(SmallArgs a, bool random, cudaStream_t st) {
   const int64_t avg = (a.p.num_chains + a.p.num_reads - 1) / a.p.num_reads;
   a.cap = (int32_t)(avg < kMaxReplicas ? (avg > 1 ? avg : 1) : kMaxReplicas);
   a.cap += a.cap & 1;  // pairs of words stay 8-byte aligned
-  const int nw = a.cap < kMaxSmallWarps ? a.cap : kMaxSmallWarps;
+  // a cluster per read while the reads leave SMs idle and a CTA keeps four
+  // chains or more; the chains of a CTA in equal turns of its warps
+  int cs = 1;
+  while (cs < 8 && a.p.num_reads * cs * 2 <= kSmallFill &&
+         a.cap / (2 * cs) >= 4)
+    cs *= 2;
+  const int per = (a.cap + cs - 1) / cs;
+  const int turns = (per + kMaxSmallWarps - 1) / kMaxSmallWarps;
+  const int nw = (per + turns - 1) / turns;
   const size_t smem = SmallSmem::bytes(a.cap);
   const void* f = random ? (const void*)k_sweep_small<true>
                          : (const void*)k_sweep_small<false>;
   cudaError_t e = cudaFuncSetAttribute(
       f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((unsigned)a.p.num_reads), block(32 * (nw + 1));
-  if (random)
-    k_sweep_small<true><<<grid, block, smem, st>>>(a);
-  else
-    k_sweep_small<false><<<grid, block, smem, st>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(a.p.num_reads * cs));
+  cfg.blockDim = dim3(32 * (nw + 1));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cs;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return random ? cudaLaunchKernelEx(&cfg, k_sweep_small<true>, a)
+                : cudaLaunchKernelEx(&cfg, k_sweep_small<false>, a);
 }
 
 }  // namespace pysa_gb
