@@ -13,6 +13,8 @@
 //
 // k_logz_exact enumerates all 2^n states in Gray-code order in f64, with an
 // online log-sum-exp per thread.
+#include <type_traits>
+
 #include "aux.cuh"
 #include "ais_api.h"
 
@@ -194,17 +196,246 @@ __global__ void __launch_bounds__(128) k_ais(const AisArgs a) {
   }
 }
 
-// Small instances (n <= 32): one thread per sample, its spins in one word
-// and its fields in a shared-memory column [32][128] (conflict-free), the
-// instance's couplings in shared memory too (the row of the visited spin is
-// the same for every thread: a broadcast).  The arithmetic is k_ais's: the
-// same f32 field updates (a rejected attempt adds 0 * J, which changes no
-// field but possibly the sign of a zero), the same f64 energy and weights,
-// the same uniforms (one draw of 4 per 4 steps instead of one per step).
-// No shuffles or ballots, and a warp covers 32 samples instead of 8.
+// Thresholds of one beta step in field units (see FieldThreshold): with y =
+// +-field signed so that dn = scale y, a move is accepted when y >= th + off
+// and rejected when y < tl + off, off shifting both by the reference's log
+// ratio for the spin's value; in between, and for a beta that is not a plain
+// positive number, ais_accept decides.
+struct AisThreshold {
+  float tl1, tl0, th1, th0, up, cap;
+  __device__ __forceinline__ AisThreshold(float beta, float scale, double lr,
+                                          bool uniform_ref) {
+    constexpr float kLn2 = 0.69314718056f;
+    const bool plain = beta >= 1e-30f && beta < 1e30f;
+    const float inv = plain ? 1.0f / (beta * scale) : 0.0f;
+    // a set bit going down changes the log ratio by -c
+    const float c = uniform_ref ? 0.0f
+                                : (float)((1.0 - (double)beta) * lr);
+    const float m = fmaf(1e-6f, fabsf(c), 3e-5f) * inv;
+    tl1 = kLn2 * 1.000001f * inv;
+    th1 = kLn2 * 0.999999f * inv;
+    tl0 = plain ? -m : -INFINITY;
+    // (NaN: no y is above it, an infinite one included)
+    th0 = plain ? m : __int_as_float(0x7fc00000);
+    up = plain ? c * inv : 0.0f;
+    // the uniform reference accepts every dn >= 0
+    cap = !plain ? th0 : uniform_ref ? 0.0f : INFINITY;
+  }
+  __device__ __forceinline__ void at(uint32_t x, float& tl, float& th) const {
+    const float l2 = log2_uniform(x);
+    tl = fmaf(tl1, l2, tl0);
+    th = fminf(fmaf(th1, l2, th0), cap);
+  }
+};
+
+// Exact pair (hi, lo) + x (Knuth's two-sum).
+__device__ __forceinline__ void energy_add(float2& p, float x) {
+  const float s = p.x + x;
+  const float bb = s - p.x;
+  p.y += (p.x - (s - bb)) + (x - bb);
+  p.x = s;
+}
+// The pair rounded to f32 (infinite or NaN sums have no second part).
+__device__ __forceinline__ float energy_of(const float2& p) {
+  return fabsf(p.x) < INFINITY ? p.x + p.y : p.x;
+}
+
+// A warp per sample, the visiting positions in turn (n <= 32 NC).  Lane l
+// holds the fields of columns l, l + 32, ... in registers and, as bits m of
+// one word, the spins 32 m + l; the instance's couplings are in shared
+// memory.  Row, thresholds and the fields after a flip do not depend on the
+// decision, which only selects: about 60 cycles a position whatever the
+// acceptance.  A decision inside the band has its sweep done again with the
+// exact rule.  For few samples: the kernels that hold several samples per
+// warp or thread need fewer instructions each, but too few warps then leave
+// every SM waiting.  Measured for n = 96, 1000 samples, 200 steps: 12.7 ms
+// with 8 samples per warp, 1.64 ms here.
+template <int NC, bool RANDOM>
+__global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
+  extern __shared__ __align__(16) float Jt[];  // [n][32 NC]
+  const int inst = blockIdx.y;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (a.replicas[inst] != 1) {
+    if (blockIdx.x == 0 && tid == 0) set_status(a.status, PYSA_GB_ERR_ARG);
+    return;
+  }
+  const int n = a.n_tab[inst], ld = a.ld_tab[inst];
+  const int64_t samples = a.reads[inst];
+  const int WPC = blockDim.x >> 5;
+  if ((int64_t)blockIdx.x * WPC >= samples) return;  // whole CTA
+  const float* Jp = a.J + a.j_off[inst];
+  for (int e = tid; e < n * 32 * NC; e += blockDim.x) {
+    const int r = e / (32 * NC), c = e % (32 * NC);
+    Jt[e] = c < n ? Jp[(int64_t)r * ld + c] : 0.0f;
+  }
+  __syncthreads();
+  const int64_t my = (int64_t)blockIdx.x * WPC + warp;
+  if (my >= samples) return;
+  const int64_t myc = a.chain_off[inst] + my;
+  const bool ising = a.problem_type == PYSA_GB_ISING;
+  const float scale = ising ? 2.0f : 1.0f;
+  const bool uniform_ref = a.ref != 1;
+  const int words = (n + 31) >> 5;
+  float h[NC];
+  uint32_t sp = 0u;  // bit m: spin 32 m + lane
+#pragma unroll
+  for (int m = 0; m < NC; ++m) {
+    const int col = 32 * m + lane;
+    h[m] = col < n ? a.fields[myc * a.field_ld + col] : 0.0f;
+    if (m < words)
+      sp |= ((a.spins[myc * a.words + m] >> lane) & 1u) << m;
+  }
+  float2 E = make_float2(a.energies[myc], 0.0f);
+  double lw = 0.0;
+  float beta_old = 0.0f;
+  const double lr = uniform_ref ? 0.0 : log((1.0 - a.p) / a.p);
+  const double logp = uniform_ref ? 0.0 : log(a.p);
+  const double log1p_ = uniform_ref ? 0.0 : log(1.0 - a.p);
+  // columns past n hold no spin: their bits stay 0
+  auto ones = [&]() {
+    return uniform_ref ? 0 : __reduce_add_sync(0xffffffffu, __popc(sp));
+  };
+  for (int k = 0; k < a.num_temps; ++k) {
+    const float beta = a.temps[k];
+    if (a.order == 1)
+      lw += ais_dlw(beta, beta_old, energy_of(E), n, ones(), logp, log1p_,
+                    uniform_ref);
+    const int32_t* perm =
+        a.perm + ((int64_t)k * a.num_instances + inst) * a.max_n;
+    const AisThreshold at(beta, scale, lr, uniform_ref);
+    // one sweep; EXACT asks ais_accept where the thresholds have no answer,
+    // otherwise returns whether some decision needed it
+    auto sweep = [&](auto exact_t) {
+      constexpr bool EXACT = decltype(exact_t)::value;
+      uint32_t unsure = 0u;
+      for (int b = 0; b < words; ++b) {
+        const int t0 = 32 * b;
+        int il = t0 + lane;
+        if (RANDOM) il = il < n ? perm[il] : 0;
+        float tl, th;
+        {
+          uint32_t x[4], v[4];
+          draw4(a.seed, TAG_AIS, (uint32_t)inst, (uint32_t)k, (uint32_t)my,
+                (uint32_t)(8 * b + (lane & 7)), x);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            v[q] = __shfl_sync(0xffffffffu, x[q], lane >> 2);
+          const int q = lane & 3;
+          at.at(q < 2 ? (q ? v[1] : v[0]) : (q == 2 ? v[2] : v[3]), tl, th);
+        }
+        auto turn = [&](int t) {
+          const int p = t - t0;
+          const int i = RANDOM ? __shfl_sync(0xffffffffu, il, p) : t;
+          const int mi = i >> 5, l = i & 31;
+          const float* row = Jt + i * (32 * NC) + lane;
+          const bool sb =
+              ((__shfl_sync(0xffffffffu, sp, l) >> mi) & 1u) != 0u;
+          const float d = sb ? -scale : scale;
+          const float off = sb ? at.up : -at.up;
+          const float thp = __shfl_sync(0xffffffffu, th, p) + off;
+          const float tlp = __shfl_sync(0xffffffffu, tl, p) + off;
+          float hm = h[0];
+#pragma unroll
+          for (int m = 1; m < NC; ++m) hm = m == mi ? h[m] : hm;
+          const float hv = __shfl_sync(0xffffffffu, hm, l);
+          float v[NC];
+#pragma unroll
+          for (int m = 0; m < NC; ++m) v[m] = fmaf(d, row[32 * m], h[m]);
+          const float y = sb ? hv : -hv;
+          bool acc = y >= thp;
+          if constexpr (EXACT) {
+            if (!acc && !(y < tlp))
+              acc = ais_accept(beta, scale * y, sb, lr, uniform_ref,
+                               draw1(a.seed, TAG_AIS, (uint32_t)inst,
+                                     (uint32_t)k, (uint32_t)my, (uint32_t)t));
+          } else {
+            unsure |= (!acc && !(y < tlp)) ? 1u : 0u;
+          }
+#pragma unroll
+          for (int m = 0; m < NC; ++m) h[m] = acc ? v[m] : h[m];
+          sp ^= acc && lane == l ? 1u << mi : 0u;
+          energy_add(E, acc ? -(scale * y) : 0.0f);
+        };
+        const int te = t0 + 32 < n ? t0 + 32 : n;
+        if constexpr (EXACT) {
+#pragma unroll 1
+          for (int t = t0; t < te; ++t) turn(t);
+        } else {
+#pragma unroll 4
+          for (int t = t0; t < te; ++t) turn(t);
+        }
+      }
+      return unsure != 0u;
+    };
+    float h0[NC];
+#pragma unroll
+    for (int m = 0; m < NC; ++m) h0[m] = h[m];
+    const uint32_t sp0 = sp;
+    const float2 E0 = E;
+    if (sweep(std::false_type{})) {
+#pragma unroll
+      for (int m = 0; m < NC; ++m) h[m] = h0[m];
+      sp = sp0;
+      E = E0;
+      sweep(std::true_type{});
+    }
+    if (a.order == 0)
+      lw += ais_dlw(beta, beta_old, energy_of(E), n, ones(), logp, log1p_,
+                    uniform_ref);
+    beta_old = beta;
+  }
+  if (lane == 0) {
+    a.log_w[myc] = lw;
+    a.energies[myc] = energy_of(E);
+  }
+#pragma unroll
+  for (int m = 0; m < NC; ++m) {
+    const uint32_t w = __ballot_sync(0xffffffffu, (sp >> m) & 1u);
+    if (m < words && lane == 0) a.spins[myc * a.words + m] = w;
+  }
+}
+
+// Two f32 multiply-adds at once (each lane of the pair rounded as fmaf).
+__device__ __forceinline__ uint64_t fma2(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float half2(uint64_t v, bool hi) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return hi ? b : a;
+}
+
+// Two pairs from shared memory.  Volatile: the couplings never change, and
+// unrolled code would otherwise try to keep all of them in registers.
+__device__ __forceinline__ ulonglong2 load_pairs(uint32_t addr) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];"
+               : "=l"(v.x), "=l"(v.y)
+               : "r"(addr));
+  return v;
+}
+
+// Small instances (n <= NP <= 32), many samples: one thread per sample, its
+// spins in one word and its fields in NP registers as pairs, the instance's
+// couplings in shared memory (the row of the visited spin is the same for
+// every thread: broadcast 16-byte loads).  A position costs NP / 2 paired
+// multiply-adds and NP / 4 loads; a rejected attempt adds 0 * J, which changes
+// no field but possibly the sign of a zero.  Bound by instruction issue: the
+// Philox draw (one per four positions) and the field updates take most of
+// it.  Measured for 64 instances of n = 24, 1024 samples, 200 steps: 4.33 ms
+// with the fields in shared memory and f64 energies, 1.18 ms here (random
+// order 4.42 and 1.75).
+template <int NP, bool RANDOM>
 __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
-  __shared__ float Js[32 * 32];
-  __shared__ float Hs[32 * 128];
+  __shared__ __align__(16) float Js[NP * NP];
+  const uint32_t js_addr = smem_addr(Js);
   const int inst = blockIdx.y;
   const int tid = threadIdx.x;
   if (a.replicas[inst] != 1) {
@@ -216,68 +447,113 @@ __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
   const int64_t samples = a.reads[inst];
   if ((int64_t)blockIdx.x * blockDim.x >= samples) return;  // whole CTA
   const float* Jp = a.J + a.j_off[inst];
-  for (int e = tid; e < 32 * 32; e += blockDim.x) {
-    const int r = e >> 5, c = e & 31;
+  for (int e = tid; e < NP * NP; e += blockDim.x) {
+    const int r = e / NP, c = e % NP;
     Js[e] = (r < n && c < n) ? Jp[(int64_t)r * ld + c] : 0.0f;
   }
   const int64_t my = (int64_t)blockIdx.x * blockDim.x + tid;
   const bool valid = my < samples;
   const int64_t myc = a.chain_off[inst] + (valid ? my : 0);
-  float* H = Hs + tid;  // field of spin c at H[c * 128]
-  for (int c = 0; c < 32; ++c)
-    H[c * 128] = (valid && c < n) ? a.fields[myc * a.field_ld + c] : 0.0f;
+  uint64_t H[NP / 2];
+#pragma unroll
+  for (int c = 0; c < NP / 2; ++c)
+    H[c] = pack2(
+        valid && 2 * c < n ? a.fields[myc * a.field_ld + 2 * c] : 0.0f,
+        valid && 2 * c + 1 < n ? a.fields[myc * a.field_ld + 2 * c + 1]
+                               : 0.0f);
   __syncthreads();
   if (!valid) return;
   const bool ising = a.problem_type == PYSA_GB_ISING;
+  const float scale = ising ? 2.0f : 1.0f;
+  const bool uniform_ref = a.ref != 1;
   uint32_t word = a.spins[myc * a.words];
-  double E = (double)a.energies[myc];
-  int ones = __popc(word);
+  float2 E = make_float2(a.energies[myc], 0.0f);
   double lw = 0.0;
   float beta_old = 0.0f;
-  const double lr = a.ref == 1 ? log((1.0 - a.p) / a.p) : 0.0;
-  const double logp = a.ref == 1 ? log(a.p) : 0.0;
-  const double log1p_ = a.ref == 1 ? log(1.0 - a.p) : 0.0;
+  const double lr = uniform_ref ? 0.0 : log((1.0 - a.p) / a.p);
+  const double logp = uniform_ref ? 0.0 : log(a.p);
+  const double log1p_ = uniform_ref ? 0.0 : log(1.0 - a.p);
   for (int k = 0; k < a.num_temps; ++k) {
     const float beta = a.temps[k];
-    if (a.order == 1) {
-      lw += ais_dlw(beta, beta_old, (float)E, n, ones, logp, log1p_,
-                    a.ref != 1);
-    }
+    if (a.order == 1)
+      lw += ais_dlw(beta, beta_old, energy_of(E), n, __popc(word), logp,
+                    log1p_, uniform_ref);
     const int32_t* perm =
         a.perm + ((int64_t)k * a.num_instances + inst) * a.max_n;
+    const AisThreshold at(beta, scale, lr, uniform_ref);
     uint32_t rnd[4];
-    for (int t = 0; t < n; ++t) {
-      if ((t & 3) == 0)
+    auto turn = [&](int t, int i, float hv, uint32_t x) {
+      const bool sb = (word >> i) & 1u;
+      const float y = sb ? hv : -hv;
+      const float off = sb ? at.up : -at.up;
+      float tl, th;
+      at.at(x, tl, th);
+      bool acc = y >= th + off;
+      if (!acc && !(y < tl + off))
+        acc = ais_accept(beta, scale * y, sb, lr, uniform_ref, x);
+      word ^= acc ? 1u << i : 0u;
+      energy_add(E, acc ? -(scale * y) : 0.0f);
+      const float d = acc ? (sb ? -scale : scale) : 0.0f;
+      const uint64_t dd = pack2(d, d);
+      const uint32_t row = js_addr + (uint32_t)(i * NP * 4);
+#pragma unroll
+      for (int c = 0; c < NP / 4; ++c) {
+        const ulonglong2 j = load_pairs(row + 16 * c);
+        H[2 * c] = fma2(dd, j.x, H[2 * c]);
+        H[2 * c + 1] = fma2(dd, j.y, H[2 * c + 1]);
+      }
+    };
+    if constexpr (RANDOM) {
+#pragma unroll 1
+      for (int t = 0; t < n; t += 4) {
+        int ids[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ids[q] = t + q < n ? perm[t + q] : 0;
         draw4(a.seed, TAG_AIS, (uint32_t)inst, (uint32_t)k, (uint32_t)my,
               (uint32_t)(t >> 2), rnd);
-      const uint32_t x = (t & 3) == 0 ? rnd[0] : (t & 3) == 1 ? rnd[1]
-                         : (t & 3) == 2 ? rnd[2] : rnd[3];
-      const int i = a.update == PYSA_GB_RANDOM ? perm[t] : t;
-      const float hv = H[i * 128];
-      const bool sbit = (word >> i) & 1u;
-      const float dn = ising ? (sbit ? 2.0f * hv : -2.0f * hv)
-                             : (sbit ? hv : -hv);
-      const bool acc = ais_accept(beta, dn, sbit, lr, a.ref != 1, x);
-      if (acc) {
-        E -= (double)dn;
-        ones += sbit ? -1 : 1;
-        word ^= 1u << i;
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          if (t + q >= n) break;
+          const int i = q < 2 ? (q ? ids[1] : ids[0])
+                              : (q == 2 ? ids[2] : ids[3]);
+          // the spin is the same in every thread: a uniform branch picks its
+          // register
+          uint64_t pr = 0ull;
+          switch (i >> 1) {
+#define PYSA_GB_FIELD(c) \
+  case c:                \
+    if constexpr (c < NP / 2) pr = H[c < NP / 2 ? c : 0]; \
+    break;
+            PYSA_GB_FIELD(0) PYSA_GB_FIELD(1) PYSA_GB_FIELD(2)
+            PYSA_GB_FIELD(3) PYSA_GB_FIELD(4) PYSA_GB_FIELD(5)
+            PYSA_GB_FIELD(6) PYSA_GB_FIELD(7) PYSA_GB_FIELD(8)
+            PYSA_GB_FIELD(9) PYSA_GB_FIELD(10) PYSA_GB_FIELD(11)
+            PYSA_GB_FIELD(12) PYSA_GB_FIELD(13) PYSA_GB_FIELD(14)
+            PYSA_GB_FIELD(15)
+#undef PYSA_GB_FIELD
+            default: break;
+          }
+          turn(t + q, i, half2(pr, i & 1),
+               q < 2 ? (q ? rnd[1] : rnd[0]) : (q == 2 ? rnd[2] : rnd[3]));
+        }
       }
-      const float d = acc ? (ising ? (sbit ? -2.0f : 2.0f)
-                                   : (sbit ? -1.0f : 1.0f))
-                          : 0.0f;
-      const float* Jr = Js + i * 32;
-#pragma unroll 8
-      for (int c = 0; c < n; ++c) H[c * 128] = fmaf(d, Jr[c], H[c * 128]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < NP; ++t) {
+        if (t >= n) break;  // uniform
+        if ((t & 3) == 0)
+          draw4(a.seed, TAG_AIS, (uint32_t)inst, (uint32_t)k, (uint32_t)my,
+                (uint32_t)(t >> 2), rnd);
+        turn(t, t, half2(H[t >> 1], t & 1), rnd[t & 3]);
+      }
     }
-    if (a.order == 0) {
-      lw += ais_dlw(beta, beta_old, (float)E, n, ones, logp, log1p_,
-                    a.ref != 1);
-    }
+    if (a.order == 0)
+      lw += ais_dlw(beta, beta_old, energy_of(E), n, __popc(word), logp,
+                    log1p_, uniform_ref);
     beta_old = beta;
   }
   a.log_w[myc] = lw;
-  a.energies[myc] = (float)E;
+  a.energies[myc] = energy_of(E);
   a.spins[myc * a.words] = word;
 }
 
@@ -293,15 +569,65 @@ static cudaError_t launch_ais_t(const AisArgs& a, int64_t max_samples,
   return cudaGetLastError();
 }
 
+template <int NC>
+static cudaError_t launch_turn_t(const AisArgs& a, int64_t max_samples,
+                                 cudaStream_t st) {
+  const bool random = a.update == PYSA_GB_RANDOM;
+  const int wpc = NC >= 8 ? 16 : 4;  // samples that share the couplings
+  const size_t smem = (size_t)a.max_n * 32 * NC * 4;
+  const void* f = random ? (const void*)k_ais_turn<NC, true>
+                         : (const void*)k_ais_turn<NC, false>;
+  cudaError_t e = cudaFuncSetAttribute(
+      f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  dim3 grid((unsigned)((max_samples + wpc - 1) / wpc),
+            (unsigned)a.num_instances);
+  if (random)
+    k_ais_turn<NC, true><<<grid, 32 * wpc, smem, st>>>(a);
+  else
+    k_ais_turn<NC, false><<<grid, 32 * wpc, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int NP>
+static cudaError_t launch_small_t(const AisArgs& a, int64_t max_samples,
+                                  cudaStream_t st) {
+  const int64_t blocks = (max_samples + 127) / 128;
+  dim3 grid((unsigned)(blocks > 0 ? blocks : 1), (unsigned)a.num_instances);
+  if (a.update == PYSA_GB_RANDOM)
+    k_ais_small<NP, true><<<grid, 128, 0, st>>>(a);
+  else
+    k_ais_small<NP, false><<<grid, 128, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+// Few samples: a warp each.  Many: threads (n <= 32) or warps holding several
+// samples, which need fewer instructions per attempt once the GPU is full.
+// Whole calls with 200 (n = 20) or 50 (n >= 50) steps, warp per sample against
+// the kernel for many: n = 20, 4096 samples 2.0 against 2.3 ms; n = 96, 24000
+// samples 9.5 against 12.1; n = 50, 16000 4.0 against 4.4; n = 200, 16000
+// 17.5 against 24.4.
+constexpr int64_t kTurnSamples = 4096;  // n <= 32
+constexpr int64_t kTurnSamplesWide = 24576;
+// Widest instance whose couplings the warp-per-sample kernel keeps in shared
+// memory (n x 256 floats at n > 128).
+constexpr int kTurnMaxN = 220;
+
 cudaError_t launch_ais(const AisArgs& a, int64_t max_samples, cudaStream_t st) {
-  if (a.max_n <= 32) {
-    const int64_t blocks = (max_samples + 127) / 128;
-    dim3 grid((unsigned)(blocks > 0 ? blocks : 1), (unsigned)a.num_instances);
-    k_ais_small<<<grid, 128, 0, st>>>(a);
-    return cudaGetLastError();
-  }
+  const int64_t total = max_samples * a.num_instances;
   const int nc = (a.max_n + 31) / 32;
-  if (nc <= 1) return launch_ais_t<1, 8>(a, max_samples, st);
+  if (nc <= 1) {
+    if (total <= kTurnSamples) return launch_turn_t<1>(a, max_samples, st);
+    if (a.max_n <= 8) return launch_small_t<8>(a, max_samples, st);
+    if (a.max_n <= 16) return launch_small_t<16>(a, max_samples, st);
+    if (a.max_n <= 24) return launch_small_t<24>(a, max_samples, st);
+    return launch_small_t<32>(a, max_samples, st);
+  }
+  if (total <= kTurnSamplesWide && a.max_n <= kTurnMaxN) {
+    if (nc <= 2) return launch_turn_t<2>(a, max_samples, st);
+    if (nc <= 4) return launch_turn_t<4>(a, max_samples, st);
+    return launch_turn_t<8>(a, max_samples, st);
+  }
   if (nc <= 2) return launch_ais_t<2, 8>(a, max_samples, st);
   if (nc <= 4) return launch_ais_t<4, 8>(a, max_samples, st);
   if (nc <= 8) return launch_ais_t<8, 4>(a, max_samples, st);
