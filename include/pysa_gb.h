@@ -175,8 +175,10 @@ typedef struct {
   int32_t plain_live;       /* host, from pysa_gb_tc_setup: bit v set when
                                plain variant v still has instances */
   int32_t tc_fusable;       /* host, from pysa_gb_tc_setup: 1 when every
-                               tensor-core instance's R divides its chains
-                               per CTA (exchange can run inside the kernel) */
+                               tensor-core work item holds whole reads
+                               (exchange can run inside the kernel): every R
+                               at most the chains per CTA, and the chain
+                               slots left empty worth it */
   int32_t *tc_sched;        /* [2 + tc_num_items] device scratch of the
                                persistent tensor-core kernel */
   int32_t tc_unit_sweeps;   /* sweeps per work unit of that kernel (0: 8) */
@@ -212,9 +214,9 @@ typedef struct {
   /* caller: chains per tensor-core work item (0: automatic -- a CTA's full
    * tensor memory, 128 / F chains, halved while the batch would leave SMs
    * idle); otherwise the largest multiple of each instance's granule (R
-   * when R divides 128 / F, else 32) not above min(this, 128 / F).  Read
-   * by pysa_gb_tc_setup; pysa_gb_tc_workspace sizes for the smallest
-   * items any value can give. */
+   * when items hold whole reads or R divides 128 / F, else 32) not above
+   * min(this, 128 / F).  Read by pysa_gb_tc_setup; pysa_gb_tc_workspace
+   * sizes for the smallest items any value can give. */
   int32_t tc_item_chains;
   /* host, from pysa_gb_tc_setup: bit v set when every work item of fold
    * variant v (F = 1, 2, 4) belongs to an instance of the same n.  Fused

@@ -374,29 +374,60 @@ static inline bool tc_selected(const pysa_gb_host_tables* host, int i,
   return !is_sparse(host, i) && n >= (min_n < 64 ? 64 : min_n) && n <= 2048;
 }
 
-// Chains per tensor-core work item of every selected instance.  fixed = 0:
-// a CTA's full tensor memory (128/F chains), halved while the batch would
-// fill fewer CTAs than the GPU has SMs and the halves still hold whole reads
-// (or whole warps when R does not divide 128/F).  fixed > 0: the largest
-// multiple of the instance's granule (R, or 32) not above min(fixed, 128/F),
-// at least one granule.  fixed < 0: one granule (the smallest items, for
-// sizing).  0 for instances left to the plain kernel.
+// Whether the tensor-core work items of a batch hold whole reads, so that
+// several sweeps run in one launch with the exchange inside: every R fits a
+// CTA's chains, and the chain slots left empty (R need not divide 128 / F)
+// cost less than a launch and an exchange kernel per sweep.  Estimated from
+// 64-spin blocks of 4 us with the SMs full, 1.1 of that and 14 us per sweep
+// unfused.  Measured (whole calls, unfused -> fused): n = 200, 3 reads of 9,
+// 100 random sweeps 10.7 -> 5.3 ms; n = 500, 200 reads of 24, 32 sweeps 3.7 ->
+// 2.6; n = 900, 256 reads of 24 7.4 -> 4.3; n = 1800, 128 reads of 24, 16
+// sweeps 8.2 -> 4.0.
+static bool tc_whole_reads(int num_instances, const pysa_gb_host_tables* host,
+                           int min_n) {
+  double whole = 0.0, full = 0.0;  // item-blocks
+  double nb_max = 0.0;
+  for (int i = 0; i < num_instances; ++i) {
+    if (!tc_selected(host, i, min_n)) continue;
+    const int cc = tc_chains_per_cta(host->n[i]), R = host->replicas[i];
+    if (R > cc) return false;
+    const int64_t reads = host->reads[i], per = cc / R;
+    const double nb = (host->n[i] + 63) / 64;
+    whole += nb * (double)((reads + per - 1) / per);
+    full += nb * (double)((reads * R + cc - 1) / cc);
+    nb_max = nb > nb_max ? nb : nb_max;
+  }
+  const double sms = sm_count();
+  auto blocks = [&](double work) {  // per sweep, at least one item's
+    return work / sms > nb_max ? work / sms : nb_max;
+  };
+  return 4.0 * blocks(whole) <= 4.4 * blocks(full) + 14.0;
+}
+
+// Chains per tensor-core work item of every selected instance, in granules
+// of R where items hold whole reads (or R divides 128 / F), of 32 otherwise.
+// fixed = 0: as many granules as a CTA's tensor memory holds (128 / F
+// chains), halved while the batch would fill fewer CTAs than the GPU has
+// SMs.  fixed > 0: the largest multiple of the granule not above min(fixed,
+// 128 / F), at least one granule.  fixed < 0: the smallest granule any choice
+// may use (for sizing).  0 for instances left to the plain kernel.
 static std::vector<int> tc_item_sizes(int num_instances,
                                       const pysa_gb_host_tables* host,
                                       int min_n, int fixed) {
   std::vector<int> size(num_instances, 0), gran(num_instances, 32);
+  const bool whole = tc_whole_reads(num_instances, host, min_n);
   for (int i = 0; i < num_instances; ++i) {
     if (!tc_selected(host, i, min_n)) continue;
-    size[i] = tc_chains_per_cta(host->n[i]);
-    if (size[i] % host->replicas[i] == 0) gran[i] = host->replicas[i];
-    if (gran[i] > size[i]) gran[i] = size[i];
+    const int cc = tc_chains_per_cta(host->n[i]), R = host->replicas[i];
     if (fixed < 0) {
-      size[i] = gran[i];
-    } else if (fixed > 0) {
-      const int cap = fixed < size[i] ? fixed : size[i];
-      const int m = cap / gran[i] * gran[i];
-      size[i] = m > 0 ? m : gran[i];
+      size[i] = R < 32 ? R : 32;
+      continue;
     }
+    if (whole || cc % R == 0) gran[i] = R;
+    if (gran[i] > cc) gran[i] = cc;
+    const int cap = fixed > 0 && fixed < cc ? fixed : cc;
+    const int m = cap / gran[i];
+    size[i] = (m > 0 ? m : 1) * gran[i];
   }
   if (fixed != 0) return size;
   const int sms = sm_count();
@@ -407,14 +438,12 @@ static std::vector<int> tc_item_sizes(int num_instances,
       if (!size[i]) continue;
       const int64_t chains = (int64_t)host->replicas[i] * host->reads[i];
       items += (chains + size[i] - 1) / size[i];
-      const int h = size[i] / 2;
-      can |= h >= gran[i] && h % gran[i] == 0;
+      can |= size[i] > gran[i];
     }
     if (items >= sms || !can) break;
-    for (int i = 0; i < num_instances; ++i) {
-      const int h = size[i] / 2;
-      if (size[i] && h >= gran[i] && h % gran[i] == 0) size[i] = h;
-    }
+    for (int i = 0; i < num_instances; ++i)
+      if (size[i] > gran[i])
+        size[i] = (size[i] / gran[i] + 1) / 2 * gran[i];
   }
   return size;
 }
@@ -464,7 +493,8 @@ int pysa_gb_tc_setup(const pysa_gb_problems* p, const pysa_gb_host_tables* host,
   std::vector<int32_t> flags(p->num_instances, 0);
   const PlainItemPlan plan = make_item_plan();
   int64_t bo = 0, dd = 0;
-  int live = 0, fusable = 1;
+  int live = 0;
+  const int fusable = tc_whole_reads(p->num_instances, host, min_n);
   for (int i = 0; i < p->num_instances; ++i) {
     boff[i] = bo;
     doff[i] = dd;
@@ -473,7 +503,6 @@ int pysa_gb_tc_setup(const pysa_gb_problems* p, const pysa_gb_host_tables* host,
         live |= 1 << plan.variant_of(host->n[i]);
       continue;
     }
-    if (tc_chains_per_cta(host->n[i]) % host->replicas[i] != 0) fusable = 0;
     flags[i] = 1;
     bo += tc_b_elems(host->n[i], ws->tc_terms);
     dd += tc_diag_elems(host->n[i]);
