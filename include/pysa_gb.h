@@ -300,9 +300,9 @@ int pysa_gb_set_decision_mode(int32_t mode);
 
 /* Decision mode 0's switch point: a block is decided in rounds while the
  * previous block's largest flip count of a chain was at most `flips`
- * (0..64, default 12), in sequential sub-blocks otherwise.  Same decisions
- * for every value; process-wide, for launches enqueued after the call.  No
- * counterpart in the reference. */
+ * (0..64; until the first call 12, and 6 for n > 1024), in sequential
+ * sub-blocks otherwise.  Same decisions for every value; process-wide, for
+ * launches enqueued after the call.  No counterpart in the reference. */
 int pysa_gb_set_block_round_limit(int32_t flips);
 
 /* Most CTAs of a tensor-core sweep launch (0, the default: one per SM).

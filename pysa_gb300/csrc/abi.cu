@@ -54,7 +54,8 @@ static thread_local std::string g_last_error;
 static unsigned long long* g_tc_trace = nullptr;  // diagnostics, see below
 static uint64_t g_unit_wait_ns = 0;  // diagnostics: 0 = the default bound
 static int32_t g_decision_mode = 0;   // tensor-core sweep: 0 auto, 1, 2
-static int32_t g_round_limit = 12;    // mode 0: block rounds up to this
+static int32_t g_round_limit = -1;    // mode 0: block rounds up to this many
+                                      // flips; -1: by fold (tc_round_limit)
 static int32_t g_tc_max_ctas = 0;     // tensor-core launches: 0 = SM count
 
 static int fail(int code, const std::string& msg) {
@@ -73,6 +74,16 @@ static int cuda_fail(cudaError_t e, const char* where) {
 
 // Default for the most sweeps one fused tensor-core launch covers.
 constexpr int kMaxFusedSweeps = 128;
+
+// Flips of a chain up to which the next 64-spin block is decided in rounds.
+// Fold 2 shares a chain's rounds between two lanes (visiting order) and gains
+// from them longest; at fold 4 one lane tests all 64 positions, about 1400
+// cycles a round against 14000 for the block in sequential sub-blocks.
+// Measured, ms per sweep at limits 6 / 8 / 12 / 16: Wishart n = 2048 (fold 4)
+// 0.789 / 0.807 / 0.885 / 1.064; integer QUBO n = 2000 0.2069 / 0.2073 /
+// 0.2092 / 0.2124, n = 1024 (fold 2) 0.1046 / 0.1039 / 0.1041 / 0.1046, n =
+// 300 (fold 1) 0.0704 / 0.0651 / 0.0645 / 0.0644.
+static int tc_round_limit(int fold) { return fold == 4 ? 6 : 12; }
 
 // Most sweeps of one launch of the resident small sweep (about a
 // millisecond each thousand).
@@ -704,7 +715,6 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
   ta.pad_ = 0;
   ta.unit_wait_ns = g_unit_wait_ns;
   ta.decision_mode = g_decision_mode;
-  ta.round_limit = g_round_limit;
   ta.wrap = 0;
   ta.e8 = ws->tc_fp8 != 0;
   ta.sched = ws->tc_sched;
@@ -755,6 +765,8 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       ta.fuse_exchange = fuse;
       ta.advance_counter = fuse && v == last_v && !small_live;
       ta.log_omega_stride = fuse ? o->log_omega_stride : 0;
+      ta.round_limit = g_round_limit >= 0 ? g_round_limit
+                                          : tc_round_limit(folds[v]);
       e = launch_tc(ta, folds[v], random, sms, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc sweep launch");
     }
