@@ -45,8 +45,8 @@ namespace pysa_gb {
 constexpr int kTW = 256;
 
 // Decision mode of a block: block rounds (D64) while the previous block's
-// largest flip count of any chain was at most TcArgs::round_limit (default
-// 12), else sequential sub-blocks.  A round costs about as much as 6-10
+// largest flip count of any chain was at most TcArgs::round_limit (12, and 6
+// at fold 4, by default), else sequential sub-blocks.  A round costs about as much as 6-10
 // sequential spins, so the rounds win while flips are rare.
 
 // RND: random visiting order (one permutation per instance and sweep); the
@@ -376,6 +376,27 @@ __device__ __noinline__ void redo_subblock(const RedoCtx& x, uint32_t* wcur,
   *dEb = e;
 }
 
+// The exchange pass of one read with the exact rule (pysa/utils.py:44-58), out
+// of line: slot R - 1 starts with replica cb; pair k's other replica, its
+// energy and the betas' difference are in B2, E2 and D, its uniform in X.
+static __device__ __noinline__ void exact_pass(int R, int cb, const float* E,
+                                               const int32_t* B2,
+                                               const float* E2,
+                                               const float* D,
+                                               const uint32_t* X,
+                                               int32_t* B) {
+  float ce = E[cb];
+  for (int k = 0; k < R - 1; ++k) {
+    const int b2 = B2[k];
+    const float e2 = E2[k];
+    const bool sw = pt_accept(__fmul_rn(__fsub_rn(ce, e2), D[k]), X[k]);
+    B[R - k - 1] = sw ? b2 : cb;
+    cb = sw ? cb : b2;
+    ce = sw ? ce : e2;
+  }
+  B[0] = cb;
+}
+
 // Log-omega of an item's reads (pysa/ais.py:79-112), a warp per read: terms
 // of the sorted ladder from f32 products, summed in f64.  E: the chains'
 // energies.  Out of line: it runs only with get_part_fun, and inlined it
@@ -473,6 +494,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
   int32_t* ex_B2 = reinterpret_cast<int32_t*>(dl_s + 17 * CC);
   float* ex_E2 = dl_s + 21 * CC;
   float* ex_D = dl_s + 25 * CC;
+  float* ex_H = dl_s + 29 * CC;  // accept from here on ([4][CC])
   const uint32_t smem_base = smem_addr(smem);
   // A operand: physical row m, and the element of position j (< 64) of a
   // row set to +-1 (QUBO) or +-2 (Ising) deltas
@@ -1687,6 +1709,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
           int32_t* B = ex_B + warp * CC;
           uint32_t* X = ex_X + warp * CC;
           float* Lx = ex_L + warp * CC;
+          float* Hx = ex_H + warp * CC;
           float* Bt = ex_T + warp * CC;
           for (int k = lane; k < R; k += 32) Bt[k] = betas[k];
           for (int r = warp; r < nreads; r += 4) {
@@ -1699,7 +1722,11 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 const uint32_t x = draw1(a.seed, TAG_PT, (uint32_t)inst, sweep,
                                          lread, (uint32_t)k);
                 X[k] = x;
-                Lx[k] = log_uniform_f32(x);
+                // log u and its band (pt_accept_lf)
+                const float lf = log_uniform_f32(x);
+                const float m = fmaf(2e-6f, fabsf(lf), 3.1e-5f);
+                Lx[k] = lf - m;
+                Hx[k] = fminf(lf + m, 0.0f);
               }
             }
             __syncwarp();
@@ -1721,18 +1748,29 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             }
             __syncwarp();
             if (lane == 0 && R > 1) {
-              int cb = B[R - 1];
+              // without branches: accept at de >= hi, reject below lo; a pair
+              // in between (the exact rule's) has the pass made again.  The
+              // pass ends every sweep with all roles waiting: with a branch
+              // per test it took about 100 cycles a pair (sk128, R = 32: 26.5
+              // -> 25.9 ms per 1000 sweeps; QUBO 1024, R = 64: 51.0 -> 50.0
+              // ms per 500)
+              const int cb0 = B[R - 1];
+              int cb = cb0;
               float ce = E[cb];
+              uint32_t unsure = 0u;
+#pragma unroll 4
               for (int k = 0; k < R - 1; ++k) {
                 const int b2 = B2[k];
                 const float e2 = E2[k];
                 const float de = __fmul_rn(__fsub_rn(ce, e2), Dk[k]);
-                const bool sw = pt_accept_lf(de, Lx[k], X[k]);
+                const bool sw = de >= Hx[k];
+                unsure |= (!sw && !(de < Lx[k])) ? 1u : 0u;
                 B[R - k - 1] = sw ? b2 : cb;   // final: no later pair
                 cb = sw ? cb : b2;
                 ce = sw ? ce : e2;
               }
               B[0] = cb;
+              if (unsure) exact_pass(R, cb0, E, B2, E2, Dk, X, B);
             }
             __syncwarp();
             for (int k = lane; k < R; k += 32) {
