@@ -708,6 +708,7 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
   ta.tc_b = ws->tc_b;
   ta.tc_diag = ws->tc_diag;
   ta.seed = o->seed;
+  ta.keys = philox_keys(o->seed);
   ta.recompute_every = o->recompute_every;
   ta.use_pt = o->use_pt;
   ta.exchange_every = o->exchange_every;
@@ -854,11 +855,7 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
   ca.seed = o->seed;
   ca.width = ws->csr_width;
   ca.pad_ = 0;
-  for (int r = 0; r < 10; ++r) {
-    ca.round_keys[2 * r] = (uint32_t)o->seed + (uint32_t)r * 0x9E3779B9u;
-    ca.round_keys[2 * r + 1] =
-        (uint32_t)(o->seed >> 32) + (uint32_t)r * 0xBB67AE85u;
-  }
+  ca.keys = philox_keys(o->seed);
   for (int sw = 0; sw < num_sweeps; ++sw) {
     if (use_tc && (phases & 1)) {
       if (random) {

@@ -51,6 +51,41 @@ __device__ __forceinline__ void draw4(uint64_t seed, uint32_t tag,
                 (uint32_t)(seed >> 32), out);
 }
 
+// The ten round keys of a seed, k0 and k1 in turn.  As kernel parameters they
+// are constant operands of the rounds' logic instructions.
+struct PhiloxKeys {
+  uint32_t k[20];
+};
+inline PhiloxKeys philox_keys(uint64_t seed) {
+  PhiloxKeys r;
+  for (int i = 0; i < 10; ++i) {
+    r.k[2 * i] = (uint32_t)seed + (uint32_t)i * 0x9E3779B9u;
+    r.k[2 * i + 1] = (uint32_t)(seed >> 32) + (uint32_t)i * 0xBB67AE85u;
+  }
+  return r;
+}
+
+// draw4 with the round keys given.
+__device__ __forceinline__ void draw4_keys(const PhiloxKeys& keys,
+                                           uint32_t tag, uint32_t inst,
+                                           uint32_t a, uint32_t b, uint32_t q,
+                                           uint32_t out[4]) {
+  uint32_t c0 = q, c1 = a, c2 = b, c3 = (inst << 4) | tag;
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c0;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
+    c0 = (uint32_t)(p1 >> 32) ^ c1 ^ keys.k[2 * r];
+    c1 = (uint32_t)p1;
+    c2 = (uint32_t)(p0 >> 32) ^ c3 ^ keys.k[2 * r + 1];
+    c3 = (uint32_t)p0;
+  }
+  out[0] = c0;
+  out[1] = c1;
+  out[2] = c2;
+  out[3] = c3;
+}
+
 // Key of chain `chain`'s sweep stream: the seed, changed by the chain's
 // stream key when one is set (see pysa_gb_state.stream_key).
 __device__ __forceinline__ uint64_t chain_seed(uint64_t seed,

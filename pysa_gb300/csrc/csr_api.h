@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pysa_gb.h"
+#include "common.cuh"
 
 namespace pysa_gb {
 
@@ -23,7 +24,7 @@ struct CsrArgs {
   uint64_t seed;
   int32_t width;  // 0: grouped rows; 4/8/16/32: fixed records
   int32_t pad_;
-  uint32_t round_keys[20];  // Philox round keys of seed: k0, k1 per round
+  PhiloxKeys keys;  // of seed
 };
 
 // The level schedule of every sparse instance's visiting order, written into

@@ -301,28 +301,6 @@ struct QuadSlab {
   static constexpr int PER_LANE = (4 * PIECES + 31) / 32;
 };
 
-// Philox4x32-10 with the ten round keys in kernel parameters (constant
-// operands of the rounds' logic instructions): draws 4 q .. 4 q + 3 of the
-// sweep stream of chain `b`.
-__device__ __forceinline__ void draw4_keys(const CsrArgs& a, uint32_t inst,
-                                           uint32_t sweep, uint32_t b,
-                                           uint32_t q, uint32_t out[4]) {
-  uint32_t c0 = q, c1 = sweep, c2 = b, c3 = (inst << 4) | TAG_SWEEP;
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const uint64_t p0 = (uint64_t)0xD2511F53u * c0;
-    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
-    c0 = (uint32_t)(p1 >> 32) ^ c1 ^ a.round_keys[2 * r];
-    c1 = (uint32_t)p1;
-    c2 = (uint32_t)(p0 >> 32) ^ c3 ^ a.round_keys[2 * r + 1];
-    c3 = (uint32_t)p0;
-  }
-  out[0] = c0;
-  out[1] = c1;
-  out[2] = c2;
-  out[3] = c3;
-}
-
 // 32 x 32 bit transpose over a warp: lane l's bit b becomes lane b's bit l.
 __device__ __forceinline__ uint32_t warp_transpose(uint32_t v, int lane) {
 #pragma unroll
@@ -452,7 +430,7 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
       draw4(chain_seed(a.seed, valid ? a.s.stream_key : nullptr, chain),
             TAG_SWEEP, (uint32_t)inst, sweep, cl, (uint32_t)q, x);
     else
-      draw4_keys(a, (uint32_t)inst, sweep, cl, (uint32_t)q, x);
+      draw4_keys(a.keys, TAG_SWEEP, (uint32_t)inst, sweep, cl, (uint32_t)q, x);
 #pragma unroll
     for (int k = 0; k < 4; ++k) ft.at(x[k], tl[k], th[k]);
   };

@@ -98,9 +98,9 @@ struct TcCfg {
   static constexpr bool HELP = F == 2;
   // F == 4: the three idle slices' warps write the A rows of sub-blocks 0-2
   static constexpr bool APUT = F == 4;
-  // F == 2, visiting order: block rounds run on all four decision warps,
-  // two lanes per chain (the other slice's warps would idle)
-  static constexpr bool PAIRS = F == 2 && !RND;
+  // F == 2: block rounds run on all four decision warps, two lanes per chain
+  // (the other slice's warps would idle)
+  static constexpr bool PAIRS = F == 2;
   // 1 / (beta scale) of each chain (+inf for beta <= 0), kept with beta_s
   static constexpr size_t INVB_OFF = BETA_OFF + CC * 4;
   static constexpr size_t CORR_OFF = INVB_OFF + CC * 4;
@@ -117,7 +117,11 @@ struct TcCfg {
   // by the log-uniform helper warps
   static constexpr size_t POSB_OFF = PERM_OFF + PERM_BYTES;
   static constexpr size_t POSB_BYTES = RND ? (size_t)2 * 2 * CC * 4 : 0;
-  static constexpr size_t BAR_OFF = (POSB_OFF + POSB_BYTES + 63) / 64 * 64;
+  // RND, F > 1: per decision warp, the block's columns in its slice and their
+  // positions (position << 16 | column), up to 64 and padding
+  static constexpr size_t NEED_OFF = (POSB_OFF + POSB_BYTES + 15) / 16 * 16;
+  static constexpr size_t NEED_BYTES = (RND && F > 1) ? (size_t)4 * 64 * 4 : 0;
+  static constexpr size_t BAR_OFF = (NEED_OFF + NEED_BYTES + 63) / 64 * 64;
   // a_full, mma_done, h_ready, jbb_full[2], jbb_free[2], rc_full, rc_done,
   // lf_full[2], lf_free[2], full[NS], free[NS], drain, mma_done_b[2]
   static constexpr int NBARS = 16 + 2 * NS;
@@ -835,36 +839,46 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
           // warp's copy (same address in every lane: a broadcast load)
           auto spos = [&](int k) { return perm_s[warp * 64 + k]; };
           if constexpr (RND && F > 1) {
-            // every decision warp copies the block's fields held in its own
-            // slice (TMEM lanes belong to warps) into hbuf[k][chain]
+            // Every decision warp copies the block's fields held in its own
+            // slice (TMEM lanes belong to warps) into hbuf[k][chain].  The
+            // slice's columns are listed first, so that the loads run 16 at
+            // a time with no branch between them (fold 2: 6.3k -> 1.1k cycles
+            // a block; reading the whole slice 64 columns at a time and
+            // picking took 12k).
+            uint32_t* need =
+                reinterpret_cast<uint32_t*>(smem + C::NEED_OFF) + warp * 64;
+            const uint32_t in0 = __ballot_sync(0xffffffffu, ps0 == q);
+            const uint32_t in1 = __ballot_sync(0xffffffffu, ps1 == q);
+            const int cnt = __popc(in0) + __popc(in1);
+            const uint32_t lt = (1u << lane) - 1u;
+            if (ps0 == q)
+              need[__popc(in0 & lt)] = ((uint32_t)lane << 16) | (uint32_t)pc0;
+            if (ps1 == q)
+              need[__popc(in0) + __popc(in1 & lt)] =
+                  ((uint32_t)(32 + lane) << 16) | (uint32_t)pc1;
+            __syncwarp();
             bool hok = !*sh.abort;
             if (hok && wait_h)
               hok = tc_wait(sh.h_ready, (Gb - 1) & 1, sh, status);
             hok = __all_sync(0xffffffffu, hok);
             if (hok) {
               tc::fence_after_sync();
-              for (int k0 = 0; k0 < 64; k0 += 16) {
-                uint32_t r[16];
-                int mine = 0;  // bit kk: position k0 + kk lives in my slice
+              for (int i0 = 0; i0 < cnt; i0 += 16) {
+                uint32_t w[16], r[16];
 #pragma unroll
-                for (int kk = 0; kk < 16; ++kk) {
-                  const int k = k0 + kk;
-                  const int sl =
-                      __shfl_sync(0xffffffffu, k < 32 ? ps0 : ps1, k & 31);
-                  const int col =
-                      __shfl_sync(0xffffffffu, k < 32 ? pc0 : pc1, k & 31);
-                  r[kk] = 0u;
-                  if (sl == q) {
-                    r[kk] = tc::tmem_ld1_nowait(taddr + lane_base +
-                                                (uint32_t)col);
-                    mine |= 1 << kk;
-                  }
+                for (int e = 0; e < 16; ++e)  // the last one again past the end
+                  w[e] = need[i0 + e < cnt ? i0 + e : cnt - 1];
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                  r[e] = tc::tmem_ld1_nowait(taddr + lane_base +
+                                             (w[e] & 0xFFFFu));
+                tc::tmem_wait_ld16(r);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                  const int k = (int)(w[e] >> 16);
+                  hbuf[k * CC + c] = __uint_as_float(r[e]);
                 }
-                tc::tmem_wait_ld();
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk)
-                  if ((mine >> kk) & 1)
-                    hbuf[(k0 + kk) * CC + c] = __uint_as_float(r[kk]);
               }
             }
             named_sync_128();
@@ -889,15 +903,17 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             const int hf = lane >> 4;
             const int cc =
                 8 * (((lane >> 3) & 1) ? 7 - warp : warp) + (lane & 7);
+            // In random order the gather above has left the fields in hbuf
+            // ([64][chain]) and the spins by position are in posb.
             bool ok = !*sh.abort;
-            if (ok && q == qt && wait_h)
+            if (!RND && ok && q == qt && wait_h)
               ok = tc_wait(sh.h_ready, (Gb - 1) & 1, sh, status);
             if (ok) ok = tc_wait(&sh.jbb_full[Gb & 1], (Gb >> 1) & 1, sh, status);
             if (ok) ok = tc_wait(&sh.lf_full[Gb & 1], (Gb >> 1) & 1, sh, status);
             ok = __all_sync(0xffffffffu, ok);
             if (L == 0) stamp(a, Gb, 0);
             if (L == 0) stamp(a, Gb, 1);
-            if (ok && q == qt) {
+            if (!RND && ok && q == qt) {
               tc::fence_after_sync();
               float hl[64];
               tc::tmem_ld64(taddr + lane_base + co, hl);
@@ -907,15 +923,17 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                     make_float4(hl[4 * q4], hl[4 * q4 + 1], hl[4 * q4 + 2],
                                 hl[4 * q4 + 3]);
             }
-            named_sync_128();  // the fields are in dl_s
+            if (!RND) named_sync_128();  // the fields are in dl_s
             if (L == 0) stamp(a, Gb, 8);
             ok = __all_sync(0xffffffffu, ok && !*sh.abort);
             if (ok) {
               const bool pvalid = cc < item.nchains;
               const float* jb = jbb + (Gb & 1) * 4096;
               const float* lfb = lf_s + (Gb & 1) * 64 * CC;
-              const uint32_t o0 = spins_s[(2 * t) * CC + cc];
-              const uint32_t o1 = spins_s[(2 * t + 1) * CC + cc];
+              const uint32_t o0 = RND ? posb[((Gb & 1) * 2 + 0) * CC + cc]
+                                      : spins_s[(2 * t) * CC + cc];
+              const uint32_t o1 = RND ? posb[((Gb & 1) * 2 + 1) * CC + cc]
+                                      : spins_s[(2 * t + 1) * CC + cc];
               const uint32_t om = hf ? o1 : o0;  // this lane's half
               const float pbeta = beta_s[cc];
               const float scale = ising ? 2.0f : 1.0f;
@@ -924,14 +942,21 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
               const float band0 = banded ? 3e-5f * invbs : 0.0f;
               const float band1 = banded ? 1e-6f * invbs : 0.0f;
               float h[32], w[32];
+              if constexpr (RND) {
 #pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4) {
-                const float4 v = *reinterpret_cast<const float4*>(
-                    dl_s + cidx(cc, 32 * hf + 4 * q4));
-                h[4 * q4 + 0] = v.x;
-                h[4 * q4 + 1] = v.y;
-                h[4 * q4 + 2] = v.z;
-                h[4 * q4 + 3] = v.w;
+                for (int k = 0; k < 32; ++k)  // positions past n hold nothing
+                  h[k] = 32 * hf + k < kmax ? hbuf[(32 * hf + k) * CC + cc]
+                                            : 0.0f;
+              } else {
+#pragma unroll
+                for (int q4 = 0; q4 < 8; ++q4) {
+                  const float4 v = *reinterpret_cast<const float4*>(
+                      dl_s + cidx(cc, 32 * hf + 4 * q4));
+                  h[4 * q4 + 0] = v.x;
+                  h[4 * q4 + 1] = v.y;
+                  h[4 * q4 + 2] = v.z;
+                  h[4 * q4 + 3] = v.w;
+                }
               }
 #pragma unroll
               for (int q4 = 0; q4 < 8; ++q4) {
@@ -1071,7 +1096,18 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 }
               }
               if (pvalid) {
-                spins_s[(2 * t + hf) * CC + cc] = om ^ fm;
+                if constexpr (RND) {
+                  // flips back to the scattered spins (the chain's other
+                  // lane may flip bits of the same word)
+                  uint32_t fb = fm;
+                  while (fb) {
+                    const int sp = spos(32 * hf + __ffs(fb) - 1);
+                    fb &= fb - 1u;
+                    atomicXor(spins_s + (sp >> 5) * CC + cc, 1u << (sp & 31));
+                  }
+                } else {
+                  spins_s[(2 * t + hf) * CC + cc] = om ^ fm;
+                }
                 if (hf == 0) dE_s[cc] += (double)dEb;
               }
               blk_mf = __reduce_max_sync(
@@ -1169,6 +1205,24 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             // bit k: position k of the block flipped (chains the CTA holds,
             // positions < kmax)
             uint64_t bflips = 0ull;
+            // random order, fold 1: the fields of positions k0 ... k0 + 15,
+            // single columns of this thread's lane (column 0 stands in past
+            // the end: no branch between the loads)
+            auto load_scattered = [&](int k0, float* out) {
+              uint32_t r[16];
+              int sp[16];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) sp[j] = spos(k0 + j);
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                r[j] = tc::tmem_ld1_nowait(taddr + lane_base +
+                                           (uint32_t)(sp[j] < 0 ? 0 : sp[j]));
+              tc::tmem_wait_ld16(r);
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                out[j] = k0 + j < kmax ? __uint_as_float(r[j]) : 0.0f;
+            };
             // fields of sub-block g with the corrections of every earlier
             // sub-block of the block
             auto fields = [&](int g, float* hs) {
@@ -1180,18 +1234,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                   hs[j] = 16 * g + j < kmax ? hbuf[(16 * g + j) * CC + c]
                                             : 0.0f;
               } else {
-                uint32_t r[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  const int sp = spos(16 * g + j);
-                  r[j] = 0u;
-                  if (sp >= 0)
-                    r[j] = tc::tmem_ld1_nowait(taddr + lane_base +
-                                               (uint32_t)sp);
-                }
-                tc::tmem_wait_ld16(r);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) hs[j] = __uint_as_float(r[j]);
+                load_scattered(16 * g, hs);
               }
               if (lead) stamp(a, Gb, 8 + 3 * g);
               // sub-blocks before the previous one: precomputed by the
@@ -1257,20 +1300,8 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 for (int k = 0; k < 64; ++k)
                   h[k] = k < kmax ? hbuf[k * CC + c] : 0.0f;
               } else {
-                uint32_t r[16];
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-#pragma unroll
-                  for (int j = 0; j < 16; ++j) {
-                    const int sp = spos(16 * g + j);
-                    r[j] = 0u;
-                    if (sp >= 0)
-                      r[j] = tc::tmem_ld1_nowait(taddr + lane_base + (uint32_t)sp);
-                  }
-                  tc::tmem_wait_ld16(r);
-#pragma unroll
-                  for (int j = 0; j < 16; ++j) h[16 * g + j] = __uint_as_float(r[j]);
-                }
+                for (int g = 0; g < 4; ++g) load_scattered(16 * g, h + 16 * g);
               }
               if (lead) stamp(a, Gb, 8);
               // the block's fields as loaded (a candidate's field at its
@@ -2076,26 +2107,25 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             for (int it = hid; it < CC * 16; it += 64) {
               const int c2 = it % CC, quad = it / CC;
               const uint32_t cl = (uint32_t)(item.chain0 + c2 - chain_base);
-              const uint64_t sk =
-                  c2 < item.nchains
-                      ? chain_seed(a.seed, a.s.stream_key, item.chain0 + c2)
-                      : a.seed;
               uint32_t x[4];
-              draw4(sk, TAG_SWEEP, (uint32_t)inst, sweep, cl,
-                    (uint32_t)(16 * t + quad), x);
+              if (a.s.stream_key && c2 < item.nchains)
+                draw4(chain_seed(a.seed, a.s.stream_key, item.chain0 + c2),
+                      TAG_SWEEP, (uint32_t)inst, sweep, cl,
+                      (uint32_t)(16 * t + quad), x);
+              else
+                draw4_keys(a.keys, TAG_SWEEP, (uint32_t)inst, sweep, cl,
+                           (uint32_t)(16 * t + quad), x);
               // a = log u - m: the rejection bound in the log domain, m =
               // 3e-5 + 1e-6 |log u| the band of the f32 log (over three
-              // times the error of __logf plus the roundings of a
-              // threshold); the deciders scale it by 1 / (beta scale)
+              // times its error plus the roundings of a threshold); log u <
+              // 0, so a is linear in log2 u.  The deciders scale it by
+              // 1 / (beta scale)
+              constexpr float kLn2 = 0.69314718056f * 1.000001f;
               float4 v;
-              v.x = log_uniform_f32(x[0]);
-              v.y = log_uniform_f32(x[1]);
-              v.z = log_uniform_f32(x[2]);
-              v.w = log_uniform_f32(x[3]);
-              v.x -= fmaf(1e-6f, fabsf(v.x), 3e-5f);
-              v.y -= fmaf(1e-6f, fabsf(v.y), 3e-5f);
-              v.z -= fmaf(1e-6f, fabsf(v.z), 3e-5f);
-              v.w -= fmaf(1e-6f, fabsf(v.w), 3e-5f);
+              v.x = fmaf(kLn2, log2_uniform(x[0]), -3e-5f);
+              v.y = fmaf(kLn2, log2_uniform(x[1]), -3e-5f);
+              v.z = fmaf(kLn2, log2_uniform(x[2]), -3e-5f);
+              v.w = fmaf(kLn2, log2_uniform(x[3]), -3e-5f);
               *reinterpret_cast<float4*>(out + cidx(c2, 4 * quad)) = v;
             }
           }
@@ -2108,20 +2138,32 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             if (go && Gs > G0 && Gb - Gs <= 1)
               go = tc_wait(&sh.lf_free[(Gs - 1) & 1], ((Gs - 1) >> 1) & 1, sh,
                            status);
-            if (go) {
+            if (__all_sync(0xffffffffu, go)) {
               const int32_t* pr =
                   a.perm + ((int64_t)(sweep % (uint32_t)a.perm_slots) *
                                 a.p.num_instances + inst) * a.p.max_n +
                   64 * t;
               const int kmax = n - 64 * t < 64 ? n - 64 * t : 64;
-              for (int c2 = hid; c2 < CC; c2 += 64) {
+              // lane l holds the spins at positions l and 32 + l; a warp's
+              // lanes take the same one by shuffle, so the spin words' loads
+              // of a group run together
+              const int pa = lane < kmax ? pr[lane] : 0;
+              const int pb = 32 + lane < kmax ? pr[32 + lane] : 0;
+              for (int c0 = 32 * (warp - 6); c0 < CC; c0 += 64) {
+                const int c2 = c0 + lane;
                 uint32_t w0 = 0u, w1 = 0u;
-                for (int k = 0; k < kmax; ++k) {
-                  const int sp = pr[k];
-                  const uint32_t bit =
-                      (spins_s[(sp >> 5) * CC + c2] >> (sp & 31)) & 1u;
-                  if (k < 32) w0 |= bit << k; else w1 |= bit << (k - 32);
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k) {
+                  const int s0 = __shfl_sync(0xffffffffu, pa, k);
+                  const int s1 = __shfl_sync(0xffffffffu, pb, k);
+                  w0 |= ((spins_s[(s0 >> 5) * CC + c2] >> (s0 & 31)) & 1u)
+                        << k;
+                  w1 |= ((spins_s[(s1 >> 5) * CC + c2] >> (s1 & 31)) & 1u)
+                        << k;
                 }
+                // positions past the end hold no spin
+                if (kmax < 64) w1 &= kmax > 32 ? (1u << (kmax - 32)) - 1u : 0u;
+                if (kmax < 32) w0 &= (1u << kmax) - 1u;
                 posb[((Gb & 1) * 2 + 0) * CC + c2] = w0;
                 posb[((Gb & 1) * 2 + 1) * CC + c2] = w1;
               }

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pysa_gb.h"
+#include "common.cuh"
 
 namespace pysa_gb {
 
@@ -24,6 +25,7 @@ struct TcArgs {
   const float* tc_diag;
   const TcItem* items;
   uint64_t seed;
+  PhiloxKeys keys;          // of seed
   int32_t recompute_every;  // >0: H and E rebuilt when sweep % this == 0
   int32_t num_items;        // items of this fold
   int32_t unit_sweeps;      // sweeps per work unit (wrap: of the launch)
