@@ -601,38 +601,73 @@ void launch_exchange(const XArgs& a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------- visiting orders
-// Fisher-Yates for (instance, sweep): j = floor(x (i+1) / 2^32); draws made
-// in parallel, swaps by one thread.  Block per instance.
-__global__ void k_perm(const PermArgs a) {
-  extern __shared__ int32_t sh[];
+// Fisher-Yates for (instance, sweep): for i from n - 1 down to 1 swap places i
+// and j_i = floor(x_i (i + 1) / 2^32).  Block per instance.
+//
+// The swaps run in rounds instead of one after another: in a round every
+// swap still to do claims its two places, the one that comes first in the
+// sequence (the largest i) winning each, and the swaps holding both claims
+// are done.  A swap waits exactly for the earlier ones that share a place
+// with it, so the order is the sequential one; the rounds are about 3 log2 n
+// (Shun, Gu, Blelloch, Fineman and Gibbons, "Sequential random permutation,
+// list contraction and tree contraction are highly parallel", SODA 2015).
+// Claims of a round outrank those of earlier ones, so none is cleared.
+// Measured (one thread swapping before): n = 1024, 16 orders 38 -> 12 us; n =
+// 4096 150 -> 20 us.
+constexpr int kPermSmem = 232448;
+
+__global__ void __launch_bounds__(1024) k_perm(const PermArgs a) {
+  extern __shared__ uint32_t sh[];
   const int inst = blockIdx.x;
   const int n = a.p.n[inst];
   // grid row y: the sweep y after the current one (orders made ahead)
   const uint32_t sweep = (uint32_t)(*a.sweep_counter) + blockIdx.y;
-  int32_t* p = sh;
-  uint32_t* x = reinterpret_cast<uint32_t*>(sh + a.p.max_n);
+  uint32_t* claim = sh;                                           // [max_n]
+  uint16_t* p = reinterpret_cast<uint16_t*>(claim + a.p.max_n);   // [max_n]
+  uint16_t* js = p + a.p.max_n;                                   // [max_n]
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    p[i] = i;
-    x[i] = draw1(a.seed, TAG_PERM, (uint32_t)inst, sweep, 0u, (uint32_t)i);
+    const uint32_t x =
+        draw1(a.seed, TAG_PERM, (uint32_t)inst, sweep, 0u, (uint32_t)i);
+    p[i] = (uint16_t)i;
+    js[i] = (uint16_t)(((uint64_t)x * (uint64_t)(i + 1)) >> 32);
+    claim[i] = 0u;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = n - 1; i > 0; --i) {
-      const int j = (int)(((uint64_t)x[i] * (uint64_t)(i + 1)) >> 32);
-      const int32_t t = p[i];
-      p[i] = p[j];
-      p[j] = t;
+  // bit k of todo: swap threadIdx.x + k blockDim.x is still to do
+  uint32_t todo = 0u;
+  for (int k = 0; k < 32; ++k) {
+    const int i = (int)threadIdx.x + k * (int)blockDim.x;
+    if (i > 0 && i < n) todo |= 1u << k;
+  }
+  for (uint32_t round = 1;; ++round) {
+    for (uint32_t b = todo; b; b &= b - 1u) {
+      const int i = (int)threadIdx.x + (__ffs(b) - 1) * (int)blockDim.x;
+      const uint32_t c = (round << 16) | (uint32_t)i;
+      atomicMax(claim + i, c);
+      atomicMax(claim + js[i], c);
     }
+    __syncthreads();
+    for (uint32_t b = todo; b; b &= b - 1u) {
+      const int k = __ffs(b) - 1;
+      const int i = (int)threadIdx.x + k * (int)blockDim.x, j = js[i];
+      const uint32_t c = (round << 16) | (uint32_t)i;
+      if (claim[i] == c && claim[j] == c) {
+        const uint16_t t = p[i];
+        p[i] = p[j];
+        p[j] = t;
+        todo &= ~(1u << k);
+      }
+    }
+    if (!__syncthreads_or(todo != 0u)) break;
   }
-  __syncthreads();
   int32_t* out = a.perm + ((int64_t)(sweep % (uint32_t)a.perm_slots) *
                                a.p.num_instances + inst) * (int64_t)a.p.max_n;
   for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = p[i];
 }
 
 // The same orders for instances too wide for k_perm's shared memory (up to
-// 65536 spins): the draws are staged in the output row, the positions held
-// as 16-bit values in shared memory.
+// 65536 spins), one swap after another: the draws are staged in the output
+// row, the positions held as 16-bit values in shared memory.
 __global__ void k_perm_wide(const PermArgs a) {
   extern __shared__ uint16_t pw[];
   const int inst = blockIdx.x;
@@ -660,22 +695,26 @@ __global__ void k_perm_wide(const PermArgs a) {
 }
 
 void launch_perm(const PermArgs& a, cudaStream_t st, int count) {
-  const size_t sm = sizeof(int32_t) * 2 * (size_t)a.p.max_n;
+  // claims, places and partners: 8 bytes per spin, up to n = 29 056 (and 32
+  // swaps per thread)
+  const size_t sm = 8 * (size_t)a.p.max_n;
   dim3 grid((unsigned)a.p.num_instances, (unsigned)(count > 0 ? count : 1));
-  if (sm <= 48 * 1024) {
-    k_perm<<<grid, 256, sm, st>>>(a);
-    return;
-  }
-  const size_t smw = sizeof(uint16_t) * (size_t)a.p.max_n;  // <= 128 KB
   static bool attr[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr[dev]) {
+    cudaFuncSetAttribute(k_perm, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kPermSmem);
     cudaFuncSetAttribute(k_perm_wide,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(uint16_t) * PYSA_GB_MAX_N));
     attr[dev] = true;
   }
+  if (sm <= (size_t)kPermSmem) {
+    k_perm<<<grid, a.p.max_n <= 2048 ? 512 : 1024, sm, st>>>(a);
+    return;
+  }
+  const size_t smw = sizeof(uint16_t) * (size_t)a.p.max_n;  // <= 128 KB
   k_perm_wide<<<grid, 256, smw, st>>>(a);
 }
 

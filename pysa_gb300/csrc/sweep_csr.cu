@@ -197,21 +197,44 @@ __global__ void __launch_bounds__(kSchedThreads)
         tb = cut ? (int)first[u] : 4 * u;
         te = cut ? (int)first[u + 1] : (4 * u + 4 < n ? 4 * u + 4 : n);
       }
+      // the units of the spins that this one reads, the first kDeps of them
+      // kept in registers over the rounds (all for rows of 4 entries)
+      constexpr int kDeps = 16;
+      int dep[kDeps], nd = 0;
+#pragma unroll
+      for (int d = 0; d < kDeps; ++d) dep[d] = u;  // itself: no dependence
+      if (a.width == 4) {
+#pragma unroll
+        for (int d = 0; d < kDeps; ++d) {
+          const int t = tb + (d >> 2);
+          if (t < te)
+            dep[d] = unit_of(pos_of(
+                column((int64_t)4 * spin_at(t) + (d & 3))));
+        }
+        nd = kDeps;
+      }
       for (;;) {
         bool up = false;
         int m = 0;
-        for (int t = tb; t < te; ++t) {
-          int64_t e, e1;
-          for (entries(spin_at(t), e, e1); e < e1; ++e) {
-            const int uc = unit_of(pos_of(column(e)));
-            if (uc < u) {
-              m = max(m, lev[uc] + 1);
-            } else if (uc > u && lev[uc] <= lev[u]) {
-              // a later unit may flip a spin that this one reads: the rows
-              // name it also where the other row lacks the entry
-              atomicMax(const_cast<int32_t*>(lev) + uc, lev[u] + 1);
-              up = true;
-            }
+        auto meet = [&](int uc) {
+          if (uc < u) {
+            m = max(m, lev[uc] + 1);
+          } else if (uc > u && lev[uc] <= lev[u]) {
+            // a later unit may flip a spin that this one reads: the rows
+            // name it also where the other row lacks the entry
+            atomicMax(const_cast<int32_t*>(lev) + uc, lev[u] + 1);
+            up = true;
+          }
+        };
+        if (nd) {
+          if (u < nu)
+#pragma unroll
+            for (int d = 0; d < kDeps; ++d) meet(dep[d]);
+        } else {
+          for (int t = tb; t < te; ++t) {
+            int64_t e, e1;
+            for (entries(spin_at(t), e, e1); e < e1; ++e)
+              meet(unit_of(pos_of(column(e))));
           }
         }
         if (u < nu && m > lev[u]) {
