@@ -395,23 +395,6 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
   }
 }
 
-// Two f32 multiply-adds at once (each lane of the pair rounded as fmaf).
-__device__ __forceinline__ uint64_t fma2(uint64_t x, uint64_t y, uint64_t z) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
-  return d;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float half2(uint64_t v, bool hi) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return hi ? b : a;
-}
-
 // Two pairs from shared memory.  Volatile: the couplings never change, and
 // unrolled code would otherwise try to keep all of them in registers.
 __device__ __forceinline__ ulonglong2 load_pairs(uint32_t addr) {

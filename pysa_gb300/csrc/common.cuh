@@ -346,4 +346,26 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Two f32 multiply-adds at once (each lane of the pair rounded as fmaf).
+__device__ __forceinline__ uint64_t fma2(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float half2(uint64_t v, bool hi) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return hi ? b : a;
+}
+
 }  // namespace pysa_gb

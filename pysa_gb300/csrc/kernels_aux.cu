@@ -119,8 +119,10 @@ __global__ void __launch_bounds__(32 * kFieldWarps)
 // x 32 TC columns) and walks the n rows 32 at a time: the J tile (cp.async,
 // double-buffered) is read once per CH chains instead of once per chain, and
 // the chains' spins become +-1 / 0 multipliers in shared memory, so a row is
-// one shared load and two broadcasts per 8 TC multiply-adds.  Bound by those
-// shared loads (three 16-byte ones per 32 multiply-adds); a warp of f64
+// one shared load and two broadcasts per 8 TC multiply-adds, done two at a
+// time (f32x2 over pairs of chains: half the issue slots, which were two
+// thirds taken).  Bound by the shared loads (three 16-byte ones per 16 paired
+// multiply-adds) and the multiply-adds themselves; a warp of f64
 // instructions takes about 64 times the cycles of an f32 one on this GPU, so
 // f64 is kept out of the loop by adding each 32-row partial sum into an f32
 // pair with an exact two-sum.  The pair holds the sum of the partial sums to
@@ -130,10 +132,10 @@ __global__ void __launch_bounds__(32 * kFieldWarps)
 // decades).  A cluster of up to 8 CTAs splits the columns while there are too
 // few chains to fill the GPU; its energies meet in rank 0 through distributed
 // shared memory.
-// Measured against one CTA per chain with f64 accumulation: n = 2048, 9728
-// chains 14.2 -> 2.7 ms; n = 777, 9728 chains 2.92 -> 0.55 ms; n = 1000, 4096
-// chains 0.97 -> 0.37 ms; n = 64, 20000 chains 0.139 -> 0.052 ms; n = 912,
-// 100 chains 0.24 -> 0.064 ms (times with the launch).
+// Measured: n = 2048, 8192 chains 2.6 -> 1.87 ms; n = 1024, 16384 chains
+// 1.3 -> 0.96; n = 512, 65536 chains 1.19 -> 0.95 (single multiply-adds before;
+// one CTA per chain with f64 accumulation took 14.2 ms at n = 2048, 9728
+// chains, this tile 2.7 with single multiply-adds).
 
 // s + e = a + b exactly (Knuth's two-sum).
 __device__ __forceinline__ float two_sum(float a, float b, float& e) {
@@ -148,6 +150,19 @@ __device__ __forceinline__ void pair_add(float2& p, float x) {
   float e;
   p.x = two_sum(p.x, x, e);
   p.y += e;
+}
+
+// The same for two pairs at once: hi, lo and x hold two f32 each.  The
+// differences are multiply-adds by -1 (the product is exact).
+__device__ __forceinline__ void pair_add2(uint64_t& hi, uint64_t& lo,
+                                          uint64_t x) {
+  const uint64_t m1 = pack2(-1.0f, -1.0f);
+  const uint64_t s = add2(hi, x);
+  const uint64_t bb = fma2(hi, m1, s);
+  const uint64_t ea = fma2(fma2(bb, m1, s), m1, hi);
+  const uint64_t eb = fma2(bb, m1, x);
+  hi = s;
+  lo = add2(lo, add2(ea, eb));
 }
 
 // Field of one column in f64, for the columns whose f32 pair left the finite
@@ -193,7 +208,8 @@ struct FieldTile {
   static constexpr size_t J_BYTES = (size_t)32 * W * 4;
   static constexpr size_t M_BYTES = (size_t)32 * CH * 4;
   static constexpr size_t E_BYTES = (size_t)CG * CH * 8;
-  static constexpr size_t BYTES = 2 * (J_BYTES + M_BYTES) + E_BYTES;
+  static constexpr size_t P_BYTES = (size_t)8 * 32 * kFieldWarps * 8;
+  static constexpr size_t BYTES = 2 * (J_BYTES + M_BYTES) + E_BYTES + P_BYTES;
 };
 
 template <int TC, int CG>
@@ -206,6 +222,9 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
   float* mt = reinterpret_cast<float*>(fsm + 2 * T::J_BYTES);  // [2][32][CH]
   float2* es =                                                 // [CG][CH]
       reinterpret_cast<float2*>(fsm + 2 * (T::J_BYTES + T::M_BYTES));
+  // this thread's energy pairs of its warp's 8 chains, a row of 256 apart
+  // (16 registers that the loop over the rows needs)
+  float2* eps = es + T::E_BYTES / 8 + threadIdx.x;
   cg::cluster_group cl = cg::this_cluster();
   const int csize = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -233,9 +252,8 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
         ld % 4 == 0 && reinterpret_cast<uintptr_t>(J) % 16 == 0;
     const int nt = (n + 31) >> 5;
     const int64_t cw = c0 + 8 * wg;  // this warp's first chain
-    float2 ep[8];
-#pragma unroll
-    for (int g = 0; g < 8; ++g) ep[g] = make_float2(0.0f, 0.0f);
+    for (int g = 0; g < 8; ++g)
+      eps[g * 32 * kFieldWarps] = make_float2(0.0f, 0.0f);
 
     for (int base = rank * T::W; base < n; base += csize * T::W) {
       auto stage = [&](int t, int buf) {  // rows 32 t ... of J
@@ -277,11 +295,11 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncthreads();
 
-      float2 F[8][TC];
+      uint64_t Fh[4][TC], Fl[4][TC];  // chains 2 q, 2 q + 1
 #pragma unroll
-      for (int g = 0; g < 8; ++g)
+      for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int k = 0; k < TC; ++k) F[g][k] = make_float2(0.0f, 0.0f);
+        for (int k = 0; k < TC; ++k) Fh[q][k] = Fl[q][k] = 0ull;
       for (int t = 0; t < nt; ++t) {
         const int buf = t & 1;
         uint32_t wn = 0u;
@@ -289,11 +307,11 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
           stage(t + 1, buf ^ 1);
           wn = word(t + 1);
         }
-        float part[8][TC];
+        uint64_t part[4][TC];
 #pragma unroll
-        for (int g = 0; g < 8; ++g)
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int k = 0; k < TC; ++k) part[g][k] = 0.0f;
+          for (int k = 0; k < TC; ++k) part[q][k] = 0ull;
         const float* jr = jt + buf * (32 * T::W) + (wc * 32 + lane) * TC;
         const float* mr8 = mt + buf * (32 * T::CH) + 8 * wg;
         // rows past n are zero in the tile: they add +-0
@@ -307,22 +325,23 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
 #pragma unroll
             for (int k = 0; k < TC; ++k) v[k] = jr[r * T::W + k];
           }
-          const float4 m0 =
-              *reinterpret_cast<const float4*>(mr8 + r * T::CH);
-          const float4 m1 =
-              *reinterpret_cast<const float4*>(mr8 + r * T::CH + 4);
-          const float m[8] = {m0.x, m0.y, m0.z, m0.w,
-                              m1.x, m1.y, m1.z, m1.w};
+          const ulonglong2 m0 =
+              *reinterpret_cast<const ulonglong2*>(mr8 + r * T::CH);
+          const ulonglong2 m1 =
+              *reinterpret_cast<const ulonglong2*>(mr8 + r * T::CH + 4);
+          const uint64_t m[4] = {m0.x, m0.y, m1.x, m1.y};
 #pragma unroll
-          for (int g = 0; g < 8; ++g)
+          for (int k = 0; k < TC; ++k) {
+            const uint64_t vv = pack2(v[k], v[k]);
 #pragma unroll
-            for (int k = 0; k < TC; ++k)
-              part[g][k] = fmaf(m[g], v[k], part[g][k]);
+            for (int q = 0; q < 4; ++q) part[q][k] = fma2(m[q], vv, part[q][k]);
+          }
         }
 #pragma unroll
-        for (int g = 0; g < 8; ++g)
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int k = 0; k < TC; ++k) pair_add(F[g][k], part[g][k]);
+          for (int k = 0; k < TC; ++k)
+            pair_add2(Fh[q][k], Fl[q][k], part[q][k]);
         if (t + 1 < nt) {
           put_mult(wn, buf ^ 1);
           asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -342,9 +361,11 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
         const uint32_t* sw = a.s.spins + c * a.p.words;
         const uint32_t wv = sw[col0 >> 5];  // TC divides 32: one word
         float H[TC];
+        float2 ep = eps[g * 32 * kFieldWarps];
 #pragma unroll
         for (int k = 0; k < TC; ++k) {
-          const float hi = F[g][k].x, lo = F[g][k].y;
+          const float hi = half2(Fh[g >> 1][k], g & 1);
+          const float lo = half2(Fl[g >> 1][k], g & 1);
           float e1, e2, e3;
           const float s1 = two_sum(hi, hc[k], e1);
           const float t1 = two_sum(e1, lo, e2);
@@ -355,14 +376,15 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
           const float sg = up ? 1.0f : (ising ? -1.0f : 0.0f);
           if (fabsf(hi) < INFINITY && fabsf(s1) < INFINITY) {
             const float s2 = two_sum(half, hc[k], e1);
-            pair_add(ep[g], sg * s2);
-            ep[g].y += sg * (e1 + 0.5f * lo);
+            pair_add(ep, sg * s2);
+            ep.y += sg * (e1 + 0.5f * lo);
           } else if (col0 + k < n) {
             H[k] = (float)(field_f64(J, ld, n, sw, ising, col0 + k) +
                            (double)hc[k]);
-            ep[g].x = __int_as_float(0x7fc00000);  // energy in f64 below
+            ep.x = __int_as_float(0x7fc00000);  // energy in f64 below
           }
         }
+        eps[g * 32 * kFieldWarps] = ep;
         float* out = a.fields + c * a.field_ld + col0;
         if (vec_out && col0 + TC <= n) {
           if constexpr (TC == 4)
@@ -379,6 +401,9 @@ __global__ void __launch_bounds__(32 * kFieldWarps, 2)
     if (a.set_energies) {
       // lane sums of the pairs: three halving steps leave chain 4 b4 + 2 b3
       // + b2 (bits of the lane) in every lane, two more finish the sum
+      float2 ep[8];
+#pragma unroll
+      for (int g = 0; g < 8; ++g) ep[g] = eps[g * 32 * kFieldWarps];
 #pragma unroll
       for (int o = 4; o; o >>= 1) {
         const bool up = lane & (4 * o);
@@ -464,7 +489,11 @@ static cudaError_t launch_fields_t(const PrepArgs& a, int csize,
 // still gives every SM work; up to 128 columns, 64 chains; up to 32 columns,
 // one column a lane.  Few chains, or few per instance (a tile's chains are
 // done one instance after another), take 8 chains x 256 columns, the columns
-// split over a cluster.
+// split over a cluster.  The wider tiles also split their columns, by up to 4
+// and evenly, while there are fewer than 8 waves of them: the last wave is
+// then shorter (n = 2048, 256 tiles: 2.21 ms at 1, 2.16 at 2, 1.87 at 4, 2.00
+// at 8; n = 1024, 512 tiles: 1.10, 0.96, 0.96; 13 waves of n = 64 .. 1536:
+// 6.5, 7.0, 8.6).
 static cudaError_t launch_fields(const PrepArgs& a, cudaStream_t st) {
   const int64_t chains = a.p.num_chains;
   const int64_t per = chains / (a.p.num_instances > 0 ? a.p.num_instances : 1);
@@ -476,8 +505,12 @@ static cudaError_t launch_fields(const PrepArgs& a, cudaStream_t st) {
     return launch_fields_t<4, 1>(a, 1, st);
   const int passes = (n + 255) / 256;
   if (per >= 32 && chains / 32 * passes >= kFill) {
+    const int64_t tiles = chains / 32;
     int cs = 1;
-    while (cs < 8 && cs < passes && chains / 32 * cs < kFill) cs *= 2;
+    while (cs < 8 && cs < passes &&
+           (tiles * cs < kFill ||
+            (cs < 4 && tiles < 8 * kFill && passes % (2 * cs) == 0)))
+      cs *= 2;
     return launch_fields_t<4, 2>(a, cs, st);
   }
   int cs = 1;
