@@ -357,6 +357,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
   return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
   uint64_t d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));

@@ -154,15 +154,43 @@ __device__ __forceinline__ void pair_add(float2& p, float x) {
 
 // The same for two pairs at once: hi, lo and x hold two f32 each.  The
 // differences are multiply-adds by -1 (the product is exact).
+__device__ __forceinline__ uint64_t two_sum2(uint64_t a, uint64_t b,
+                                             uint64_t& e) {
+  const uint64_t m1 = pack2(-1.0f, -1.0f);
+  const uint64_t s = add2(a, b);
+  const uint64_t bb = fma2(a, m1, s);
+  const uint64_t ea = fma2(fma2(bb, m1, s), m1, a);
+  e = add2(ea, fma2(bb, m1, b));
+  return s;
+}
 __device__ __forceinline__ void pair_add2(uint64_t& hi, uint64_t& lo,
                                           uint64_t x) {
-  const uint64_t m1 = pack2(-1.0f, -1.0f);
-  const uint64_t s = add2(hi, x);
-  const uint64_t bb = fma2(hi, m1, s);
-  const uint64_t ea = fma2(fma2(bb, m1, s), m1, hi);
-  const uint64_t eb = fma2(bb, m1, x);
-  hi = s;
-  lo = add2(lo, add2(ea, eb));
+  uint64_t e;
+  hi = two_sum2(hi, x, e);
+  lo = add2(lo, e);
+}
+// Three f32 a value: the sum to 2^-72 of its largest term.
+struct Triple2 {
+  uint64_t a, b, c;
+  __device__ __forceinline__ void add(uint64_t x) {
+    uint64_t e, f;
+    a = two_sum2(a, x, e);
+    b = two_sum2(b, e, f);
+    c = add2(c, f);
+  }
+  __device__ __forceinline__ void add(const Triple2& t) {
+    add(t.a);
+    add(t.b);
+    add(t.c);
+  }
+};
+__device__ __forceinline__ void lane_sum(Triple2& t) {
+  for (int o = 16; o; o >>= 1) {
+    const Triple2 u = {__shfl_xor_sync(0xffffffffu, t.a, o),
+                       __shfl_xor_sync(0xffffffffu, t.b, o),
+                       __shfl_xor_sync(0xffffffffu, t.c, o)};
+    t.add(u);
+  }
 }
 
 // Field of one column in f64, for the columns whose f32 pair left the finite
@@ -758,9 +786,8 @@ void launch_perm(const PermArgs& a, cudaStream_t st, int count) {
 template <typename T>
 __device__ __forceinline__ void energy64_body(
     int ptype, int n, int ld, const T* J, const T* h, const uint32_t* spins,
-    int words, double* out) {
+    int words, int64_t c, double* out) {
   __shared__ double e_s[8];
-  const int64_t c = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t* sw = spins + c * words;
   const bool ising = ptype == PYSA_GB_ISING;
@@ -791,21 +818,121 @@ __device__ __forceinline__ void energy64_body(
 __global__ void __launch_bounds__(256) k_energy64(
     int ptype, int n, int ld, const double* J, const double* h,
     const uint32_t* spins, int words, double* out) {
-  energy64_body<double>(ptype, n, ld, J, h, spins, words, out);
+  energy64_body<double>(ptype, n, ld, J, h, spins, words, blockIdx.x, out);
 }
 
-// Same with instance inst's f32 couplings and fields of the problem tables.
-// Sparse instances from their stored rows (thread per row, fixed
-// reduction order).
+// ---- the same with instance inst's f32 couplings of the problem tables
+// Dense instances: a cluster takes 4 states, its warps (32 columns x 128
+// rows) units of their sum s (J s + 2 h).  f64 instructions run at 1/64 of the
+// f32 rate and one state's n^2 of them took nearly all of the time, so every
+// lane adds its products, which are exact, into triples of f32 (two states at
+// a time) that carry 72 bits, more than the f64 sum they stand in for, and
+// converts once at the end, after the lanes and warps have been added.  Bound by their 14 paired f32 instructions a
+// product and two states.  QUBO, n = 1284, 128 states: 366 us with f64, 99 so.  A state whose sum leaves the f32 range (or meets an infinity or NaN) is
+// added in f64 as before.
+constexpr int kE64Chunk = 1024;  // rows whose multipliers are staged
+constexpr int kE64Rows = 128;    // rows of a unit
+
+__global__ void __launch_bounds__(256) k_energy64_dense(
+    const pysa_gb_problems p, int inst, const uint32_t* spins, int words,
+    int64_t count, double* out) {
+  namespace cg = cooperative_groups;
+  __shared__ ulonglong2 mult[kE64Chunk];  // [row]: the 4 states' s
+  __shared__ Triple2 e_s[2][8];  // [states 2 q, 2 q + 1][warp]
+  __shared__ int bad_s[4];
+  if (is_sparse_inst(p, inst)) return;  // k_energy64_tables'
+  cg::cluster_group cl = cg::this_cluster();
+  const int csize = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t c0 = 4 * (int64_t)(blockIdx.x / csize);
+  const bool ising = p.problem_type == PYSA_GB_ISING;
+  const int n = p.n[inst], ld = p.ld[inst];
+  const float* J = p.J + p.j_off[inst];
+  const float* h = p.h + p.h_off[inst];
+  const float down = ising ? -1.0f : 0.0f;
+  auto spin = [&](int64_t c, int i) {  // 0 past the last state
+    return c >= count ? 0.0f
+           : (spins[c * words + (i >> 5)] >> (i & 31)) & 1u ? 1.0f : down;
+  };
+  Triple2 E[2] = {};
+  const int nt = (n + 31) >> 5;
+  for (int r0 = 0; r0 < n; r0 += kE64Chunk) {
+    const int rows = n - r0 < kE64Chunk ? n - r0 : kE64Chunk;
+    __syncthreads();
+    for (int i = tid; i < rows; i += 256)
+      mult[i] = make_ulonglong2(
+          pack2(spin(c0, r0 + i), spin(c0 + 1, r0 + i)),
+          pack2(spin(c0 + 2, r0 + i), spin(c0 + 3, r0 + i)));
+    __syncthreads();
+    const int units = nt * ((rows + kE64Rows - 1) / kE64Rows);
+    for (int u = rank * 8 + warp; u < units; u += 8 * csize) {
+      const int b = u / nt, col = 32 * (u - b * nt) + lane;
+      const bool in = col < n;
+      const int i1 = (b + 1) * kE64Rows < rows ? (b + 1) * kE64Rows : rows;
+      const float* Jc = J + (int64_t)r0 * ld + (in ? col : 0);
+      Triple2 F[2] = {};
+#pragma unroll 4
+      for (int i = b * kE64Rows; i < i1; ++i) {
+        const float v = in ? Jc[(int64_t)i * ld] : 0.0f;
+        const uint64_t vv = pack2(v, v);
+        const ulonglong2 m = mult[i];
+        F[0].add(mul2(vv, m.x));
+        F[1].add(mul2(vv, m.y));
+      }
+      const float h2 = in && r0 == 0 && b == 0 ? 2.0f * h[col] : 0.0f;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint64_t s =
+            in ? pack2(spin(c0 + 2 * q, col), spin(c0 + 2 * q + 1, col))
+               : 0ull;
+        E[q].add(mul2(F[q].a, s));
+        E[q].add(mul2(F[q].b, s));
+        E[q].add(mul2(F[q].c, s));
+        E[q].add(mul2(pack2(h2, h2), s));
+      }
+    }
+  }
+  // lanes, then the cluster's warps (two a lane), still as triples
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    lane_sum(E[q]);
+    if (lane == 0) e_s[q][warp] = E[q];
+  }
+  cl.sync();
+  if (rank == 0) {
+    if (warp < 2) {
+      Triple2 t = {};
+      for (int i = lane; i < 8 * csize; i += 32)
+        t.add(*cl.map_shared_rank(&e_s[warp][i & 7], i >> 3));
+      lane_sum(t);
+      if (lane < 2) {
+        const bool hi = lane;
+        const int64_t c = c0 + 2 * warp + lane;
+        const float a = half2(t.a, hi);
+        const bool bad = !(fabsf(a) < INFINITY) && c < count;
+        bad_s[2 * warp + lane] = bad;
+        if (!bad && c < count)
+          out[c] = 0.5 * ((double)a + ((double)half2(t.b, hi) +
+                                       (double)half2(t.c, hi)));
+      }
+    }
+    __syncthreads();
+    for (int q = 0; q < 4; ++q) {
+      if (!bad_s[q]) continue;  // uniform
+      energy64_body<float>(p.problem_type, n, ld, J, h, spins, words, c0 + q,
+                           out);
+      __syncthreads();
+    }
+  }
+  cl.sync();
+}
+
+// Sparse instances from their stored rows: a CTA per state, thread per row,
+// fixed reduction order.
 __global__ void __launch_bounds__(256) k_energy64_tables(
     const pysa_gb_problems p, int inst, const uint32_t* spins, int words,
     double* out) {
-  if (!is_sparse_inst(p, inst)) {
-    energy64_body<float>(p.problem_type, p.n[inst], p.ld[inst],
-                         p.J + p.j_off[inst], p.h + p.h_off[inst], spins,
-                         words, out);
-    return;
-  }
+  if (!is_sparse_inst(p, inst)) return;  // k_energy64_dense's
   __shared__ double e_s[8];
   const int64_t c = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -841,7 +968,25 @@ void launch_energy64(int ptype, int n, int ld, const double* J,
 void launch_energy64_tables(const pysa_gb_problems& p, int inst,
                             const uint32_t* spins, int words, int64_t count,
                             double* out, cudaStream_t st) {
-  if (count > 0)
+  if (count <= 0) return;
+  // as many CTAs a cluster as have a unit for each of their warps
+  const int64_t nt = ((int64_t)p.max_n + 31) / 32;
+  const int64_t units = nt * ((p.max_n + kE64Rows - 1) / kE64Rows);
+  int cs = 1;
+  while (cs < 8 && units > 8 * cs) cs *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((count + 3) / 4 * cs));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cs;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_energy64_dense, p, inst, spins, words, count,
+                     out);
+  if (p.csr_row_off)
     k_energy64_tables<<<(unsigned)count, 256, 0, st>>>(p, inst, spins, words,
                                                        out);
 }
