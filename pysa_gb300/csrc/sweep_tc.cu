@@ -25,11 +25,12 @@
 //
 // Roles: warps 0-3 decide (thread = TMEM lane; with F > 1 only the warps of
 // the slice holding the block's columns, the others help: at F = 2 they
-// compute the older sub-blocks' corrections and write A rows, at F = 4 they
-// write A rows; in block rounds at F = 2 all four decide, two lanes per
-// chain, from fields the holding slice stashes in shared memory), warp 4
-// issues MMAs, warp 5 produces stages, warps 6-7 precompute the next
-// block's log-uniforms.  Every wait is bounded; a
+// compute the older sub-blocks' corrections and write A rows; an item of at
+// most 32 chains, so every one at F = 4, passes the sub-blocks of a block from
+// decision warp to decision warp; in block rounds at F = 2 all four decide,
+// two lanes per chain, from fields the holding slice stashes in shared
+// memory), warp 4 issues MMAs, warp 5 produces stages, warps 6-7 precompute
+// the next block's log-uniforms.  Every wait is bounded; a
 // timeout sets the status word and an abort flag that releases every other
 // wait.
 #include <cuda_fp8.h>
@@ -96,8 +97,6 @@ struct TcCfg {
   // F == 2: corrections of sub-blocks 2 and 3 from the older sub-blocks,
   // computed by the idle slice's threads ([2][16][CC] floats)
   static constexpr bool HELP = F == 2;
-  // F == 4: the three idle slices' warps write the A rows of sub-blocks 0-2
-  static constexpr bool APUT = F == 4;
   // F == 2: block rounds run on all four decision warps, two lanes per chain
   // (the other slice's warps would idle)
   static constexpr bool PAIRS = F == 2;
@@ -106,10 +105,11 @@ struct TcCfg {
   static constexpr size_t CORR_OFF = INVB_OFF + CC * 4;
   static constexpr size_t CORR_BYTES = HELP ? (size_t)2 * 16 * CC * 4 : 0;
   // RND, F > 1: fields of the block's 64 scattered columns, gathered by the
-  // warps whose slices hold them ([64][CC] floats)
+  // warps whose slices hold them; F == 4: the block's fields for the relay's
+  // warps ([64][CC] floats)
   static constexpr size_t HBUF_OFF = CORR_OFF + CORR_BYTES;
   static constexpr size_t HBUF_BYTES =
-      (RND && F > 1) ? (size_t)64 * CC * 4 : 0;
+      ((RND && F > 1) || F == 4) ? (size_t)64 * CC * 4 : 0;
   // RND: each decision warp's copy of the block's 64 permutation entries
   static constexpr size_t PERM_OFF = HBUF_OFF + HBUF_BYTES;
   static constexpr size_t PERM_BYTES = RND ? (size_t)4 * 64 * 4 : 0;
@@ -232,15 +232,16 @@ __device__ __forceinline__ void named_sync_dec() {
   __syncwarp();
   asm volatile("barrier.sync 3, 128;" ::: "memory");
 }
-// Fold 4: the deciding warp announces sub-blocks 0-2 without waiting; the
-// three other warps wait for it (the same barrier, 128 threads in all)
-__device__ __forceinline__ void named_arrive_aput() {
+// Relay of a block's sub-blocks over the decision warps: the holder announces
+// the stashed fields (step 0, 128 threads), the warp of sub-block g its
+// decisions to the later ones (step g + 1).
+__device__ __forceinline__ void relay_arrive(int id, int threads) {
   __syncwarp();
-  asm volatile("barrier.arrive 3, 128;" ::: "memory");
+  asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
-__device__ __forceinline__ void named_sync_aput() {
+__device__ __forceinline__ void relay_sync(int id, int threads) {
   __syncwarp();
-  asm volatile("barrier.sync 3, 128;" ::: "memory");
+  asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 __device__ __forceinline__ void named_sync_helpers() {
@@ -279,6 +280,30 @@ __device__ __forceinline__ uint32_t e4m3_bits(float d) {
   return ((((u >> 23) & 0xFFu) - 120u) << 3) | ((u >> 24) & 0x80u);
 }
 
+// Sub-block gg's 16 deltas into an A row.
+template <bool E8>
+__device__ __forceinline__ void put_deltas(unsigned char* rowp, int gg,
+                                           const float* d) {
+  if constexpr (E8) {
+    uint32_t pkg[4];
+#pragma unroll
+    for (int j = 0; j < 16; j += 4)
+      pkg[j >> 2] = e4m3_bits(d[j]) | (e4m3_bits(d[j + 1]) << 8) |
+                    (e4m3_bits(d[j + 2]) << 16) | (e4m3_bits(d[j + 3]) << 24);
+    *reinterpret_cast<uint4*>(rowp + gg * 128) =
+        make_uint4(pkg[0], pkg[1], pkg[2], pkg[3]);
+  } else {
+    uint32_t pkg[8];
+#pragma unroll
+    for (int j = 0; j < 16; j += 2)
+      pkg[j >> 1] = bf16_bits(d[j]) | (bf16_bits(d[j + 1]) << 16);
+    *reinterpret_cast<uint4*>(rowp + (2 * gg) * 128) =
+        make_uint4(pkg[0], pkg[1], pkg[2], pkg[3]);
+    *reinterpret_cast<uint4*>(rowp + (2 * gg + 1) * 128) =
+        make_uint4(pkg[4], pkg[5], pkg[6], pkg[7]);
+  }
+}
+
 // The rare exact redo of one deciding thread's sub-block (some decision of
 // the warp fell inside the f32 band), kept out of line: inlined, its code
 // and registers slow the fast path by about 12 %.  It rebuilds the
@@ -290,6 +315,7 @@ struct RedoCtx {
   float* dl_s;              // deltas [64][CC]
   const float* corr_s;      // helper corrections (fold 2)
   const float* hbuf;        // gathered fields (random order, fold > 1)
+  const float* stash;       // or the block's fields [64][CC] (relay)
   const int32_t* perm_w;    // this warp's visiting positions (random order)
   const float* lfb;         // log-uniforms [chain][64], cidx() order
   uint32_t taddr;           // TMEM address of the thread's lane
@@ -308,7 +334,10 @@ __device__ __noinline__ void redo_subblock(const RedoCtx& x, uint32_t* wcur,
   constexpr int CC = 128 / F;
   const int g = x.g, c = x.c;
   float hs[16];
-  if constexpr (!RND) {
+  if (x.stash) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) hs[j] = x.stash[(16 * g + j) * CC + c];
+  } else if constexpr (!RND) {
     tc::tmem_ld16(x.taddr + x.co + 16 * g, hs);
   } else if constexpr (F > 1) {
 #pragma unroll
@@ -617,6 +646,8 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
     const int words = (n + 31) >> 5;
     const int64_t chain_base = a.p.chain_off[inst];
     const bool valid = warp < 4 && c < item.nchains;
+    // sequential sub-blocks one warp each (below)
+    const bool relay = F == 4 || item.nchains <= 32;
     const int64_t chain = item.chain0 + c;
     const uint32_t chain_local = (uint32_t)(chain - chain_base);
     const uint32_t G0 = G, RG0 = RG;
@@ -1124,6 +1155,277 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
               if (L == 0) count(a, 0, 1);
               fence_proxy_async();
             }
+          } else if (relay && !d64) {
+            // ------------------- sub-blocks in a relay of the four warps
+            // At most 32 chains: one warp's lanes would hold them all and the
+            // three others idle.  Warp g (counted from the one whose TMEM
+            // lanes hold the block, which stashes the 64 fields in shared
+            // memory) takes sub-block g: it prepares its thresholds, adds
+            // the older sub-blocks' corrections as they are announced, and
+            // only those of the one before it and its own 16 decisions are
+            // left on the block's critical path.  Same corrections in the
+            // same order as in the sub-blocks of one warp below.  Bound by
+            // that path: 16 dependent decisions, then 16 rows of 16.
+            // Measured: 128 spins, 1000 sweeps of 3200 chains in items of 32
+            // 24.5 -> 19.1 ms; 912 spins, 40 sweeps of 300 in items of 30
+            // 4.93 -> 4.14; 2048 spins, 24 sweeps of 8192 22.6 -> 22.3
+            // (there the couplings' way from L2 is the longer one).
+            const int holder = F == 1 ? 0 : F == 2 ? 2 * qt : qt;
+            const int g = (warp - holder) & 3;
+            const bool rvalid = lane < item.nchains;
+            const bool gathered = RND && F > 1;  // hbuf is filled above
+            bool ok = !*sh.abort;
+            if (ok && g == 0 && wait_h && !gathered)
+              ok = tc_wait(sh.h_ready, (Gb - 1) & 1, sh, status);
+            if (ok) ok = tc_wait(&sh.jbb_full[Gb & 1], (Gb >> 1) & 1, sh, status);
+            if (ok) ok = tc_wait(&sh.lf_full[Gb & 1], (Gb >> 1) & 1, sh, status);
+            ok = __all_sync(0xffffffffu, ok);
+            const bool lead = ok && g == 0 && lane == 0;
+            if (lead) stamp(a, Gb, 0);
+            // fields [64][CC]: folds 1 and 2 use columns 32 .. 63 of dl_s,
+            // whose chains this item does not have
+            float* stash = F == 4 || gathered ? hbuf : dl_s + 32;
+            float* deb_s = reinterpret_cast<float*>(epart_s);  // [32]
+            uint32_t* cnt_s = reinterpret_cast<uint32_t*>(deb_s + 32);
+            const float* jb = jbb + (Gb & 1) * 4096 + 16 * g;
+            uint64_t hs2[8];
+            if (g == 0 && ok && !gathered) {
+              tc::fence_after_sync();
+              float h[64];
+              if constexpr (!RND) {
+                tc::tmem_ld64(taddr + lane_base + co, h);
+              } else {
+#pragma unroll
+                for (int k0 = 0; k0 < 64; k0 += 16) {
+                  uint32_t r[16];
+                  int sp[16];
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) sp[j] = spos(k0 + j);
+                  __syncwarp();
+#pragma unroll
+                  for (int j = 0; j < 16; ++j)
+                    r[j] = tc::tmem_ld1_nowait(
+                        taddr + lane_base + (uint32_t)(sp[j] < 0 ? 0 : sp[j]));
+                  tc::tmem_wait_ld16(r);
+#pragma unroll
+                  for (int j = 0; j < 16; ++j)
+                    h[k0 + j] = k0 + j < kmax ? __uint_as_float(r[j]) : 0.0f;
+                }
+              }
+#pragma unroll
+              for (int k = 0; k < 64; ++k) stash[k * CC + lane] = h[k];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) hs2[i] = pack2(h[2 * i], h[2 * i + 1]);
+            }
+            if (lead) stamp(a, Gb, 8);
+            if (!gathered) {
+              if (g == 0) relay_arrive(4, 128);
+            }
+            // thresholds of this sub-block (the rule of the sub-blocks below)
+            const float rbeta = beta_s[lane];
+            const float scale = ising ? 2.0f : 1.0f;
+            const float invbs = invb_s[lane];
+            const bool banded = rvalid && invbs < INFINITY;
+            const float band0 = banded ? 3e-5f * invbs : 0.0f;
+            const float band1 = banded ? 1e-6f * invbs : 0.0f;
+            const float* lfb = lf_s + (Gb & 1) * 64 * CC;
+            float tl[16], th[16];
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+              const float4 v = *reinterpret_cast<const float4*>(
+                  lfb + cidx(lane, 16 * g + 4 * q4));
+              const float ak[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int j = 4 * q4 + i;
+                tl[j] = ak[i] * invbs;
+                th[j] = fminf(fmaf(2.0f * band1, fabsf(ak[i]),
+                                   tl[j] + 2.0f * band0), 0.0f);
+              }
+            }
+            const uint32_t ow =
+                RND ? posb[((Gb & 1) * 2 + (g >> 1)) * CC + lane]
+                    : spins_s[(2 * t + (g >> 1)) * CC + lane];
+            const int sb = 16 * (g & 1);
+            const uint32_t sbits = ow >> sb;  // spins before the sub-block
+            const int nlive = kmax - 16 * g;
+            const uint32_t live_mask =
+                nlive >= 16 ? 0xFFFFu : nlive > 0 ? (1u << nlive) - 1u : 0u;
+            if (gathered) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int k = 16 * g + 2 * i;
+                hs2[i] = pack2(k < kmax ? hbuf[k * CC + lane] : 0.0f,
+                               k + 1 < kmax ? hbuf[(k + 1) * CC + lane] : 0.0f);
+              }
+            } else if (g > 0) {
+              relay_sync(4, 128);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int k = 16 * g + 2 * i;
+                hs2[i] = pack2(stash[k * CC + lane], stash[(k + 1) * CC + lane]);
+              }
+            }
+            // 16 rows of corrections from sub-block pg
+            auto rows = [&](int pg, uint64_t* acc) {
+#pragma unroll 8
+              for (int k = 0; k < 16; ++k) {
+                const float d = dl_s[(16 * pg + k) * CC + lane];
+                const uint64_t dd = pack2(d, d);
+                const ulonglong2* jr = reinterpret_cast<const ulonglong2*>(
+                    jb + (16 * pg + k) * 64);
+#pragma unroll
+                for (int q4 = 0; q4 < 4; ++q4) {
+                  const ulonglong2 v = jr[q4];
+                  acc[2 * q4] = fma2(dd, v.x, acc[2 * q4]);
+                  acc[2 * q4 + 1] = fma2(dd, v.y, acc[2 * q4 + 1]);
+                }
+              }
+            };
+#pragma unroll 1
+            for (int pg = 0; pg < g - 1; ++pg) {  // before the previous one
+              relay_sync(5 + pg, 32 * (4 - pg));
+              if constexpr (!C::HELP) {
+                if (ok) rows(pg, hs2);
+              }
+            }
+            if constexpr (C::HELP) {
+              // fold 2 sums these first, as its helpers do
+              if (g > 1) {
+                uint64_t cs[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) cs[i] = 0ull;
+                if (ok)
+                  for (int pg = 0; pg < g - 1; ++pg) rows(pg, cs);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  corr_s[((g - 2) * 16 + 2 * i) * CC + lane] = half2(cs[i], false);
+                  corr_s[((g - 2) * 16 + 2 * i + 1) * CC + lane] =
+                      half2(cs[i], true);
+                  hs2[i] = add2(hs2[i], cs[i]);
+                }
+              }
+            }
+            float dEb = 0.0f;
+            uint32_t cnt = 0u;
+            if (g > 0) {
+              relay_sync(5 + g - 1, 32 * (5 - g));
+              dEb = deb_s[lane];
+              cnt = cnt_s[lane];
+              if (ok) rows(g - 1, hs2);
+            }
+            if (lead) stamp(a, Gb, 9);
+            float dcur[16];
+            uint32_t wcur = ow, flips = 0u;
+            bool unc = false;
+            const float dEsave = dEb;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float hj = half2(hs2[j >> 1], j & 1);
+              const bool sbit = (sbits >> j) & 1u;
+              const float x = sbit ? hj : -hj;
+              const bool acc = x >= th[j];
+              unc |= !acc && !(x < tl[j]);
+              const float dl = acc ? (sbit ? -scale : scale) : 0.0f;
+              dcur[j] = dl;
+              dEb = fmaf(dl, hj, dEb);
+              flips |= acc ? (1u << j) : 0u;
+              if (j < 15) {
+                const uint64_t dd = pack2(dl, dl);
+                const ulonglong2* jr = reinterpret_cast<const ulonglong2*>(
+                    jb + (16 * g + j) * 64);
+                // (a pair's already decided half is not read again)
+#pragma unroll
+                for (int q4 = (j + 1) >> 2; q4 < 4; ++q4) {
+                  const ulonglong2 v = jr[q4];
+                  if (4 * q4 + 1 > j) hs2[2 * q4] = fma2(dd, v.x, hs2[2 * q4]);
+                  if (4 * q4 + 3 > j)
+                    hs2[2 * q4 + 1] = fma2(dd, v.y, hs2[2 * q4 + 1]);
+                }
+              }
+            }
+            wcur ^= (flips & live_mask) << sb;
+            if (__any_sync(0xffffffffu, ok && unc)) {
+              // rare: the whole sub-block again with the exact f64 rule
+              RedoCtx rx;
+              rx.jb = jb - 16 * g;
+              rx.dl_s = dl_s;
+              rx.corr_s = corr_s;
+              rx.hbuf = hbuf;
+              rx.stash = gathered ? nullptr : stash;
+              rx.perm_w = perm_s + warp * 64;
+              rx.lfb = lfb;
+              rx.taddr = taddr + lane_base;
+              rx.co = co;
+              rx.kmax = kmax;
+              rx.c = lane;
+              rx.g = g;
+              rx.i0 = i0;
+              rx.sb = sb;
+              rx.valid = rvalid;
+              rx.ising = ising;
+              rx.beta = rbeta;
+              rx.seed = chain_seed(a.seed, a.s.stream_key, item.chain0 + lane);
+              rx.inst = (uint32_t)inst;
+              rx.sweep = sweep;
+              rx.chain_local = (uint32_t)(item.chain0 + lane - chain_base);
+              rx.wsave = ow;
+              rx.dEsave = dEsave;
+              redo_subblock<F, RND>(rx, &wcur, &dEb);
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                dcur[j] = dl_s[(16 * g + j) * CC + lane];
+            }
+            const uint32_t fm =
+                rvalid ? ((wcur ^ ow) >> sb) & 0xFFFFu : 0u;
+            cnt += __popc(fm);
+            if (g < 3) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                dl_s[(16 * g + j) * CC + lane] = dcur[j];
+              deb_s[lane] = dEb;
+              cnt_s[lane] = cnt;
+              relay_arrive(5 + g, 32 * (4 - g));
+            }
+            if (lead) stamp(a, Gb, 10);
+            if (ok) {
+              if constexpr (!RND) {
+                // this sub-block's half of the spin word
+                if (rvalid)
+                  reinterpret_cast<uint16_t*>(
+                      spins_s + (2 * t + (g >> 1)) * CC + lane)[g & 1] =
+                      (uint16_t)(wcur >> sb);
+              } else {
+                uint32_t fb = fm;
+                while (fb) {
+                  const int sp = spos(16 * g + __ffs(fb) - 1);
+                  fb &= fb - 1u;
+                  atomicXor(spins_s + (sp >> 5) * CC + lane, 1u << (sp & 31));
+                }
+              }
+              if (g == 3 && rvalid) dE_s[lane] += (double)dEb;
+              // A rows once the MMAs that read this buffer are done (the
+              // last block's; fold 4 has two buffers, a unit's first two
+              // blocks follow the previous unit's, which are all done)
+              bool a_ok = true;
+              if constexpr (C::A_NBUF == 2) {
+                a_ok = Gb < G0 + 2 ||
+                       tc_wait(&sh.mma_done_b[Gb & 1], ((Gb >> 1) - 1) & 1, sh,
+                               status);
+              } else {
+                a_ok = Gb == G0 || tc_wait(sh.mma_done, (Gb - 1) & 1, sh, status);
+              }
+              if (a_ok) {
+                unsigned char* rowp = a_row(
+                    128 - CC + lane +
+                    (C::A_NBUF == 2 ? 128 * (int)(Gb & 1) : 0));
+                put_deltas<E8>(rowp, g, dcur);
+              }
+              if (g == 3)
+                blk_mf = __reduce_max_sync(0xffffffffu, rvalid ? cnt : 0u);
+              if (lead) count(a, 1, 1);
+            }
+            fence_proxy_async();
           } else {
           bool go = q == qt && !*sh.abort;
           // fields of this block: the previous block's critical MMA (not
@@ -1148,27 +1450,9 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
           // one sub-block's deltas of chain c into its A row (one copy,
           // seen by every slice's MMA)
           auto put_a = [&](int gg, const float* d) {
-            unsigned char* rowp = a_row(
-                128 - CC + c + (C::A_NBUF == 2 ? 128 * (int)(Gb & 1) : 0));
-            if constexpr (E8) {
-              uint32_t pkg[4];
-#pragma unroll
-              for (int j = 0; j < 16; j += 4)
-                pkg[j >> 2] = e4m3_bits(d[j]) | (e4m3_bits(d[j + 1]) << 8) |
-                              (e4m3_bits(d[j + 2]) << 16) |
-                              (e4m3_bits(d[j + 3]) << 24);
-              *reinterpret_cast<uint4*>(rowp + gg * 128) =
-                  make_uint4(pkg[0], pkg[1], pkg[2], pkg[3]);
-            } else {
-              uint32_t pkg[8];
-#pragma unroll
-              for (int j = 0; j < 16; j += 2)
-                pkg[j >> 1] = bf16_bits(d[j]) | (bf16_bits(d[j + 1]) << 16);
-              *reinterpret_cast<uint4*>(rowp + (2 * gg) * 128) =
-                  make_uint4(pkg[0], pkg[1], pkg[2], pkg[3]);
-              *reinterpret_cast<uint4*>(rowp + (2 * gg + 1) * 128) =
-                  make_uint4(pkg[4], pkg[5], pkg[6], pkg[7]);
-            }
+            put_deltas<E8>(
+                a_row(128 - CC + c +
+                      (C::A_NBUF == 2 ? 128 * (int)(Gb & 1) : 0)), gg, d);
           };
           if (go) {
             tc::fence_after_sync();
@@ -1289,7 +1573,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             // mode-dependent decisions: rounds over the whole block (few
             // flips) or four sequential sub-blocks of 16 spins
             uint64_t flips64 = 0ull;
-            if (d64) {
+            if (F == 4 || d64) {  // (fold 4's sub-blocks are the relay's)
               // ---------------------------------------- block rounds (D64)
               // The block's 64 fields in registers.  A round tests every
               // undecided position against the current fields at once: the
@@ -1509,6 +1793,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 rx.dl_s = dl_s;
                 rx.corr_s = corr_s;
                 rx.hbuf = hbuf;
+                rx.stash = nullptr;
                 rx.perm_w = perm_s + warp * 64;
                 rx.lfb = lfb;
                 rx.taddr = taddr + lane_base;
@@ -1547,11 +1832,6 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 if (g == 3 && (Gb == G0 || tc_wait(sh.mma_done, (Gb - 1) & 1,
                                                    sh, status)))
                   put_a(3, dcur);
-              } else if constexpr (C::APUT) {
-                // sub-blocks 0-2 go to the other slices' warps; the last
-                // sub-block's rows here, after the previous block's MMAs
-                if (g == 2) named_arrive_aput();
-                if (g == 3 && a_buffer_free()) put_a(3, dcur);
               } else {
                 if (g == 1)
                   a_early =
@@ -1566,7 +1846,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
               if (lead) stamp(a, Gb, 10 + 3 * g);
               if (C::HELP && g < 3) named_sync_dec();  // sub-block g published
             }
-            if (!C::HELP && !C::APUT && !a_early) {
+            if (!C::HELP && !a_early) {
               if (Gb > G0) {
                 if (lead) stamp(a, Gb, 2);
                 const bool a_ok =
@@ -1611,20 +1891,6 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             blk_mf = __reduce_max_sync(
                 0xffffffffu, valid ? (uint32_t)__popcll(flips64) : 0u);
             if (lead) count(a, d64 ? 0 : 1, 1);
-            fence_proxy_async();
-          } else if (C::APUT && !d64) {
-            // one of the three other slices' warps (or every warp after an
-            // abort): the A rows of sub-block hr once sub-blocks 0-2 are
-            // decided and the previous block's MMAs are done
-            named_sync_aput();
-            const int hr = (q + 3 - qt) & 3;  // 0, 1, 2 for q = qt+1, +2, +3
-            if (hr < 3 && __all_sync(0xffffffffu, !*sh.abort) &&
-                a_buffer_free()) {
-              float d[16];
-#pragma unroll
-              for (int j = 0; j < 16; ++j) d[j] = dl_s[(16 * hr + j) * CC + c];
-              put_a(hr, d);
-            }
             fence_proxy_async();
           } else if (C::HELP && !d64) {
             // helper (the other slice's thread of chain c), or a deciding
