@@ -92,6 +92,15 @@ def uniform_partition_fun(n: int):
     return n * np.log(2)
 
 
+def uniform_samples(n: int, problem_type: str, count: int) -> np.ndarray:
+    """`count` draws of uniform_prob_initialization, one after another: the
+    same numbers of the same stream in one call."""
+    if problem_type not in ("qubo", "ising"):
+        raise ValueError(f"problem_type=='{problem_type}' not supported.")
+    x = np.random.randint(2, size=(count, n))
+    return x if problem_type == "qubo" else 2 * x - 1
+
+
 # --------------------------------------------- "bernoulli" (pysa/ais.py:175-226)
 def bernoulli_prob_initialization(n: int, problem_type: str,
                                   initial_args=(0.5,)):
@@ -103,6 +112,16 @@ def bernoulli_prob_initialization(n: int, problem_type: str,
     else:
         raise ValueError(f"problem_type=='{problem_type}' not supported.")
     return np.array(state)
+
+
+def bernoulli_samples(n: int, problem_type: str, count: int,
+                      initial_args=(0.5,)) -> np.ndarray:
+    """`count` draws of bernoulli_prob_initialization, one after another: the
+    same numbers of the same stream in one call."""
+    if problem_type not in ("qubo", "ising"):
+        raise ValueError(f"problem_type=='{problem_type}' not supported.")
+    x = np.random.binomial(1, 1 - initial_args[0], size=(count, n))
+    return x if problem_type == "qubo" else 2 * x - 1
 
 
 def bernoulli_ref_prob(state: Vector, p: float, pos: int = -1):

@@ -9,9 +9,12 @@
 namespace pysa_gb {
 
 // ------------------------------------------------------------ J packing
-// packed[i][l * LS + m] = J[i][32 m + l] (0 outside the instance).
+// packed[i][l * LS + m] = J[i][32 m + l] (0 outside the instance); blockIdx.y
+// instances at even steps.
 __global__ void k_pack_rows(const float* J, int ld, int n, int nc, int ls,
-                            float* packed) {
+                            float* packed, int64_t j_step, int64_t p_step) {
+  J += blockIdx.y * j_step;
+  packed += blockIdx.y * p_step;
   const int row_len = 32 * ls;
   const int64_t total = (int64_t)n * row_len;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
@@ -24,11 +27,13 @@ __global__ void k_pack_rows(const float* J, int ld, int n, int nc, int ls,
 }
 
 void launch_pack_rows(const float* J, int ld, int n, int nc, int ls,
-                      float* packed, cudaStream_t st) {
+                      float* packed, int count, int64_t j_step,
+                      int64_t p_step, cudaStream_t st) {
   const int64_t total = (int64_t)n * 32 * ls;
   int blocks = (int)((total + 255) / 256);
   if (blocks > 4096) blocks = 4096;
-  k_pack_rows<<<blocks, 256, 0, st>>>(J, ld, n, nc, ls, packed);
+  k_pack_rows<<<dim3(blocks, count), 256, 0, st>>>(J, ld, n, nc, ls, packed,
+                                                   j_step, p_step);
 }
 
 // -------------------------------------------------- fields and energies

@@ -221,7 +221,7 @@ extern "C" int pysa_gb_sweeps_noalloc(const pysa_gb_problems* p,
       return pysa_gb_internal_fail(PYSA_GB_ERR_ARG, "sweeps_noalloc: ld < n");
     launch_pack_rows(p->J + host->j_off[i], host->ld[i], host->n[i],
                      plain_variant(v).nc, plan.row_floats[v] / 32,
-                     ws.packed_j + poff, st);
+                     ws.packed_j + poff, 1, 0, 0, st);
     poff += (int64_t)host->n[i] * plan.row_floats[v];
   }
   cudaError_t e = cudaGetLastError();

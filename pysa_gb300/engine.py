@@ -150,6 +150,39 @@ class Instance:
     reads: int
 
 
+_TORCH = {np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64,
+          np.dtype(np.float32): torch.float32}
+
+
+def _carve(specs: list, host: bool = True):
+    """(name, array or (length, dtype)) pieces at 256-byte steps of one block.
+    Returns (the zeroed host block holding the arrays, or its size without
+    `host`; {name: host view, or (length, dtype)}; {name: offset})."""
+    off, kind, at = {}, {}, 0
+    for k, a in specs:
+        ln, dt = (a.size, a.dtype) if isinstance(a, np.ndarray) else a
+        off[k], kind[k] = at, (int(ln), np.dtype(dt))
+        at += (int(ln) * np.dtype(dt).itemsize + 255) // 256 * 256
+    if not host:
+        return at, kind, off
+    blk = np.zeros(at, np.uint8)
+    views = _views(blk, kind, off)
+    for k, a in specs:
+        if isinstance(a, np.ndarray):
+            views[k][:] = a
+    return blk, views, off
+
+
+def _views(block, pieces: dict, off: dict) -> dict:
+    """The pieces of a block (host array or device tensor of bytes)."""
+    out = {}
+    for k, v in pieces.items():
+        ln, dt = (v.size, v.dtype) if isinstance(v, np.ndarray) else v
+        b = block[off[k]:off[k] + ln * dt.itemsize]
+        out[k] = b.view(dt if isinstance(block, np.ndarray) else _TORCH[dt])
+    return out
+
+
 class PTBatch:
 
     def __init__(self, problem_type: str, instances: list[Instance],
@@ -221,22 +254,27 @@ class PTBatch:
         self.num_chains, self.num_reads = ct, rt
         self.max_n = int(n.max()) if I else 1
         self.words = (self.max_n + 31) // 32
-        Jcat = np.zeros(max(jt, 1), np.float32)
-        hcat = np.zeros(max(ht, 1), np.float32)
-        lad = np.zeros(max(lt, 1), np.float32)
-        lsort = np.zeros(max(lt, 1), np.int32)
+        read_inst = np.repeat(np.arange(I, dtype=np.int32), Rd)
+        # the tables in one host block and one copy to the device
+        host, tv, off = _carve(
+            [("n", n), ("R", R), ("Rd", Rd), ("ld", ld), ("j_off", j_off),
+             ("h_off", h_off), ("chain_off", chain_off),
+             ("read_off", read_off), ("ladder_off", ladder_off),
+             ("read_inst", read_inst if rt else np.zeros(1, np.int32)),
+             ("J", (max(jt, 1), np.float32)), ("h", (max(ht, 1), np.float32)),
+             ("ladder", (max(lt, 1), np.float32)),
+             ("lsort", (max(lt, 1), np.int32))])
+        Jcat, hcat, lad, lsort = (tv[k] for k in ("J", "h", "ladder", "lsort"))
         for i, x in enumerate(instances):
             ni, li = int(n[i]), int(ld[i])
             if not flags[i]:
-                blk = np.zeros((ni, li), np.float32)
                 # transposed: row j = change of every field when spin j flips
-                blk[:, :ni] = np.asarray(_dense(x.J), np.float32).T
-                Jcat[j_off[i]:j_off[i] + ni * li] = blk.ravel()
+                Jcat[j_off[i]:j_off[i] + ni * li].reshape(ni, li)[:, :ni] = \
+                    np.asarray(_dense(x.J), np.float32).T
             hcat[h_off[i]:h_off[i] + ni] = np.asarray(x.h, np.float32)
             lad[ladder_off[i]:ladder_off[i] + R[i]] = x.ladder
             lsort[ladder_off[i]:ladder_off[i] + R[i]] = np.argsort(
                 np.asarray(x.ladder, np.float32), kind="stable")
-        read_inst = np.repeat(np.arange(I, dtype=np.int32), Rd)
         dev = self.device
         # sparse-row instances and their tables (flags above)
         self.sparse = np.asarray(flags, np.int32) if I else np.zeros(
@@ -271,11 +309,7 @@ class PTBatch:
         def T(a):
             return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
 
-        self._t = dict(n=T(n), R=T(R), Rd=T(Rd), ld=T(ld), j_off=T(j_off),
-                       h_off=T(h_off), chain_off=T(chain_off),
-                       read_off=T(read_off), ladder_off=T(ladder_off),
-                       read_inst=T(read_inst if rt else np.zeros(1, np.int32)),
-                       J=T(Jcat), h=T(hcat), ladder=T(lad), lsort=T(lsort))
+        self._t = _views(T(host), tv, off)
         if self.has_sparse:
             self._t.update(
                 csr_row_off=T(row_off), csr_ent_off=T(ent_off),
@@ -300,15 +334,18 @@ class PTBatch:
         C, W = max(ct, 1), self.words
         z = lambda *s, dt: torch.zeros(*s, dtype=dt, device=dev)  # noqa: E731
         self.spins = z(C, W, dt=torch.int32)
-        self.energies = z(C, dt=torch.float32)
-        self.beta_idx = z(C, dt=torch.int32)
-        self.chain_beta = z(C, dt=torch.float32)
-        self.best_energy = z(C, dt=torch.float32)
-        self.best_sweep = z(C, dt=torch.int32)
         self.best_spins = z(C, W, dt=torch.int32)
-        self.sweep_counter = z(1, dt=torch.int64)
-        self.status = z(1, dt=torch.int32)
-        self.ticket = z(1, dt=torch.int32)
+        # the per-chain words in one block: what fetch() reads comes first
+        nb, sv, off = _carve(
+            [("energies", (C, np.float32)), ("beta_idx", (C, np.int32)),
+             ("best_energy", (C, np.float32)), ("best_sweep", (C, np.int32)),
+             ("status", (1, np.int32)), ("ticket", (1, np.int32)),
+             ("sweep_counter", (1, np.int64)), ("chain_beta", (C, np.float32))],
+            host=False)
+        self._small_layout = (sv, off)
+        self._small = z(nb, dt=torch.uint8)
+        for k, t_ in _views(self._small, sv, off).items():
+            setattr(self, k, t_)
         self.log_omega = None
         self.s = _lib.State(_ptr(self.spins), _ptr(self.energies),
                             _ptr(self.beta_idx), _ptr(self.chain_beta),
@@ -574,6 +611,19 @@ class PTBatch:
         self._graphs = {}
         self._P_keep = P  # alive until the stream has read it
 
+    def _slots0(self) -> torch.Tensor:
+        """Temperature slots 0..R-1 of every read (pysa/sa.py:325), on the
+        device; made once per batch."""
+        if not hasattr(self, "_bidx0"):
+            per = self.R.astype(np.int64) * self.Rd
+            b0 = np.zeros(max(self.num_chains, 1), np.int32)
+            if self.num_chains:
+                b0[:] = ((np.arange(self.num_chains) -
+                          np.repeat(self.chain_off, per)) %
+                         np.repeat(np.maximum(self.R, 1), per))
+            self._bidx0 = torch.from_numpy(b0).to(self.device)
+        return self._bidx0
+
     def set_states_device(self, states: torch.Tensor, energies=None,
                           best_global: bool = False):
         """Chains from device float states [num_chains, n] (+-1 or 0/1) of a
@@ -594,12 +644,7 @@ class PTBatch:
         if energies is not None:
             self.energies.copy_(torch.as_tensor(energies).reshape(-1).to(
                 device=self.device, dtype=torch.float32))
-        if not hasattr(self, "_bidx0"):
-            self._bidx0 = torch.from_numpy(np.concatenate([
-                np.tile(np.arange(self.R[i], dtype=np.int32), self.Rd[i])
-                for i in range(len(self.instances))
-            ]) if self.num_chains else np.zeros(1, np.int32)).to(self.device)
-        self.beta_idx.copy_(self._bidx0)
+        self.beta_idx.copy_(self._slots0())
         self.sweep_counter.zero_()
         self.status.zero_()
         self.ticket.zero_()
@@ -634,11 +679,7 @@ class PTBatch:
         if energies is not None:
             self.energies.copy_(torch.from_numpy(
                 np.ascontiguousarray(energies, np.float32).reshape(-1)))
-        bidx = np.concatenate([
-            np.tile(np.arange(self.R[i], dtype=np.int32), self.Rd[i])
-            for i in range(len(self.instances))
-        ]) if self.num_chains else np.zeros(1, np.int32)
-        self.beta_idx.copy_(torch.from_numpy(bidx))
+        self.beta_idx.copy_(self._slots0())
         self.sweep_counter.zero_()
         self.status.zero_()
         self.ticket.zero_()
@@ -714,7 +755,10 @@ class PTBatch:
               "recompute")
 
     def check_status(self):
-        code = int(self.status.item())
+        self._check_code(int(self.status.item()))
+
+    @staticmethod
+    def _check_code(code: int):
         if code != 0:
             what = {-4: "a bounded wait ran out",
                     -6: "energy drift: the accumulated energies left their "
@@ -723,16 +767,41 @@ class PTBatch:
             raise _lib.LibraryError(f"device reported status {code} ({what})")
 
     # --------------------------------------------------------- read back
+    def _to_host(self, t: torch.Tensor) -> np.ndarray:
+        """A device tensor as a new host array.  Large ones pass a pinned
+        buffer of at most 32 MB that the batch keeps: a copy straight into
+        fresh pages has the device fault them in (24.6 MB: 1 to 22 ms; so
+        under 1)."""
+        nb = t.numel() * t.element_size()
+        if nb < 4 << 20:
+            return t.cpu().numpy()
+        if getattr(self, "_pin", None) is None:
+            self._pin = torch.empty(min(nb, 32 << 20), dtype=torch.uint8,
+                                    pin_memory=True)
+        src = t.contiguous().view(-1).view(torch.uint8)
+        out = torch.empty(t.shape, dtype=t.dtype)
+        dst = out.view(-1).view(torch.uint8)
+        step = self._pin.numel()
+        for o in range(0, nb, step):
+            m = min(step, nb - o)
+            self._pin[:m].copy_(src[o:o + m])
+            dst[o:o + m].copy_(self._pin[:m])
+        return out.numpy()
+
     def fetch(self) -> dict:
         torch.cuda.synchronize(self.device)
-        self.check_status()
+        sv, off = self._small_layout
+        end = off["ticket"]  # status and what comes before it: one copy
+        h = _views(self._to_host(self._small[:end]),
+                   {k: v for k, v in sv.items() if off[k] < end}, off)
+        self._check_code(int(h["status"][0]))
         out = dict(
-            spins=self.spins.cpu().numpy().view("<u4"),
-            energies=self.energies.cpu().numpy(),
-            beta_idx=self.beta_idx.cpu().numpy(),
-            best_energy=self.best_energy.cpu().numpy(),
-            best_sweep=self.best_sweep.cpu().numpy(),
-            best_spins=self.best_spins.cpu().numpy().view("<u4"),
+            spins=self._to_host(self.spins).view("<u4"),
+            energies=h["energies"],
+            beta_idx=h["beta_idx"],
+            best_energy=h["best_energy"],
+            best_sweep=h["best_sweep"],
+            best_spins=self._to_host(self.best_spins).view("<u4"),
         )
         if self.log_omega is not None:
             out["log_omega"] = self.log_omega.cpu().numpy()
@@ -788,15 +857,18 @@ def run_ais_batch(problem_type: str, instances: list, temps: np.ndarray, *,
     batch = PTBatch(problem_type, insts, perm_slots=max(len(temps), 1),
                     kernel="plain")
     words = batch.words
-    ns_all = {int(np.asarray(x0).shape[1]) for _, _, x0 in instances}
-    if len(ns_all) == 1:  # one packing call for the whole batch
-        packed = pack_spins(np.concatenate(
-            [np.asarray(x0) for _, _, x0 in instances]), problem_type, words)
+    x0s = [np.asarray(x0) for _, _, x0 in instances]
+    ns_all = {int(x0.shape[1]) for x0 in x0s}
+    if len(ns_all) == 1 and all(x0.dtype == np.float32 for x0 in x0s):
+        # packed (and below unpacked) on the device
+        batch.set_states_device(torch.from_numpy(np.ascontiguousarray(
+            x0s[0] if len(x0s) == 1 else np.concatenate(x0s))))
+    elif len(ns_all) == 1:  # one packing call for the whole batch
+        batch.set_states(pack_spins(np.concatenate(x0s), problem_type, words),
+                         None)
     else:
-        packed = np.concatenate([
-            pack_spins(np.asarray(x0), problem_type, words)
-            for _, _, x0 in instances])
-    batch.set_states(packed, None)
+        batch.set_states(np.concatenate([
+            pack_spins(x0, problem_type, words) for x0 in x0s]), None)
     temps_d = torch.from_numpy(temps).to(batch.device)
     C = max(batch.num_chains, 1)
     log_w = torch.zeros(C, dtype=torch.float64, device=batch.device)
@@ -813,16 +885,17 @@ def run_ais_batch(problem_type: str, instances: list, temps: np.ndarray, *,
           "ais")
     torch.cuda.synchronize(batch.device)
     batch.check_status()
-    spins = batch.spins.cpu().numpy().view("<u4")
     lw = log_w.cpu().numpy()
-    # one unpacking call when every instance has the same n
-    every = (unpack_spins(spins, next(iter(ns_all)), problem_type, np.float32)
-             if len(ns_all) == 1 else None)
+    # one unpacking when every instance has the same n
+    if len(ns_all) == 1:
+        every = batch._to_host(batch.unpack_device())
+    else:
+        spins = batch._to_host(batch.spins).view("<u4")
     out = []
-    for i, (_, _, x0) in enumerate(instances):
-        ns, n = np.asarray(x0).shape
+    for i, x0 in enumerate(x0s):
+        ns, n = x0.shape
         c0 = int(batch.chain_off[i])
-        smp = (every[c0:c0 + ns] if every is not None else
+        smp = (every[c0:c0 + ns] if len(ns_all) == 1 else
                unpack_spins(spins[c0:c0 + ns], n, problem_type, np.float32))
         out.append((smp, lw[c0:c0 + ns]))
     return out

@@ -244,15 +244,15 @@ class Solver(object):
                         return np.random.randint(2, size=(R, N)).astype(
                             self.float_type)
 
-                    def draw_small():
-                        return np.random.randint(2, size=(R, N))
+                    def draw_small(k):
+                        return np.random.randint(2, size=(k, R, N))
                 elif self.problem_type == 'ising':
                     def draw():
                         return 2 * np.random.randint(2, size=(R, N)).astype(
                             self.float_type) - 1
 
-                    def draw_small():
-                        return 2 * np.random.randint(2, size=(R, N)) - 1
+                    def draw_small(k):
+                        return 2 * np.random.randint(2, size=(k, R, N)) - 1
                 else:
                     raise ValueError(
                         f"self.problem_type=='{self.problem_type}' not supported.")
@@ -301,13 +301,16 @@ class Solver(object):
         t0 = time()
         Rd = int(num_reads)
         if Rd and draw_small is not None:
-            # the same NumPy RNG calls, read after read, with the values
-            # (0/1 or +-1) written straight into one int8 array: no float
-            # copies on the host and a quarter of the bytes to the device,
-            # where they become float32 exactly
+            # the same numbers of the NumPy stream, read after read, a few
+            # million values a call, with the values (0/1 or +-1) written
+            # straight into one int8 array: no float copies on the host and
+            # a quarter of the bytes to the device, where they become
+            # float32 exactly
             states0 = np.empty((Rd, R, N), np.int8)
-            for r in range(Rd):
-                states0[r] = draw_small()
+            step = max(1, (1 << 22) // max(R * N, 1))
+            for r in range(0, Rd, step):
+                k = min(step, Rd - r)
+                states0[r:r + k] = draw_small(k)
         elif Rd:
             states0 = np.stack([draw() for _ in range(Rd)])
         else:
@@ -360,15 +363,15 @@ class Solver(object):
         bsp = res['best_spins'].reshape(Rd, R, words)
 
         best_states, best_energies, best_sweeps = [], [], []
-        for r in range(Rd):
-            if parallel:  # pysa/simulation.py:174-177
-                k = int(np.argmin(be[r]))
-                best_states.append(
-                    unpack_spins(bsp[r, k], N, self.problem_type,
-                                 self.float_type))
-                best_energies.append(np.dtype(self.float_type).type(be[r, k]))
-                best_sweeps.append(np.int32(bs[r, k]))
-            else:  # pysa/simulation.py:204-225, strict < in (sweep, replica)
+        if parallel and Rd:  # pysa/simulation.py:174-177
+            at = (np.arange(Rd), np.argmin(be, axis=1))
+            best_states = list(unpack_spins(bsp[at], N, self.problem_type,
+                                            self.float_type))
+            best_energies = list(be[at].astype(self.float_type))
+            best_sweeps = list(bs[at].astype(np.int32))
+        else:
+            for r in range(Rd):
+                # pysa/simulation.py:204-225, strict < in (sweep, replica)
                 order = np.lexsort((np.arange(R), bs[r], be[r]))
                 k = int(order[0])
                 if init_e[r, 0] <= be[r, k]:
@@ -403,17 +406,16 @@ class Solver(object):
             best_energies = [dt.type(x) for x in e64[Rd * R:]]
 
         rows = []
+        with np.errstate(divide='ignore'):
+            temps_all = np.divide(1, np.broadcast_to(betas, (Rd, R))
+                                  if sort_output_temps else betas[bidx])
         for r in range(Rd):
             out_states = out_states_all[r]
             out_energies = energies[r]
             if sort_output_temps:  # pysa/sa.py:380-387
-                out_betas = betas
                 out_states = out_states[bidx[r]]
                 out_energies = out_energies[bidx[r]]
-            else:
-                out_betas = betas[bidx[r]]
-            with np.errstate(divide='ignore'):
-                out_temps = np.divide(1, out_betas)
+            out_temps = temps_all[r]
             row = {
                 'states': out_states,
                 'energies': out_energies,
@@ -457,16 +459,16 @@ class Solver(object):
             logZ0 = _ais.uniform_partition_fun(self.n_vars)
             p = 0.5
 
-            def init():
-                return _ais.uniform_prob_initialization(
-                    self.n_vars, self.problem_type, None)
+            def init(count):
+                return _ais.uniform_samples(self.n_vars, self.problem_type,
+                                            count)
         elif reference_prob == "bernoulli":
             logZ0 = _ais.bernoulli_partition_fun(self.n_vars)
             p = float(reference_args[0])
 
-            def init():
-                return _ais.bernoulli_prob_initialization(
-                    self.n_vars, self.problem_type, reference_args)
+            def init(count):
+                return _ais.bernoulli_samples(self.n_vars, self.problem_type,
+                                              count, reference_args)
         else:
             raise ValueError("Reference Probability not recognized.")
         if update_strategy not in ('random', 'sequential'):
@@ -478,8 +480,8 @@ class Solver(object):
                          dtype=self.float_type)
         couplings = beta * self.couplings.astype(self.float_type)
         local_fields = beta * self.local_fields.astype(self.float_type)
-        initial = np.array([init().astype(self.float_type)
-                            for _ in range(num_samps)])
+        count = len(range(num_samps))
+        initial = init(count).astype(self.float_type) if count else np.array([])
         if seed is None:
             seed = secrets.randbits(64)
         samples, log_omegas = run_ais(
