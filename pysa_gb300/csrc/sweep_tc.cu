@@ -2144,8 +2144,6 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
     } else if (warp == 4) {
       // ============================================================== MMA
       if (lane == 0) {
-        // rows [r_lo, r_hi) of the kTW-row B tile in `slot` against A slice
-        // qq, into the field columns kTW j + r_lo ...
         // Descriptors of the A region's and the B ring's starts, built once:
         // a view or stage further in adds its byte offset / 16 to the
         // address field (shared addresses stay below 2^18, so it never
@@ -2153,42 +2151,54 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
         // deciding warp that is nearly always ready, and every instruction
         // on its path waits for an issue slot, so it keeps few instructions
         // per MMA (microbenchmark: a block's MMA sequence beside such a warp
-        // 10.3k cycles with descriptors built per call, 4.9k prebuilt).
+        // 10.3k cycles with descriptors built per call, 4.9k prebuilt; in place,
+        // 2048 spins, 24 sweeps of 8192 chains: 17.6 ms with 64-bit descriptor
+        // sums, a division a stage and both terms' stages given back together,
+        // 14.3 so; 1024 spins, 500 sweeps of 16384: 48.1 and 45.0).
         const uint64_t a_desc0 =
             tc::smem_desc(smem_base + (uint32_t)C::A_OFF, 128, C::SBO);
         const uint64_t b_desc0 =
             tc::smem_desc(smem_base + (uint32_t)C::B_OFF, 128, C::SBO);
-        auto mma_rows = [&](uint32_t slot, int qq, int j, int r_lo, int r_hi,
-                            uint32_t acc, int ab) {
-          if (r_hi <= r_lo) return;
-          const uint32_t idesc =
-              r_hi - r_lo == kTW
-                  ? idesc_full
-                  : (E8 ? tc::idesc_e4m3(128, r_hi - r_lo)
-                        : tc::idesc_bf16(128, r_hi - r_lo));
-          // slice qq's view: 128 rows starting (128 - CC - qq CC) rows in;
-          // K steps (16 BF16 or 32 E4M3 elements: two core matrices) are
-          // 256 bytes apart: 16 in the address field
-          const uint64_t ad =
-              a_desc0 +
-              (uint64_t)((uint32_t)((128 - CC - qq * CC + 128 * ab) >> 3) *
-                         (C::SBO >> 4));
-          const uint64_t bd =
-              b_desc0 + (uint64_t)(slot * (uint32_t)(C::B_STAGE >> 4) +
-                                   (uint32_t)(r_lo / 8) * (C::SBO >> 4));
+        constexpr uint32_t kRow8 = C::SBO >> 4;  // 8 operand rows further in
+        // A tile columns d of the accumulator += A view ad x B rows bd: K
+        // steps (16 BF16 or 32 E4M3 elements: two core matrices) are 256
+        // bytes apart, 16 in the address field
+        auto mma = [&](uint32_t d, uint32_t ad, uint32_t bd, uint32_t idesc,
+                       uint32_t acc) {
           if constexpr (E8) {
 #pragma unroll
             for (int ks = 0; ks < 2; ++ks)
-              tc::mma_e4m3(taddr + kTW * j + r_lo, ad + 16u * ks,
-                           bd + 16u * ks, idesc, (acc | (uint32_t)ks) ? 1u : 0u);
+              tc::mma_e4m3(d, (a_desc0 & ~0xFFFFFFFFull) | (ad + 16u * ks),
+                           (b_desc0 & ~0xFFFFFFFFull) | (bd + 16u * ks), idesc,
+                           (acc | (uint32_t)ks) ? 1u : 0u);
           } else {
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              tc::mma_bf16(taddr + kTW * j + r_lo, ad + 16u * ks,
-                           bd + 16u * ks, idesc, (acc | (uint32_t)ks) ? 1u : 0u);
+            tc::mma4_bf16(d, ad, (uint32_t)(a_desc0 >> 32), bd,
+                          (uint32_t)(b_desc0 >> 32), idesc, acc);
           }
         };
+        // slice qq's view of A buffer ab: 128 rows starting (128 - CC - qq CC)
+        // rows in
+        auto a_view = [&](int qq, int ab) {
+          return (uint32_t)a_desc0 +
+                 (uint32_t)((128 - CC - qq * CC + 128 * ab) >> 3) * kRow8;
+        };
+        auto b_view = [&](uint32_t sl) {
+          return (uint32_t)b_desc0 + sl * (uint32_t)(C::B_STAGE >> 4);
+        };
+        // instruction descriptor for w columns (N >> 3 at bit 17)
+        auto id_of = [&](int w) {
+          return idesc_full - ((uint32_t)(kTW - w) << 14);
+        };
+        const uint32_t id_last = id_of(S - kTW * (NT - 1));  // a slice's last
         bool ok = true;
+        // ring position of stage u, kept beside it (no division a stage)
+        uint32_t slot = u % C::NS, par = (u / C::NS) & 1;
+        auto next = [&](uint32_t& sl, uint32_t& pr) {
+          if (++sl == (uint32_t)C::NS) {
+            sl = 0;
+            pr ^= 1u;
+          }
+        };
         for (int s = 0; s < KU && ok; ++s) {
           if (rc_at(s)) {
             for (int t = 0; t < NB && ok; ++t) {
@@ -2201,16 +2211,16 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 const int width = S - kTW * j < kTW ? S - kTW * j : kTW;
                 for (int term = 0; term < T && ok; ++term) {
                   for (int qq = 0; qq < F; ++qq) {
-                    const uint32_t slot = u % C::NS;
-                    if (!tc_wait(&sh.full[slot], (u / C::NS) & 1, sh, status)) {
+                    if (!tc_wait(&sh.full[slot], par, sh, status)) {
                       ok = false;
                       break;
                     }
                     tc::fence_after_sync();
-                    mma_rows(slot, qq, j, 0, width,
-                             (t | term | qq) ? 1u : 0u, 0);
+                    mma(taddr + kTW * j, a_view(qq, 0), b_view(slot),
+                        id_of(width), (t | term | qq) ? 1u : 0u);
                     tc::commit(&sh.free_[slot]);
                     ++u;
+                    next(slot, par);
                   }
                 }
               }
@@ -2228,57 +2238,77 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             const int tn = t + 1 < NB ? t + 1 : 0;
             const int qn = (64 * tn) / S, cn = 64 * tn - qn * S;
             const int jf = has_next ? cn / kTW : 0, r0 = cn % kTW;
-            asm volatile("" ::"r"(jf), "r"(r0), "r"(qn));
-            if (!tc_wait(sh.a_full, Gb & 1, sh, status)) {
-              ok = false;
-              break;
-            }
-            stamp(a, Gb, 5);
-            tc::fence_after_sync();
             const int ab = C::A_NBUF == 2 ? (int)(Gb & 1) : 0;
             // stage order: slices from qn on, tiles inside (the critical
             // one first), terms innermost -- consecutive stages write
             // different accumulator tiles, so their MMAs need not wait for
             // one another (the producer issues the same order)
-            for (int k = 0; k < F && ok; ++k) {
-              const int qq = (qn + k) % F;
-              for (int jj = 0; jj < NT && ok; ++jj) {
-                const int j = jj == 0 ? jf : (jj <= jf ? jj - 1 : jj);
-                const int width = S - kTW * j < kTW ? S - kTW * j : kTW;
-                // random order: the next block's columns are scattered, so
-                // no tile is critical; h_ready follows the whole block
-                const bool crit = !RND && jj == 0 && k == 0 && has_next;
-                for (int term = 0; term < T; ++term) {
-                  const uint32_t slot = (u + term) % C::NS;
-                  if (k * NT + jj < 4 && term == 0) stamp(a, Gb, 20 + k * NT + jj);
-                  if (!tc_wait(&sh.full[slot], ((u + term) / C::NS) & 1, sh,
-                               status)) {
-                    ok = false;
-                    break;
-                  }
-                  if (k * NT + jj < 4 && term == 0) stamp(a, Gb, 12 + k * NT + jj);
-                  tc::fence_after_sync();
-                  if (crit)
-                    mma_rows(slot, qq, j, r0, r0 + 64, 1u, ab);
-                  else
-                    mma_rows(slot, qq, j, 0, width, 1u, ab);
-                }
+            uint32_t ad = a_view(qn, ab), d = taddr + kTW * jf;
+            // random order: the next block's columns are scattered, so no
+            // tile is critical; h_ready follows the whole block
+            const bool crit = !RND && has_next;
+            ok = tc_wait(&sh.full[slot], par, sh, status);  // first stage
+            asm volatile("" ::"r"(ad), "r"(d), "r"(r0));
+            if (ok) ok = tc_wait(sh.a_full, Gb & 1, sh, status);
+            if (!ok) break;
+            stamp(a, Gb, 5);
+            tc::fence_after_sync();
+            const int w0 = jf == NT - 1 ? S - kTW * jf : kTW;
+            if (crit) {
+              uint32_t sl = slot, pr = par;
+              for (int term = 0;;) {
+                mma(d + r0, ad, b_view(sl) + (uint32_t)(r0 >> 3) * kRow8,
+                    id_of(64), 1u);
+                if (++term == T) break;
+                next(sl, pr);
+                ok = tc_wait(&sh.full[sl], pr, sh, status);
                 if (!ok) break;
-                if (crit) {
-                  // the next block's decisions may start once these land
-                  tc::commit(sh.h_ready);
-                  stamp(a, Gb, 6);
-                  for (int term = 0; term < T; ++term) {
-                    const uint32_t slot = (u + term) % C::NS;
-                    mma_rows(slot, qq, j, 0, r0, 1u, ab);
-                    mma_rows(slot, qq, j, r0 + 64, width, 1u, ab);
-                  }
+                tc::fence_after_sync();
+              }
+              if (!ok) break;
+              // the next block's decisions may start once these land
+              tc::commit(sh.h_ready);
+              stamp(a, Gb, 6);
+            }
+            for (int term = 0; term < T; ++term) {
+              if (!crit) {
+                if (term > 0) {
+                  ok = tc_wait(&sh.full[slot], par, sh, status);
+                  if (!ok) break;
+                  tc::fence_after_sync();
                 }
-                for (int term = 0; term < T; ++term)
-                  tc::commit(&sh.free_[(u + term) % C::NS]);
-                u += T;
+                mma(d, ad, b_view(slot), id_of(w0), 1u);
+              } else {
+                if (r0 > 0) mma(d, ad, b_view(slot), id_of(r0), 1u);
+                if (w0 > r0 + 64)
+                  mma(d + r0 + 64, ad,
+                      b_view(slot) + (uint32_t)((r0 >> 3) + 8) * kRow8,
+                      id_of(w0 - r0 - 64), 1u);
+              }
+              tc::commit(&sh.free_[slot]);
+              next(slot, par);
+            }
+            int k = 0, jj = 0;
+            for (int i = 1; i < F * NT && ok; ++i) {
+              if (++jj == NT) {
+                jj = 0;
+                ++k;
+                ad = a_view((qn + k) % F, ab);
+              }
+              const int j = jj == 0 ? jf : (jj <= jf ? jj - 1 : jj);
+              const uint32_t id = j == NT - 1 ? id_last : idesc_full;
+              for (int term = 0; term < T; ++term) {
+                if (!tc_wait(&sh.full[slot], par, sh, status)) {
+                  ok = false;
+                  break;
+                }
+                tc::fence_after_sync();
+                mma(taddr + kTW * j, ad, b_view(slot), id, 1u);
+                tc::commit(&sh.free_[slot]);
+                next(slot, par);
               }
             }
+            u += (uint32_t)(F * NT * T);
             if (!ok) break;
             if (!has_next || RND) {
               tc::commit(sh.h_ready);  // one phase per block

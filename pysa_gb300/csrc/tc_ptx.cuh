@@ -227,6 +227,33 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_taddr, uint64_t a_desc,
       : "memory");
 }
 
+// The four K = 16 steps of a 64-wide K tile: operands 256 bytes further in
+// each.  Descriptors as their two words: the step only touches the address
+// field of the low one (no carry), so a step is one 32-bit add an operand.
+__device__ __forceinline__ void mma4_bf16(uint32_t d_taddr, uint32_t a_lo,
+                                          uint32_t a_hi, uint32_t b_lo,
+                                          uint32_t b_hi, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 a, b;\n .reg .b32 x, y;\n"
+      " setp.ne.b32 p, %6, 0;\n"
+      " mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n"
+      " add.u32 x, %1, 16;\n add.u32 y, %3, 16;\n"
+      " mov.b64 a, {x, %2};\n mov.b64 b, {y, %4};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, 1;\n"
+      " add.u32 x, %1, 32;\n add.u32 y, %3, 32;\n"
+      " mov.b64 a, {x, %2};\n mov.b64 b, {y, %4};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, 1;\n"
+      " add.u32 x, %1, 48;\n add.u32 y, %3, 48;\n"
+      " mov.b64 a, {x, %2};\n mov.b64 b, {y, %4};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, 1;\n}\n" ::"r"(
+          d_taddr),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc),
+      "r"(accumulate)
+      : "memory");
+}
+
 // Instruction descriptor, kind::f8f6f4: D f32, A and B E4M3 (format 0),
 // both K-major; N >> 3 at bit 17, M >> 4 at bit 24.
 __host__ __device__ constexpr uint32_t idesc_e4m3(int M, int N) {
