@@ -981,21 +981,21 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
               const bool banded = pvalid && invbs < INFINITY;
               const float band0 = banded ? 3e-5f * invbs : 0.0f;
               const float band1 = banded ? 1e-6f * invbs : 0.0f;
-              float h[32], w[32];
+              uint64_t h2[16], w2[16];  // positions 2 p, 2 p + 1 of the half
               if constexpr (RND) {
 #pragma unroll
-                for (int k = 0; k < 32; ++k)  // positions past n hold nothing
-                  h[k] = 32 * hf + k < kmax ? hbuf[(32 * hf + k) * CC + cc]
-                                            : 0.0f;
+                for (int p = 0; p < 16; ++p) {  // positions past n hold nothing
+                  const int k = 32 * hf + 2 * p;
+                  h2[p] = pack2(k < kmax ? hbuf[k * CC + cc] : 0.0f,
+                                k + 1 < kmax ? hbuf[(k + 1) * CC + cc] : 0.0f);
+                }
               } else {
 #pragma unroll
                 for (int q4 = 0; q4 < 8; ++q4) {
-                  const float4 v = *reinterpret_cast<const float4*>(
+                  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(
                       dl_s + cidx(cc, 32 * hf + 4 * q4));
-                  h[4 * q4 + 0] = v.x;
-                  h[4 * q4 + 1] = v.y;
-                  h[4 * q4 + 2] = v.z;
-                  h[4 * q4 + 3] = v.w;
+                  h2[2 * q4] = v.x;
+                  h2[2 * q4 + 1] = v.y;
                 }
               }
 #pragma unroll
@@ -1003,12 +1003,14 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 const float4 v = *reinterpret_cast<const float4*>(
                     lfb + cidx(cc, 32 * hf + 4 * q4));
                 const float av[4] = {v.x, v.y, v.z, v.w};
+                float wv[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                  const int k = 4 * q4 + i;
                   const float tl = av[i] * invbs;  // -|tl|
-                  w[k] = ((om >> k) & 1u) ? -tl : tl;
+                  wv[i] = ((om >> (4 * q4 + i)) & 1u) ? -tl : tl;
                 }
+                w2[2 * q4] = pack2(wv[0], wv[1]);
+                w2[2 * q4 + 1] = pack2(wv[2], wv[3]);
               }
               const uint64_t live64 =
                   kmax >= 64 ? ~0ull : ((1ull << kmax) - 1ull);
@@ -1034,10 +1036,10 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                   m[qd] = 0u;
                   if (8 * qd + 8 > (int)lo) {
 #pragma unroll
-                    for (int jj = 7; jj >= 0; --jj) {
-                      const int k = 8 * qd + jj;
-                      m[qd] = __funnelshift_l(__float_as_uint(h[k] + w[k]),
-                                              m[qd], 1);
+                    for (int pp = 3; pp >= 0; --pp) {
+                      const uint64_t x = add2(h2[4 * qd + pp], w2[4 * qd + pp]);
+                      m[qd] = __funnelshift_l((uint32_t)(x >> 32), m[qd], 1);
+                      m[qd] = __funnelshift_l((uint32_t)x, m[qd], 1);
                     }
                   }
                 }
@@ -1051,6 +1053,16 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                 // the chain's next decision (positions up to it decided)
                 const int js = c0 ? __ffs(c0) - 1
                                   : (c1 ? 32 + __ffs(c1) - 1 : 0);
+                // what it and its flip will need, on the way while the field
+                // is picked (a candidate is nearly always accepted): with the
+                // paired sums, 1024 spins, 500 sweeps of 16384 chains 45.1 ->
+                // 43.7 ms
+                const float ak = lfb[cidx(cc, js)];
+                ulonglong2 row[8];
+#pragma unroll
+                for (int q4 = 0; q4 < 8; ++q4)
+                  row[q4] = reinterpret_cast<const ulonglong2*>(
+                      jb + js * 64 + 32 * hf)[q4];
                 // its field at decision: the lane holding position js has it
                 // in registers, corrected by this block's earlier flips in
                 // position order (the values and roundings of a rebuild from
@@ -1062,7 +1074,8 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                   const int jl = js & 31;
                   float v16[16], v8[8], v4[4], v2[2];
 #pragma unroll
-                  for (int i = 0; i < 16; ++i) v16[i] = (jl & 16) ? h[i + 16] : h[i];
+                  for (int i = 0; i < 16; ++i)
+                    v16[i] = half2((jl & 16) ? h2[8 + (i >> 1)] : h2[i >> 1], i & 1);
 #pragma unroll
                   for (int i = 0; i < 8; ++i) v8[i] = (jl & 8) ? v16[i + 8] : v16[i];
 #pragma unroll
@@ -1085,7 +1098,6 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                   const bool sbit =
                       ((js < 32 ? o0 >> js : o1 >> (js - 32)) & 1u) != 0u;
                   const float x = sbit ? hj : -hj;
-                  const float ak = lfb[cidx(cc, js)];
                   const float th = fminf(
                       fmaf(2.0f * band1, fabsf(ak), fmaf(ak, invbs, 2.0f * band0)),
                       0.0f);
@@ -1101,15 +1113,11 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                     flips64 |= bit;
                     const float dl = sbit ? -scale : scale;
                     dEb = fmaf(dl, hj, dEb);  // dl h = -dn
-                    const float4* row =
-                        reinterpret_cast<const float4*>(jb + js * 64 + 32 * hf);
+                    const uint64_t dd = pack2(dl, dl);
 #pragma unroll
                     for (int q4 = 0; q4 < 8; ++q4) {
-                      const float4 v = row[q4];
-                      h[4 * q4 + 0] = fmaf(dl, v.x, h[4 * q4 + 0]);
-                      h[4 * q4 + 1] = fmaf(dl, v.y, h[4 * q4 + 1]);
-                      h[4 * q4 + 2] = fmaf(dl, v.z, h[4 * q4 + 2]);
-                      h[4 * q4 + 3] = fmaf(dl, v.w, h[4 * q4 + 3]);
+                      h2[2 * q4] = fma2(dd, row[q4].x, h2[2 * q4]);
+                      h2[2 * q4 + 1] = fma2(dd, row[q4].y, h2[2 * q4 + 1]);
                     }
                   }
                 }
