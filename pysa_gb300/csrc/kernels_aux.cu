@@ -56,14 +56,39 @@ __device__ __forceinline__ int chain_instance(const pysa_gb_problems& p,
   return lo;
 }
 
+// s + e = a + b exactly (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float& e) {
+  const float s = a + b;
+  const float bb = s - a;
+  e = (a - (s - bb)) + (b - bb);
+  return s;
+}
+
+// Three f32 a value: the sum to 2^-72 of its largest term.
+struct Triple {
+  float a, b, c;
+  __device__ __forceinline__ void add(float x) {
+    float e, f;
+    a = two_sum(a, x, e);
+    b = two_sum(b, e, f);
+    c += f;
+  }
+  __device__ __forceinline__ float rounded() const {
+    float e;
+    const float s = two_sum(a, b, e);
+    return s + (e + c);
+  }
+};
+
 // Sparse instances: f_i = sum over row i's stored entries of J_ij s_j in f64
 // (the products are exact; padding entries have value 0), from the fixed
 // records (width > 0: entries csr_ent_off + width i ...) or the grouped
 // rows (csr_rows, 9 offsets per row).
-__device__ __forceinline__ double csr_row_dot(const pysa_gb_problems& p,
+template <typename Add>
+__device__ __forceinline__ void csr_row_terms(const pysa_gb_problems& p,
                                               int inst, int i,
-                                              const uint32_t* sw,
-                                              bool ising) {
+                                              const uint32_t* sw, bool ising,
+                                              Add add) {
   const int64_t eo = p.csr_ent_off[inst];
   int64_t beg, end;
   if (p.csr_width > 0) {
@@ -74,13 +99,19 @@ __device__ __forceinline__ double csr_row_dot(const pysa_gb_problems& p,
     beg = eo + r[0];
     end = eo + r[8];
   }
-  double f = 0.0;
   for (int64_t e = beg; e < end; ++e) {
     const int j = p.csr_col[e] & 0x7fffffff;
     const float sj = ((sw[j >> 5] >> (j & 31)) & 1u) ? 1.0f
                                                      : (ising ? -1.0f : 0.0f);
-    f += (double)(p.csr_val[e] * sj);
+    add(p.csr_val[e] * sj);
   }
+}
+__device__ __forceinline__ double csr_row_dot(const pysa_gb_problems& p,
+                                              int inst, int i,
+                                              const uint32_t* sw,
+                                              bool ising) {
+  double f = 0.0;
+  csr_row_terms(p, inst, i, sw, ising, [&](float x) { f += (double)x; });
   return f;
 }
 
@@ -89,9 +120,14 @@ __device__ __forceinline__ bool is_sparse_inst(const pysa_gb_problems& p,
   return p.csr_row_off && p.csr_row_off[inst] >= 0;
 }
 
+// CTA per chain, thread per row.  Sums in triples of f32 (f64 instructions run
+// at 1/64 of the rate; they took most of 417 us for 4000 chains of 4096 spins
+// with 4 couplings each, 146 so); a field or energy that leaves the f32
+// range is added in f64.
 __global__ void __launch_bounds__(32 * kFieldWarps)
     k_fields_csr(const PrepArgs a) {
-  __shared__ double e_s[kFieldWarps];
+  __shared__ Triple e_s[kFieldWarps];
+  __shared__ double d_s[kFieldWarps];
   const int64_t c = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
@@ -101,20 +137,64 @@ __global__ void __launch_bounds__(32 * kFieldWarps)
   const bool ising = a.p.problem_type == PYSA_GB_ISING;
   const float* h = a.p.h + a.p.h_off[inst];
   const uint32_t* sw = a.s.spins + c * a.p.words;
-  double e = 0.0;
+  auto spin = [&](int i) {
+    return ((sw[i >> 5] >> (i & 31)) & 1u) ? 1.0f : (ising ? -1.0f : 0.0f);
+  };
+  Triple e = {0.0f, 0.0f, 0.0f};  // sum_i s_i (f_i + 2 h_i)
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double f = csr_row_dot(a.p, inst, i, sw, ising);
-    const uint32_t bit = (sw[i >> 5] >> (i & 31)) & 1u;
-    const double si = bit ? 1.0 : (ising ? -1.0 : 0.0);
-    e += si * (0.5 * f + (double)h[i]);
-    a.fields[c * a.field_ld + i] = (float)(f + (double)h[i]);
+    Triple f = {0.0f, 0.0f, 0.0f};
+    csr_row_terms(a.p, inst, i, sw, ising, [&](float x) { f.add(x); });
+    const float hi = h[i], si = spin(i);
+    e.add(si * f.a);
+    e.add(si * f.b);
+    e.add(si * f.c);
+    e.add(si * (2.0f * hi));
+    f.add(hi);
+    float H = f.rounded();
+    if (!(fabsf(H) < INFINITY))
+      H = (float)(csr_row_dot(a.p, inst, i, sw, ising) + (double)hi);
+    a.fields[c * a.field_ld + i] = H;
   }
-  e = warp_sum(e);
-  if (lane == 0) e_s[warp] = e;
+  if (!a.set_energies) return;
+  const bool bad = __syncthreads_or(!(fabsf(e.a) < INFINITY));
+  if (!bad) {
+    for (int o = 16; o; o >>= 1) {
+      const Triple u = {__shfl_xor_sync(0xffffffffu, e.a, o),
+                        __shfl_xor_sync(0xffffffffu, e.b, o),
+                        __shfl_xor_sync(0xffffffffu, e.c, o)};
+      e.add(u.a);
+      e.add(u.b);
+      e.add(u.c);
+    }
+    if (lane == 0) e_s[warp] = e;
+  } else {
+    double d = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      d += (double)spin(i) * (0.5 * csr_row_dot(a.p, inst, i, sw, ising) +
+                              (double)h[i]);
+    d = warp_sum(d);
+    if (lane == 0) d_s[warp] = d;
+  }
   __syncthreads();
-  if (threadIdx.x == 0 && a.set_energies) {
+  if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int w = 0; w < nwarps; ++w) t += e_s[w];
+    if (bad) {
+      for (int w = 0; w < nwarps; ++w) t += d_s[w];
+    } else {
+      Triple s = e_s[0];
+      for (int w = 1; w < nwarps; ++w) {
+        s.add(e_s[w].a);
+        s.add(e_s[w].b);
+        s.add(e_s[w].c);
+      }
+      t = 0.5 * ((double)s.a + ((double)s.b + (double)s.c));
+      if (!(fabsf(s.a) < INFINITY)) {  // the warps' sum left the range
+        t = 0.0;
+        for (int i = 0; i < n; ++i)
+          t += (double)spin(i) * (0.5 * csr_row_dot(a.p, inst, i, sw, ising) +
+                                  (double)h[i]);
+      }
+    }
     a.s.energies[c] = (float)t;
   }
 }
@@ -141,14 +221,6 @@ __global__ void __launch_bounds__(32 * kFieldWarps)
 // 1.3 -> 0.96; n = 512, 65536 chains 1.19 -> 0.95 (single multiply-adds before;
 // one CTA per chain with f64 accumulation took 14.2 ms at n = 2048, 9728
 // chains, this tile 2.7 with single multiply-adds).
-
-// s + e = a + b exactly (Knuth's two-sum).
-__device__ __forceinline__ float two_sum(float a, float b, float& e) {
-  const float s = a + b;
-  const float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
-  return s;
-}
 
 // Pair (hi, lo) + x.
 __device__ __forceinline__ void pair_add(float2& p, float x) {
