@@ -345,8 +345,9 @@ int pysa_gb_tc_setup(const pysa_gb_problems *p,
                      const pysa_gb_host_tables *host, pysa_gb_workspace *ws,
                      void *stream);
 
-/* Local fields H = J s + h for every chain, accumulated in f64 from f32
- * products, and (if set_energies) energies E = s.(J s / 2 + h)
+/* Local fields H = J s + h for every chain, f32 products added up in f32
+ * pairs by exact two-sums (in f64 where a sum leaves the f32 range) and
+ * rounded once, and (if set_energies) energies E = s.(J s / 2 + h)
  * (pysa/ising.py:32-37, pysa/qubo.py:32-37).  Also sets chain_beta from
  * beta_idx and, if init_best, best_* from the current state
  * (best_global: best_energy = +inf). */

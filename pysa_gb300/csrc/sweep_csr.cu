@@ -23,8 +23,8 @@
 // Bound by instruction issue and, per level, by the latency of one quad's four
 // dependent attempts.  Measured against one thread per chain visiting the
 // positions one by one (times per sweep with the exchange): 64 x 64 lattice,
-// 4000 chains 1.44 -> 0.13 ms in visiting order (79 levels), 1.66 -> 0.44 ms
-// in random order (most of the rest makes the orders); 100 x 100, 2000 chains
+// 4000 chains 1.44 -> 0.13 ms in visiting order (79 levels), 1.66 -> 0.25 ms
+// in random order (half of it makes the orders and the schedule); 100 x 100, 2000 chains
 // 3.7 -> 0.39 ms; 33 x 33, 16000 chains 0.43 -> 0.19 ms.
 //
 // Row layout: the entries of row i are grouped by column % 8 (ascending

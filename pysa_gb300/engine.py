@@ -3,7 +3,7 @@
 `PTBatch` owns the device buffers of a batch of dense instances (uneven sizes
 allowed), their chains (instance x read x replica) and the workspace, and
 drives libpysa_gb: set-up (coupling packing, work list), preparation (local
-fields and energies in f64), sweeps with replica exchange (optionally replayed
+fields and energies), sweeps with replica exchange (optionally replayed
 from a captured CUDA graph) and read-back.  PyTorch only provides device
 memory and the stream.
 """
@@ -748,7 +748,7 @@ class PTBatch:
 
     def recompute(self):
         """Fields and energies of every chain from its spins (f32 partial
-        sums accumulated in f64); best_* untouched."""
+        sums accumulated in f32 pairs); best_* untouched."""
         check(self.lib.pysa_gb_prepare(ref(self.p), ref(self.s), ref(self.ws),
                                        1, 0, int(self.best_global),
                                        self._stream.cuda_stream),
