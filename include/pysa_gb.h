@@ -300,8 +300,8 @@ int pysa_gb_set_decision_mode(int32_t mode);
 
 /* Decision mode 0's switch point: a block is decided in rounds while the
  * previous block's largest flip count of a chain was at most `flips`
- * (0..64; until the first call 12, and 6 for n > 1024), in sequential
- * sub-blocks otherwise.  Same decisions for every value; process-wide, for
+ * (0..64; until the first call 12, and 4 for n > 1024 and, up to n = 512,
+ * in work items of at most 32 chains), in sequential sub-blocks otherwise.  Same decisions for every value; process-wide, for
  * launches enqueued after the call.  No counterpart in the reference. */
 int pysa_gb_set_block_round_limit(int32_t flips);
 

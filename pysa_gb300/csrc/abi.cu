@@ -55,7 +55,7 @@ static unsigned long long* g_tc_trace = nullptr;  // diagnostics, see below
 static uint64_t g_unit_wait_ns = 0;  // diagnostics: 0 = the default bound
 static int32_t g_decision_mode = 0;   // tensor-core sweep: 0 auto, 1, 2
 static int32_t g_round_limit = -1;    // mode 0: block rounds up to this many
-                                      // flips; -1: by fold (tc_round_limit)
+                                      // flips; -1: tc_round_limit
 static int32_t g_tc_max_ctas = 0;     // tensor-core launches: 0 = SM count
 
 static int fail(int code, const std::string& msg) {
@@ -75,15 +75,22 @@ static int cuda_fail(cudaError_t e, const char* where) {
 // Default for the most sweeps one fused tensor-core launch covers.
 constexpr int kMaxFusedSweeps = 128;
 
-// Flips of a chain up to which the next 64-spin block is decided in rounds.
-// Fold 2 shares a chain's rounds between two lanes (visiting order) and gains
-// from them longest; at fold 4 one lane tests all 64 positions, about 1400
-// cycles a round against 14000 for the block in sequential sub-blocks.
-// Measured, ms per sweep at limits 6 / 8 / 12 / 16: Wishart n = 2048 (fold 4)
-// 0.789 / 0.807 / 0.885 / 1.064; integer QUBO n = 2000 0.2069 / 0.2073 /
-// 0.2092 / 0.2124, n = 1024 (fold 2) 0.1046 / 0.1039 / 0.1041 / 0.1046, n =
-// 300 (fold 1) 0.0704 / 0.0651 / 0.0645 / 0.0644.
-static int tc_round_limit(int fold) { return fold == 4 ? 6 : 12; }
+// Flips of a chain up to which the next 64-spin block is decided in rounds
+// (a round costs 0.8 to 1.4 thousand cycles).  Fold 2 shares a chain's rounds
+// between two lanes and gains from them longest; where the block's sub-blocks
+// go through the four warps in a relay (fold 4, and fold 1 in items of at most
+// 32 chains) the whole block takes 6 to 8 thousand cycles in sequential form,
+// 13 thousand otherwise.  Fold 2 keeps its limit in the relay too: there the
+// two forms round differently.  Measured, ms per sweep at limits 2 / 4 / 6 /
+// 8 / 12: Wishart n = 2048 (fold 4) 0.611 / 0.612 / 0.612 / 0.648 / 0.790, n =
+// 1500 cold 0.426 / 0.449 / 0.470 / 0.476 / 0.499; integer QUBO n = 2000 0.1836
+// / 0.1764 / 0.1771 / 0.1784 / 0.1812; fold 1 relayed, n = 300 0.0249 / 0.0249 /
+// 0.0251 / 0.0266 / 0.0407, +-1 n = 200 0.0188 / 0.0184 / 0.0184 / 0.0183 /
+// 0.0183.  At 6 / 8 / 12 / 16: n = 1024 (fold 2) 0.1046 / 0.1039 / 0.1041 /
+// 0.1046, n = 300 (fold 1, one warp) 0.0704 / 0.0651 / 0.0645 / 0.0644.
+static int tc_round_limit(int fold, bool relay) {
+  return fold != 2 && relay ? 4 : 12;
+}
 
 // Most sweeps of one launch of the resident small sweep (about a
 // millisecond each thousand).
@@ -783,8 +790,12 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       ta.fuse_exchange = fuse;
       ta.advance_counter = fuse && v == last_v && !small_live;
       ta.log_omega_stride = fuse ? o->log_omega_stride : 0;
-      ta.round_limit = g_round_limit >= 0 ? g_round_limit
-                                          : tc_round_limit(folds[v]);
+      ta.round_limit = g_round_limit >= 0
+                           ? g_round_limit
+                           : tc_round_limit(folds[v], false);
+      ta.relay_round_limit = g_round_limit >= 0
+                                 ? g_round_limit
+                                 : tc_round_limit(folds[v], true);
       e = launch_tc(ta, folds[v], random, sms, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc sweep launch");
     }

@@ -46,9 +46,10 @@ namespace pysa_gb {
 constexpr int kTW = 256;
 
 // Decision mode of a block: block rounds (D64) while the previous block's
-// largest flip count of any chain was at most TcArgs::round_limit (12, and 6
-// at fold 4, by default), else sequential sub-blocks.  A round costs about as much as 6-10
-// sequential spins, so the rounds win while flips are rare.
+// largest flip count of any chain was at most TcArgs::round_limit (by default
+// 12, and 4 where the sub-blocks are relayed at folds 1 and 4), else sequential
+// sub-blocks.  A round costs about as much as 6-10 sequential spins, so the
+// rounds win while flips are rare.
 
 // RND: random visiting order (one permutation per instance and sweep); the
 // B ring keeps two stages to make room for the gathered block fields.
@@ -648,6 +649,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
     const bool valid = warp < 4 && c < item.nchains;
     // sequential sub-blocks one warp each (below)
     const bool relay = F == 4 || item.nchains <= 32;
+    const int round_limit = relay ? a.relay_round_limit : a.round_limit;
     const int64_t chain = item.chain0 + c;
     const uint32_t chain_local = (uint32_t)(chain - chain_base);
     const uint32_t G0 = G, RG0 = RG;
@@ -1991,8 +1993,8 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             // where the two forms round differently)
             d64 = a.decision_mode == 1 ||
                   (a.decision_mode == 0 &&
-                   (F == 2 ? (int)mf <= a.round_limit
-                           : (int)mf * 64 <= a.round_limit * kmax));
+                   (F == 2 ? (int)mf <= round_limit
+                           : (int)mf * 64 <= round_limit * kmax));
           }
           if (threadIdx.x == 0) {
             stamp(a, Gb, 4);

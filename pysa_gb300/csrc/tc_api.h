@@ -42,7 +42,8 @@ struct TcArgs {
                           // (0: one second)
   int32_t decision_mode;  // 0 per-block choice, 1 block rounds, 2 sub-blocks
   int32_t round_limit;    // mode 0: block rounds while the previous block's
-                          // largest flip count of a chain is at most this
+                          // largest flip count of a chain is at most this,
+  int32_t relay_round_limit;  // or this in items whose sub-blocks are relayed
   int32_t* sched;  // zeroed per launch: [0] unit queue, [1] finished CTAs,
                    // [2 + item] sweeps of the item run in this launch
   // random order: permutation of (inst, sweep) at
