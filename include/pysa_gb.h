@@ -180,7 +180,8 @@ typedef struct {
                                at most the chains per CTA, and the chain
                                slots left empty worth it */
   int32_t *tc_sched;        /* [2 + tc_num_items] device scratch of the
-                               persistent tensor-core kernel */
+                               persistent tensor-core kernel, zeroed by
+                               every call */
   int32_t tc_unit_sweeps;   /* sweeps per work unit of that kernel (0: 8) */
   int32_t tc_launch_sweeps; /* most sweeps one launch of it covers (0: 128) */
   /* random visiting order on the tensor cores: J tiles and diagonal blocks
@@ -292,17 +293,23 @@ int pysa_gb_set_unit_wait_limit(uint64_t ns);
  * chooses per block -- rounds over the whole block while the previous
  * block's largest flip count of a chain was small, sequential 16-spin
  * sub-blocks otherwise; 1 always rounds; 2 always sub-blocks.  Every mode
- * makes the same decisions (the rule of pysa/ising.py:40-63 and
- * pysa/qubo.py:40-63 in the visiting order); only the speed differs, and
- * tests pin both forms.  Applies to launches enqueued after the call,
- * process-wide.  No counterpart in the reference. */
+ * follows the same rule (pysa/ising.py:40-63 and pysa/qubo.py:40-63) in the
+ * visiting order, and a run repeats itself bit for bit in each.  The modes
+ * give the same bits where n <= 512, n > 1024, or every field sum is exact in
+ * f32 (integer couplings); for 512 < n <= 1024 with other couplings the two
+ * forms add the corrections inside a block in different orders, so that a
+ * field, and with it an energy, may differ in its last bit, and a decision
+ * or exchange that lies within that of its threshold may fall otherwise.
+ * Applies to launches enqueued after the call, process-wide.  No counterpart
+ * in the reference. */
 int pysa_gb_set_decision_mode(int32_t mode);
 
 /* Decision mode 0's switch point: a block is decided in rounds while the
  * previous block's largest flip count of a chain was at most `flips`
  * (0..64; until the first call 12, and 4 for n > 1024 and, up to n = 512,
- * in work items of at most 32 chains), in sequential sub-blocks otherwise.  Same decisions for every value; process-wide, for
- * launches enqueued after the call.  No counterpart in the reference. */
+ * in work items of at most 32 chains), in sequential sub-blocks otherwise.
+ * Results depend on it as on the decision mode; process-wide, for launches
+ * enqueued after the call.  No counterpart in the reference. */
 int pysa_gb_set_block_round_limit(int32_t flips);
 
 /* Most CTAs of a tensor-core sweep launch (0, the default: one per SM).

@@ -81,7 +81,8 @@ constexpr int kMaxFusedSweeps = 128;
 // go through the four warps in a relay (fold 4, and fold 1 in items of at most
 // 32 chains) the whole block takes 6 to 8 thousand cycles in sequential form,
 // 13 thousand otherwise.  Fold 2 keeps its limit in the relay too: there the
-// two forms round differently.  Measured, ms per sweep at limits 2 / 4 / 6 /
+// two forms round differently, and the limit is part of the result's last
+// bits.  Measured, ms per sweep at limits 2 / 4 / 6 /
 // 8 / 12: Wishart n = 2048 (fold 4) 0.611 / 0.612 / 0.612 / 0.648 / 0.790, n =
 // 1500 cold 0.426 / 0.449 / 0.470 / 0.476 / 0.499; integer QUBO n = 2000 0.1836
 // / 0.1764 / 0.1771 / 0.1784 / 0.1812; fold 1 relayed, n = 300 0.0249 / 0.0249 /
@@ -774,13 +775,20 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
   // one persistent tensor-core launch per fold: `units` work units of
   // `ku` sweeps per item (or wrap-around units over ku * units sweeps),
   // exchange fused or not
+  uint32_t tc_swept = 0;  // sweeps that this call's launches have covered
   auto tc_launches = [&](int ku, int units, int fuse) -> int {
     for (int v = 0; v < 3; ++v) {
       const int count = ws->tc_variant_count[v];
       if (count == 0) continue;
-      cudaError_t e = cudaMemsetAsync(ws->tc_sched, 0,
-                                      sizeof(int32_t) * (2 + (size_t)count), st);
+      // the queue, and before a fold's first launch its items' progress
+      int32_t* done = ws->tc_sched + 2 + ws->tc_variant_start[v];
+      cudaError_t e =
+          cudaMemsetAsync(ws->tc_sched, 0, 2 * sizeof(int32_t), st);
+      if (e == cudaSuccess && tc_swept == 0)
+        e = cudaMemsetAsync(done, 0, sizeof(int32_t) * (size_t)count, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc schedule reset");
+      ta.item_done = reinterpret_cast<uint32_t*>(done);
+      ta.sweeps_before = tc_swept;
       ta.items = reinterpret_cast<const TcItem*>(ws->tc_items) +
                  ws->tc_variant_start[v];
       ta.num_items = count;
@@ -799,6 +807,7 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       e = launch_tc(ta, folds[v], random, sms, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc sweep launch");
     }
+    tc_swept += (uint32_t)(ku * units);
     return PYSA_GB_OK;
   };
   // Fused: every instance either on the tensor cores with whole reads per

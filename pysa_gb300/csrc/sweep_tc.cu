@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
                                           // buffer 0 / 1 (two buffers)
   sh.tmem_slot = reinterpret_cast<uint32_t*>(smem + C::MISC_OFF);
   sh.abort = reinterpret_cast<volatile int32_t*>(smem + C::MISC_OFF + 8);
-  volatile int32_t* unit_s =  // [item, first sweep, sweeps] of the unit
+  volatile int32_t* unit_s =  // [item, first sweep, sweeps, form] of the unit
       reinterpret_cast<volatile int32_t*>(smem + C::MISC_OFF + 16);
   volatile uint32_t* stat_s =
       reinterpret_cast<volatile uint32_t*>(smem + C::STAT_OFF);
@@ -584,15 +584,13 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
   uint32_t G = 0;   // blocks
   uint32_t RG = 0;  // recompute blocks
   uint32_t u = 0;   // B ring stages (producer and MMA)
-  // decision warps: this block's decision mode (the same in all 128 threads);
-  // sequential until a block shows few flips
-  bool d64 = a.decision_mode == 1;
   int share = -1, piece = 0;  // thread 0, wrap-around units
 
   for (;;) {
     // ------------------------------------------------------ next unit
     if (threadIdx.x == 0) {
       int it = -1, sb = 0, sl = 0;
+      bool form = false;  // the unit's first block in rounds
       if (!*sh.abort) {
         if (a.wrap) {
           if (share < 0)
@@ -610,12 +608,14 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
           }
         }
         if (it >= 0) {
-          volatile int32_t* done = a.sched + 2 + it;  // sweeps run
-          if (*done < sb) {
+          // 2 x sweeps run + the form of the item's next block
+          volatile uint32_t* done = a.item_done + it;
+          const uint32_t need = a.sweeps_before + (uint32_t)sb;
+          if (sb > 0 && (*done >> 1) < need) {
             const uint64_t lim =
                 a.unit_wait_ns ? a.unit_wait_ns : 1000000000ull;
             const uint64_t t0 = globaltimer_ns();
-            while (*done < sb) {
+            while ((*done >> 1) < need) {
               if (globaltimer_ns() - t0 > lim) {
                 set_status(status, PYSA_GB_ERR_TIMEOUT);
                 *sh.abort = 1;
@@ -625,17 +625,26 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             }
           }
           __threadfence();  // the previous unit's stores are visible
+          form = a.decision_mode == 1 ||
+                 (a.decision_mode == 0 && (*done & 1u) != 0u);
         }
       }
       unit_s[0] = it;
       unit_s[1] = sb;
       unit_s[2] = sl;
+      unit_s[3] = form ? 1 : 0;
     }
     __syncthreads();
     const int un_item = unit_s[0];
     if (un_item < 0) break;
     const int un_first = unit_s[1];
     const int KU = unit_s[2];
+    // decision warps: this block's decision form (the same in all 128
+    // threads).  An item's first block of a call is decided in sequential
+    // sub-blocks, and a unit goes on in the form of the item's unit before it:
+    // not in the form this CTA's last unit ended in, since which unit that was
+    // depends on timing, and at fold 2 the two forms round differently
+    bool d64 = unit_s[3] != 0;
     const TcItem item = a.items[un_item];
     const uint32_t sweep_first = sweep0 + (uint32_t)un_first;
     const int inst = item.inst;
@@ -2535,8 +2544,9 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
     if (threadIdx.x == 0) {
       stamp_cta(a, 4);
       __threadfence();  // this unit's stores before its done flag
-      atomicExch(reinterpret_cast<int*>(a.sched + 2 + un_item),
-                 un_first + KU);
+      atomicExch(a.item_done + un_item,
+                 2u * (a.sweeps_before + (uint32_t)(un_first + KU)) +
+                     (d64 ? 1u : 0u));
     }
   }
 

@@ -44,8 +44,11 @@ struct TcArgs {
   int32_t round_limit;    // mode 0: block rounds while the previous block's
                           // largest flip count of a chain is at most this,
   int32_t relay_round_limit;  // or this in items whose sub-blocks are relayed
-  int32_t* sched;  // zeroed per launch: [0] unit queue, [1] finished CTAs,
-                   // [2 + item] sweeps of the item run in this launch
+  int32_t* sched;  // zeroed per launch: [0] unit queue, [1] finished CTAs
+  // zeroed per call: [item] 2 x its sweeps run in this call + 1 when its next
+  // block is to be decided in rounds
+  uint32_t* item_done;
+  uint32_t sweeps_before;  // sweeps of the call's earlier launches
   // random order: permutation of (inst, sweep) at
   // perm[((sweep % perm_slots) * num_instances + inst) * max_n]; tiles and
   // diagonal blocks repacked in that order at slot sweep % rand_slots
