@@ -305,12 +305,16 @@ int pysa_gb_set_unit_wait_limit(uint64_t ns);
 int pysa_gb_set_decision_mode(int32_t mode);
 
 /* Decision mode 0's switch point: a block is decided in rounds while the
- * previous block's largest flip count of a chain was at most `flips`
- * (0..64; until the first call 12, and 4 for n > 1024 and, up to n = 512,
- * in work items of at most 32 chains), in sequential sub-blocks otherwise.
- * Results depend on it as on the decision mode; process-wide, for launches
+ * previous block's largest flip count of a chain was at most `flips` (0..64),
+ * in sequential sub-blocks otherwise.  12, the default, is 4 for n > 1024 and,
+ * up to n = 512, in work items of at most 32 chains.  Results depend on it as on the decision mode; process-wide, for launches
  * enqueued after the call.  No counterpart in the reference. */
 int pysa_gb_set_block_round_limit(int32_t flips);
+
+/* The switch point that mode 0 would use now for an instance of n spins (64
+ * .. 2048) in work items of `chains` chains, or an error; for tests and tools.
+ * No counterpart in the reference. */
+int pysa_gb_tc_round_limit(int32_t n, int32_t chains);
 
 /* Most CTAs of a tensor-core sweep launch (0, the default: one per SM).
  * Results do not depend on it; a smaller value leaves SMs to other work and

@@ -54,8 +54,8 @@ static thread_local std::string g_last_error;
 static unsigned long long* g_tc_trace = nullptr;  // diagnostics, see below
 static uint64_t g_unit_wait_ns = 0;  // diagnostics: 0 = the default bound
 static int32_t g_decision_mode = 0;   // tensor-core sweep: 0 auto, 1, 2
-static int32_t g_round_limit = -1;    // mode 0: block rounds up to this many
-                                      // flips; -1: tc_round_limit
+static int32_t g_round_limit = 12;    // mode 0: block rounds up to this many
+                                      // flips (see tc_round_limit)
 static int32_t g_tc_max_ctas = 0;     // tensor-core launches: 0 = SM count
 
 static int fail(int code, const std::string& msg) {
@@ -82,15 +82,16 @@ constexpr int kMaxFusedSweeps = 128;
 // 32 chains) the whole block takes 6 to 8 thousand cycles in sequential form,
 // 13 thousand otherwise.  Fold 2 keeps its limit in the relay too: there the
 // two forms round differently, and the limit is part of the result's last
-// bits.  Measured, ms per sweep at limits 2 / 4 / 6 /
-// 8 / 12: Wishart n = 2048 (fold 4) 0.611 / 0.612 / 0.612 / 0.648 / 0.790, n =
-// 1500 cold 0.426 / 0.449 / 0.470 / 0.476 / 0.499; integer QUBO n = 2000 0.1836
-// / 0.1764 / 0.1771 / 0.1784 / 0.1812; fold 1 relayed, n = 300 0.0249 / 0.0249 /
-// 0.0251 / 0.0266 / 0.0407, +-1 n = 200 0.0188 / 0.0184 / 0.0184 / 0.0183 /
-// 0.0183.  At 6 / 8 / 12 / 16: n = 1024 (fold 2) 0.1046 / 0.1039 / 0.1041 /
+// bits.  Measured, ms per sweep at limits 2 / 4 / 6 / 8 / 12: Wishart n = 2048
+// (fold 4) 0.611 / 0.612 / 0.612 / 0.648 / 0.790, n = 1500 cold 0.426 / 0.449 /
+// 0.470 / 0.476 / 0.499; integer QUBO n = 2000 0.1836 / 0.1764 / 0.1771 /
+// 0.1784 / 0.1812; fold 1 relayed, n = 300 0.0249 / 0.0249 / 0.0251 / 0.0266 /
+// 0.0407, +-1 n = 200 0.0188 / 0.0184 / 0.0184 / 0.0183 / 0.0183.  At 6 / 8 / 12 / 16: n = 1024 (fold 2) 0.1046 / 0.1039 / 0.1041 /
 // 0.1046, n = 300 (fold 1, one warp) 0.0704 / 0.0651 / 0.0645 / 0.0644.
+// The default, 12, stands for this choice; any other value the caller sets is
+// taken everywhere.
 static int tc_round_limit(int fold, bool relay) {
-  return fold != 2 && relay ? 4 : 12;
+  return g_round_limit == 12 && fold != 2 && relay ? 4 : g_round_limit;
 }
 
 // Most sweeps of one launch of the resident small sweep (about a
@@ -175,6 +176,13 @@ int pysa_gb_set_block_round_limit(int32_t flips) {
     return fail(PYSA_GB_ERR_ARG, "block round limit must be in 0..64");
   g_round_limit = flips;
   return PYSA_GB_OK;
+}
+
+int pysa_gb_tc_round_limit(int32_t n, int32_t chains) {
+  if (n < 64 || n > 2048 || chains < 1)
+    return fail(PYSA_GB_ERR_ARG, "round limit: bad arguments");
+  const int fold = 128 / tc_chains_per_cta(n);
+  return tc_round_limit(fold, fold == 4 || chains <= 32);
 }
 
 int pysa_gb_set_tc_max_ctas(int32_t ctas) {
@@ -798,12 +806,8 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       ta.fuse_exchange = fuse;
       ta.advance_counter = fuse && v == last_v && !small_live;
       ta.log_omega_stride = fuse ? o->log_omega_stride : 0;
-      ta.round_limit = g_round_limit >= 0
-                           ? g_round_limit
-                           : tc_round_limit(folds[v], false);
-      ta.relay_round_limit = g_round_limit >= 0
-                                 ? g_round_limit
-                                 : tc_round_limit(folds[v], true);
+      ta.round_limit = tc_round_limit(folds[v], false);
+      ta.relay_round_limit = tc_round_limit(folds[v], true);
       e = launch_tc(ta, folds[v], random, sms, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc sweep launch");
     }
