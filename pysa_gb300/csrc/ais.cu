@@ -552,6 +552,10 @@ static cudaError_t launch_ais_t(const AisArgs& a, int64_t max_samples,
   return cudaGetLastError();
 }
 
+// Widest instance whose couplings the warp-per-sample kernel keeps in shared
+// memory (n x 256 floats at n > 128).
+constexpr int kTurnMaxN = 220;
+
 template <int NC>
 static cudaError_t launch_turn_t(const AisArgs& a, int64_t max_samples,
                                  cudaStream_t st) {
@@ -560,8 +564,10 @@ static cudaError_t launch_turn_t(const AisArgs& a, int64_t max_samples,
   const size_t smem = (size_t)a.max_n * 32 * NC * 4;
   const void* f = random ? (const void*)k_ais_turn<NC, true>
                          : (const void*)k_ais_turn<NC, false>;
-  cudaError_t e = cudaFuncSetAttribute(
-      f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr int widest = 32 * NC < kTurnMaxN ? 32 * NC : kTurnMaxN;
+  static std::atomic<uint64_t> allowed[2];
+  cudaError_t e =
+      allow_smem(f, (size_t)widest * 32 * NC * 4, allowed[random]);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((max_samples + wpc - 1) / wpc),
             (unsigned)a.num_instances);
@@ -592,9 +598,6 @@ static cudaError_t launch_small_t(const AisArgs& a, int64_t max_samples,
 // 17.5 against 24.4.
 constexpr int64_t kTurnSamples = 4096;  // n <= 32
 constexpr int64_t kTurnSamplesWide = 24576;
-// Widest instance whose couplings the warp-per-sample kernel keeps in shared
-// memory (n x 256 floats at n > 128).
-constexpr int kTurnMaxN = 220;
 
 cudaError_t launch_ais(const AisArgs& a, int64_t max_samples, cudaStream_t st) {
   const int64_t total = max_samples * a.num_instances;

@@ -8,6 +8,7 @@
 // * mbarrier and bulk-copy (TMA engine, 1-D) wrappers.  Every wait is bounded:
 //   on timeout the kernel records an error code in the status word and returns.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -49,6 +50,23 @@ __device__ __forceinline__ void draw4(uint64_t seed, uint32_t tag,
                                       uint32_t q, uint32_t out[4]) {
   philox4x32_10(q, a, b, (inst << 4) | tag, (uint32_t)seed,
                 (uint32_t)(seed >> 32), out);
+}
+
+// Lets launches of kernel `f` ask for up to `bytes` of dynamic shared memory,
+// the most that any of them needs; once per device (`done`, a bit each).  The
+// limit belongs to the kernel and not to a launch: set to every launch's own
+// size, a smaller launch on another host thread could lower it in between.
+inline cudaError_t allow_smem(const void* f, size_t bytes,
+                              std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 // The ten round keys of a seed, k0 and k1 in turn.  As kernel parameters they

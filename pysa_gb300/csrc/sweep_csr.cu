@@ -60,6 +60,9 @@ constexpr int kSchedThreads = 512;
 // Widest instance whose quads may be cut (shared memory, 16 bits per unit).
 constexpr int kSchedCutN = 8192;
 
+// Dynamic shared memory a CTA of these kernels may take (a little is static).
+constexpr size_t kCsrSmem = 232448 - 256;
+
 __host__ __device__ constexpr int csr_quads(int n) { return (n + 3) >> 2; }
 
 // Schedule entries (units, and first places of the levels) the sweep holds:
@@ -684,11 +687,11 @@ static cudaError_t launch_csr_t(const CsrArgs& a, cudaStream_t st) {
            (size_t)w * (2 * QuadSlab<D>::QUAD * 4 + 256) +
            2 * (size_t)sched_cap(n) + (RANDOM ? 2 * (size_t)n : 0);
   };
-  while (W > 2 && bytes(W) > 232448 - 256) W /= 2;
+  while (W > 2 && bytes(W) > kCsrSmem) W /= 2;
   const size_t smem = bytes(W);
-  cudaError_t e = cudaFuncSetAttribute(
-      k_sweep_csr<RANDOM, ISING, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)smem);
+  static std::atomic<uint64_t> allowed;
+  cudaError_t e = allow_smem((const void*)k_sweep_csr<RANDOM, ISING, D>,
+                             kCsrSmem, allowed);
   if (e != cudaSuccess) return e;
   k_sweep_csr<RANDOM, ISING, D><<<a.num_items, 32 * W, smem, st>>>(a);
   return cudaGetLastError();
@@ -715,8 +718,8 @@ cudaError_t launch_csr_schedule(const CsrArgs& a, bool random,
   const size_t smem = (whole > parts ? whole : parts) + 16;
   const void* f = random ? (const void*)k_csr_schedule<true>
                          : (const void*)k_csr_schedule<false>;
-  cudaError_t e = cudaFuncSetAttribute(
-      f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> allowed[2];
+  cudaError_t e = allow_smem(f, kCsrSmem, allowed[random]);
   if (e != cudaSuccess) return e;
   if (random)
     k_csr_schedule<true><<<a.p.num_instances, kSchedThreads, smem, st>>>(a);

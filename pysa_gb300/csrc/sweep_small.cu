@@ -563,8 +563,9 @@ cudaError_t launch_small(SmallArgs a, bool random, cudaStream_t st) {
   const size_t smem = SmallSmem::bytes(a.cap);
   const void* f = random ? (const void*)k_sweep_small<true>
                          : (const void*)k_sweep_small<false>;
-  cudaError_t e = cudaFuncSetAttribute(
-      f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> allowed[2];
+  cudaError_t e =
+      allow_smem(f, SmallSmem::bytes(kMaxReplicas), allowed[random]);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.p.num_reads * cs));

@@ -125,11 +125,10 @@ cudaError_t launch_wide(const WideArgs& a, bool random, int max_ctas,
   const size_t sm = wide_smem_bytes(a.p.words);
   const void* f = random ? (const void*)k_sweep_wide<true>
                          : (const void*)k_sweep_wide<false>;
-  if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(
-        f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<uint64_t> allowed[2];
+  cudaError_t e =
+      allow_smem(f, wide_smem_bytes(PYSA_GB_MAX_N / 32), allowed[random]);
+  if (e != cudaSuccess) return e;
   const int grid = a.num_items < max_ctas ? a.num_items : max_ctas;
   if (random)
     k_sweep_wide<true><<<grid, 32 * kWideWarps, sm, st>>>(a);
