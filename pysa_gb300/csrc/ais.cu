@@ -228,18 +228,6 @@ struct AisThreshold {
   }
 };
 
-// Exact pair (hi, lo) + x (Knuth's two-sum).
-__device__ __forceinline__ void energy_add(float2& p, float x) {
-  const float s = p.x + x;
-  const float bb = s - p.x;
-  p.y += (p.x - (s - bb)) + (x - bb);
-  p.x = s;
-}
-// The pair rounded to f32 (infinite or NaN sums have no second part).
-__device__ __forceinline__ float energy_of(const float2& p) {
-  return fabsf(p.x) < INFINITY ? p.x + p.y : p.x;
-}
-
 // A warp per sample, the visiting positions in turn (n <= 32 NC).  Lane l
 // holds the fields of columns l, l + 32, ... in registers and, as bits m of
 // one word, the spins 32 m + l; the instance's couplings are in shared
@@ -248,8 +236,10 @@ __device__ __forceinline__ float energy_of(const float2& p) {
 // acceptance.  A decision inside the band has its sweep done again with the
 // exact rule.  For few samples: the kernels that hold several samples per
 // warp or thread need fewer instructions each, but too few warps then leave
-// every SM waiting.  Measured for n = 96, 1000 samples, 200 steps: 12.7 ms
-// with 8 samples per warp, 1.64 ms here.
+// every SM waiting.  A lane keeps the energy change of the position it is
+// numbered after; they are added in f64 after every 32 positions.  Measured for
+// n = 96, 1000 samples, 200 steps: 12.7 ms with 8 samples per warp, 1.57 ms
+// here (random order 1.84).
 template <int NC, bool RANDOM>
 __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
   extern __shared__ __align__(16) float Jt[];  // [n][32 NC]
@@ -285,7 +275,7 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
     if (m < words)
       sp |= ((a.spins[myc * a.words + m] >> lane) & 1u) << m;
   }
-  float2 E = make_float2(a.energies[myc], 0.0f);
+  double E = (double)a.energies[myc];
   double lw = 0.0;
   float beta_old = 0.0f;
   const double lr = uniform_ref ? 0.0 : log((1.0 - a.p) / a.p);
@@ -298,11 +288,12 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
   for (int k = 0; k < a.num_temps; ++k) {
     const float beta = a.temps[k];
     if (a.order == 1)
-      lw += ais_dlw(beta, beta_old, energy_of(E), n, ones(), logp, log1p_,
+      lw += ais_dlw(beta, beta_old, (float)E, n, ones(), logp, log1p_,
                     uniform_ref);
     const int32_t* perm =
         a.perm + ((int64_t)k * a.num_instances + inst) * a.max_n;
     const AisThreshold at(beta, scale, lr, uniform_ref);
+    double dE = 0.0;  // the sweep's energy change
     // one sweep; EXACT asks ais_accept where the thresholds have no answer,
     // otherwise returns whether some decision needed it
     auto sweep = [&](auto exact_t) {
@@ -312,7 +303,7 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
         const int t0 = 32 * b;
         int il = t0 + lane;
         if (RANDOM) il = il < n ? perm[il] : 0;
-        float tl, th;
+        float tl, th, gain = 0.0f;  // of position t0 + lane
         {
           uint32_t x[4], v[4];
           draw4(a.seed, TAG_AIS, (uint32_t)inst, (uint32_t)k, (uint32_t)my,
@@ -354,16 +345,17 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
 #pragma unroll
           for (int m = 0; m < NC; ++m) h[m] = acc ? v[m] : h[m];
           sp ^= acc && lane == l ? 1u << mi : 0u;
-          energy_add(E, acc ? -(scale * y) : 0.0f);
+          gain = acc && lane == p ? scale * y : gain;
         };
         const int te = t0 + 32 < n ? t0 + 32 : n;
         if constexpr (EXACT) {
 #pragma unroll 1
           for (int t = t0; t < te; ++t) turn(t);
         } else {
-#pragma unroll 4
+#pragma unroll(NC < 8 ? 4 : 2)
           for (int t = t0; t < te; ++t) turn(t);
         }
+        dE -= warp_sum((double)gain);
       }
       return unsure != 0u;
     };
@@ -371,22 +363,22 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
 #pragma unroll
     for (int m = 0; m < NC; ++m) h0[m] = h[m];
     const uint32_t sp0 = sp;
-    const float2 E0 = E;
     if (sweep(std::false_type{})) {
 #pragma unroll
       for (int m = 0; m < NC; ++m) h[m] = h0[m];
       sp = sp0;
-      E = E0;
+      dE = 0.0;
       sweep(std::true_type{});
     }
+    E += dE;
     if (a.order == 0)
-      lw += ais_dlw(beta, beta_old, energy_of(E), n, ones(), logp, log1p_,
+      lw += ais_dlw(beta, beta_old, (float)E, n, ones(), logp, log1p_,
                     uniform_ref);
     beta_old = beta;
   }
   if (lane == 0) {
     a.log_w[myc] = lw;
-    a.energies[myc] = energy_of(E);
+    a.energies[myc] = (float)E;
   }
 #pragma unroll
   for (int m = 0; m < NC; ++m) {
@@ -394,6 +386,27 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
     if (m < words && lane == 0) a.spins[myc * a.words + m] = w;
   }
 }
+
+// One sweep's energy change as three f32 (two exact two-sums, Knuth's): to
+// 2^-72 of its largest term, more than the f64 sum it stands in for, without
+// f64 instructions (1/64 of the rate) for each attempt.  Every sweep's change
+// starts at zero and joins the sample's energy, which is f64, at its end.
+struct SweepEnergy {
+  float a = 0.0f, b = 0.0f, c = 0.0f;
+  __device__ __forceinline__ void add(float x) {
+    const float s = a + x, u = s - a;
+    const float e = (a - (s - u)) + (x - u);
+    const float t = b + e, v = t - b;
+    c += (b - (t - v)) + (e - v);
+    a = s;
+    b = t;
+  }
+  // (an infinite or NaN sum has no further parts)
+  __device__ __forceinline__ double value() const {
+    return fabsf(a) < INFINITY ? (double)a + ((double)b + (double)c)
+                               : (double)a;
+  }
+};
 
 // Two pairs from shared memory.  Volatile: the couplings never change, and
 // unrolled code would otherwise try to keep all of them in registers.
@@ -413,8 +426,8 @@ __device__ __forceinline__ ulonglong2 load_pairs(uint32_t addr) {
 // no field but possibly the sign of a zero.  Bound by instruction issue: the
 // Philox draw (one per four positions) and the field updates take most of
 // it.  Measured for 64 instances of n = 24, 1024 samples, 200 steps: 4.33 ms
-// with the fields in shared memory and f64 energies, 1.18 ms here (random
-// order 4.42 and 1.75).
+// with the fields in shared memory and an f64 addition an attempt, 1.27 ms
+// here (random order 4.42 and 1.77).
 template <int NP, bool RANDOM>
 __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
   __shared__ __align__(16) float Js[NP * NP];
@@ -450,7 +463,7 @@ __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
   const float scale = ising ? 2.0f : 1.0f;
   const bool uniform_ref = a.ref != 1;
   uint32_t word = a.spins[myc * a.words];
-  float2 E = make_float2(a.energies[myc], 0.0f);
+  double E = (double)a.energies[myc];
   double lw = 0.0;
   float beta_old = 0.0f;
   const double lr = uniform_ref ? 0.0 : log((1.0 - a.p) / a.p);
@@ -459,11 +472,12 @@ __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
   for (int k = 0; k < a.num_temps; ++k) {
     const float beta = a.temps[k];
     if (a.order == 1)
-      lw += ais_dlw(beta, beta_old, energy_of(E), n, __popc(word), logp,
+      lw += ais_dlw(beta, beta_old, (float)E, n, __popc(word), logp,
                     log1p_, uniform_ref);
     const int32_t* perm =
         a.perm + ((int64_t)k * a.num_instances + inst) * a.max_n;
     const AisThreshold at(beta, scale, lr, uniform_ref);
+    SweepEnergy dE;
     uint32_t rnd[4];
     auto turn = [&](int t, int i, float hv, uint32_t x) {
       const bool sb = (word >> i) & 1u;
@@ -475,7 +489,7 @@ __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
       if (!acc && !(y < tl + off))
         acc = ais_accept(beta, scale * y, sb, lr, uniform_ref, x);
       word ^= acc ? 1u << i : 0u;
-      energy_add(E, acc ? -(scale * y) : 0.0f);
+      dE.add(acc ? -(scale * y) : 0.0f);
       const float d = acc ? (sb ? -scale : scale) : 0.0f;
       const uint64_t dd = pack2(d, d);
       const uint32_t row = js_addr + (uint32_t)(i * NP * 4);
@@ -530,13 +544,14 @@ __global__ void __launch_bounds__(128) k_ais_small(const AisArgs a) {
         turn(t, t, half2(H[t >> 1], t & 1), rnd[t & 3]);
       }
     }
+    E += dE.value();
     if (a.order == 0)
-      lw += ais_dlw(beta, beta_old, energy_of(E), n, __popc(word), logp,
+      lw += ais_dlw(beta, beta_old, (float)E, n, __popc(word), logp,
                     log1p_, uniform_ref);
     beta_old = beta;
   }
   a.log_w[myc] = lw;
-  a.energies[myc] = energy_of(E);
+  a.energies[myc] = (float)E;
   a.spins[myc * a.words] = word;
 }
 
