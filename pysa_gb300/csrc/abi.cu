@@ -98,6 +98,34 @@ static int tc_round_limit(int fold, bool relay) {
 // millisecond each thousand).
 constexpr int kMaxSmallSweeps = 4096;
 
+// Whether a batch of small instances alone sweeps resident on the SMs (a CTA a
+// read) or in three launches a sweep: the shorter of two estimates, in ns.
+// Resident: moving a read's state in and out, which short calls of many reads
+// don't earn back, and a second launch where replica counts may differ; then a
+// time per chain and sweep, more when a read has few chains (its other warps
+// wait) or fills an SM alone.  Launches: a start-up that grows with n attempts
+// and R - 1 exchanges one after another, then a time per chain.  Measured, us a
+// sweep, resident against launches: n = 24, 20000 reads of 1, calls of 40 sweeps
+// 32 and 39, of one sweep 161 and 48; 200000 reads of 1 305 and 243; 8000 of 16
+// 109 and 148, one sweep 163 and 157; n = 8, 50000 of 2 90 and 76, 5000 of 32 90
+// and 88; n = 40, 8000 of 16 174 and 291, one sweep 259 and 300.
+static bool small_resident(const pysa_gb_problems* p, int sweeps,
+                           bool random) {
+  const double chains = (double)p->num_chains, reads = (double)p->num_reads;
+  const double n = p->max_n < kSmallMaxN ? p->max_n : kSmallMaxN;
+  const double R = reads > 0.0 ? chains / reads : 1.0;
+  const bool narrow = n <= 32.0;
+  const double io = (p->num_instances > 1 ? 2e4 : 0.0) +
+                    5e3 + 3.0 * n * n +
+                    reads * ((narrow ? 3.5 : 8.0) +
+                             R * ((narrow ? 0.35 : 0.5) + 0.0013 * R));
+  const double chain = ((0.36 + 0.025 * n) * (1.0 + R / 512.0) + 0.6 / R) *
+                       (random ? 1.1 : 1.0);
+  const double start = 1e4 + 700.0 * n + 130.0 * R;
+  const double step = narrow ? 0.27 + 0.026 * n + 0.2 / R : 0.9 + 0.03 * n;
+  return io + sweeps * chains * chain < sweeps * (start + chains * step);
+}
+
 // Streaming multiprocessors of the current device (cached per device).
 static inline bool is_sparse(const pysa_gb_host_tables* h, int i) {
   return h && h->sparse && h->sparse[i];
@@ -818,10 +846,11 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
   // CTA (or nothing to do between sweeps), or small enough to stay on an SM;
   // exchange and log-omega inside the kernels, several sweeps per launch.
   const bool between = o->use_pt || o->log_omega_stride > 0;
-  const bool fused = phases == 3 && !wider_live && ws->csr_item_count == 0 &&
-                     ws->wide_item_count == 0 && (last_v >= 0 || small_live) &&
-                     (last_v < 0 ||
-                      ((!between || ws->tc_fusable) && ws->tc_sched));
+  const bool fused =
+      phases == 3 && !wider_live && ws->csr_item_count == 0 &&
+      ws->wide_item_count == 0 &&
+      (last_v >= 0 ? (!between || ws->tc_fusable) && ws->tc_sched
+                   : small_live && small_resident(p, num_sweeps, random));
   // random order on the tensor cores: visiting orders of the next `cnt`
   // sweeps, and the tiles repacked in those orders
   auto rand_prepare = [&](int cnt) -> int {
@@ -869,16 +898,15 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
         sa.s = *s;
         sa.fields = ws->fields;
         sa.field_ld = ws->field_ld;
-        sa.cap = 0;
         sa.seed = o->seed;
         sa.num_sweeps = chunk;
         sa.use_pt = o->use_pt;
         sa.exchange_every = o->exchange_every;
         sa.log_omega_stride = o->log_omega_stride;
         sa.advance = 1;
-        sa.pad_ = 0;
+        sa.above = sa.cap = sa.warps = 0;
         sa.skip_inst = a.skip_inst;
-        cudaError_t e = launch_small(sa, random, st);
+        cudaError_t e = launch_small(sa, random, sm_count(), st);
         if (e != cudaSuccess) return cuda_fail(e, "small sweep launch");
       }
       remaining -= chunk;

@@ -19,14 +19,17 @@
 // positions in turn.  Field updates, energy sums and draws are those of the
 // plain sweep kernel, bit for bit.
 //
-// One more warp works ahead: the next sweep's visiting order and this
-// sweep's exchange draws.  While the reads are fewer than the SMs, a cluster
+// One more warp works ahead where there is something to: the next sweep's
+// visiting order and this sweep's exchange draws.  While the reads are fewer than the SMs, a cluster
 // of up to 8 CTAs shares a read's chains; energies and new betas cross
 // through distributed shared memory.
 //
 // Measured (times per sweep with exchange): n = 60, 640 chains in 20 reads,
 // log-omega 62 -> 8 us (22 on one CTA per read in rounds alone); n = 24, 4
-// chains, random order 25 -> 2.5 us (three launches per sweep before).
+// chains, random order 25 -> 2.5 us (three launches per sweep before).  Many
+// reads: rows of 32 columns up to n = 32 and CTAs of as many warps as let an SM
+// hold several, n = 24, 8000 reads of 16 chains 245 -> 109 us, n = 40 313 -> 174
+// (launches: 148 and 291).
 #include <cooperative_groups.h>
 
 #include "aux.cuh"
@@ -41,16 +44,17 @@ constexpr int kMaxSmallWarps = 31;  // chains at a time; one more works ahead
 // one spin in kDenseFlips (a round of the other form costs about as much as
 // five positions), in rounds otherwise.
 constexpr int kDenseFlips = 5;
-constexpr int64_t kSmallFill = 160;  // CTAs that give about every SM one
 
-// Shared memory of a CTA, in 4-byte words: fixed part, then per replica.
+// Shared memory of a CTA, in 4-byte words: fixed part, then per replica.  N:
+// columns kept per row, 32 or 64.
+template <int N>
 struct SmallSmem {
-  static constexpr int J = 0;                  // [64][64] couplings
-  static constexpr int PERM = J + 64 * 64;     // [2][64] visiting orders
+  static constexpr int J = 0;                  // [N][N] couplings
+  static constexpr int PERM = J + N * N;       // [2][64] visiting orders
   static constexpr int INV = PERM + 2 * 64;    // [2][64] positions of spins
   static constexpr int WORK = INV + 2 * 64;    // [2][64] helper scratch
   static constexpr int FIXED = WORK + 2 * 64;
-  static constexpr int PER = 64 + 2 + 15;      // words per replica
+  static constexpr int PER = N + 2 + 15;       // words per replica
   static size_t bytes(int cap) {  // and a byte per replica of any read
     return 4 * ((size_t)FIXED + (size_t)PER * cap) + kMaxReplicas;
   }
@@ -105,9 +109,11 @@ __device__ void small_order(uint64_t seed, uint32_t inst, uint32_t sweep,
 
 }  // namespace
 
-template <bool RANDOM>
+template <bool RANDOM, int N>
 __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
     k_sweep_small(const SmallArgs a) {
+  using Smem = SmallSmem<N>;
+  constexpr bool kTwo = N > 32;  // a second position per lane
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) uint32_t sm[];
   cg::cluster_group cl = cg::this_cluster();
@@ -115,21 +121,32 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
   auto sync_read = [&]() {  // every CTA of the read
     if (csize > 1) cl.sync(); else __syncthreads();
   };
-  const int64_t r = blockIdx.x / csize;
-  const int inst = a.p.read_inst[r];
-  const int n = a.p.n[inst];
-  const bool mine = n <= kSmallMaxN &&
-                    !(a.p.csr_row_off && a.p.csr_row_off[inst] >= 0) &&
-                    !(a.skip_inst && a.skip_inst[inst]);  // uniform per CTA
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sweep0 = (uint32_t)(*a.s.sweep_counter);
-  if (mine) {
-    const int NW = (int)(blockDim.x >> 5) - 1;  // warps with chains
+  // instances of this launch (uniform per CTA)
+  auto wanted = [&](int i) {
+    return a.p.n[i] <= kSmallMaxN && a.p.replicas[i] > a.above &&
+           a.p.replicas[i] <= a.cap &&
+           !(a.p.csr_row_off && a.p.csr_row_off[i] >= 0) &&
+           !(a.skip_inst && a.skip_inst[i]);
+  };
+  bool some = a.above == 0;
+  if (a.above > 0) {  // nearly always there is none
+    bool own = false;
+    for (int i = tid; i < a.p.num_instances; i += blockDim.x)
+      own = own || wanted(i);
+    some = __syncthreads_or(own);
+  }
+  for (int64_t r = blockIdx.x / csize; some && r < a.p.num_reads;
+       r += gridDim.x / csize) {
+    const int inst = a.p.read_inst[r];
+    if (!wanted(inst)) continue;
+    const int n = a.p.n[inst];
+    const int NW = a.warps;  // warps with chains
     const int R = a.p.replicas[inst];
-    const bool fit = R <= a.cap;  // else the state stays in global memory
-    // this CTA's chains c0 ... c1 - 1 (all of them in rank 0 if they don't
-    // fit); the energies of all, the slot map and the exchange are rank 0's
-    const int Rc = fit ? (R + csize - 1) / csize : R;
+    // this CTA's chains c0 ... c1 - 1; the energies of all, the slot map and
+    // the exchange are rank 0's
+    const int Rc = (R + csize - 1) / csize;
     const int c0 = rank * Rc < R ? rank * Rc : R;
     const int c1 = c0 + Rc < R ? c0 + Rc : R;
     const int64_t lread = r - a.p.read_off[inst];
@@ -139,61 +156,49 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
     const float scale = ising ? 2.0f : 1.0f;
     const float* betas = a.p.ladder + a.p.ladder_off[inst];
     const int32_t* sorted = a.p.ladder_sorted + a.p.ladder_off[inst];
-    float* J = reinterpret_cast<float*>(sm + SmallSmem::J);
-    int32_t* perm_s = reinterpret_cast<int32_t*>(sm + SmallSmem::PERM);
-    int32_t* inv_s = reinterpret_cast<int32_t*>(sm + SmallSmem::INV);
-    int32_t* work_s = reinterpret_cast<int32_t*>(sm + SmallSmem::WORK);
-    uint32_t* per = sm + SmallSmem::FIXED;
+    float* J = reinterpret_cast<float*>(sm + Smem::J);
+    int32_t* perm_s = reinterpret_cast<int32_t*>(sm + Smem::PERM);
+    int32_t* inv_s = reinterpret_cast<int32_t*>(sm + Smem::INV);
+    int32_t* work_s = reinterpret_cast<int32_t*>(sm + Smem::WORK);
+    uint32_t* per = sm + Smem::FIXED;
     const int cap = a.cap;
-    // per replica; the first six are copies of global state when they fit
-    float* Hs = reinterpret_cast<float*>(per);             // [cap][64]
-    uint32_t* Ss = per + 64 * cap;                         // [cap][2]
-    float* E = fit ? reinterpret_cast<float*>(per + 66 * cap)
-                   : a.s.energies + base;
-    int32_t* B = fit ? reinterpret_cast<int32_t*>(per + 67 * cap)
-                     : a.s.beta_idx + base;
-    float* beta_c = fit ? reinterpret_cast<float*>(per + 68 * cap)
-                        : a.s.chain_beta + base;
-    float* bestE = fit ? reinterpret_cast<float*>(per + 69 * cap)
-                       : a.s.best_energy + base;
-    const float* Bt = fit ? reinterpret_cast<float*>(per + 70 * cap) : betas;
-    float2* dE = reinterpret_cast<float2*>(per + 72 * cap);  // [cap]
-    float2* X2 = reinterpret_cast<float2*>(per + 74 * cap);  // draw, log
-    float2* E2 = reinterpret_cast<float2*>(per + 76 * cap);  // energy, dbeta
-    int32_t* B2 = reinterpret_cast<int32_t*>(per + 78 * cap);
-    uint32_t* LT = per + 79 * cap;                           // reject below
-    uint8_t* dense = reinterpret_cast<uint8_t*>(per + 80 * cap);  // [R]
-    auto Hc = [&](int c) {
-      return fit ? Hs + 64 * c : a.fields + (base + c) * (int64_t)a.field_ld;
-    };
-    auto Sc = [&](int c) {
-      return fit ? Ss + 2 * c : a.s.spins + (base + c) * (int64_t)a.p.words;
-    };
+    // per replica; the first six are copies of global state
+    float* Hs = reinterpret_cast<float*>(per);             // [cap][N]
+    uint32_t* Ss = per + N * cap;                          // [cap][2]
+    float* E = reinterpret_cast<float*>(per + (N + 2) * cap);
+    int32_t* B = reinterpret_cast<int32_t*>(per + (N + 3) * cap);
+    float* beta_c = reinterpret_cast<float*>(per + (N + 4) * cap);
+    float* bestE = reinterpret_cast<float*>(per + (N + 5) * cap);
+    float* Bt = reinterpret_cast<float*>(per + (N + 6) * cap);
+    float2* dE = reinterpret_cast<float2*>(per + (N + 8) * cap);  // [cap]
+    float2* X2 = reinterpret_cast<float2*>(per + (N + 10) * cap);  // draw, log
+    float2* E2 =  // energy, dbeta
+        reinterpret_cast<float2*>(per + (N + 12) * cap);
+    int32_t* B2 = reinterpret_cast<int32_t*>(per + (N + 14) * cap);
+    uint32_t* LT = per + (N + 15) * cap;                     // reject below
+    uint8_t* dense = reinterpret_cast<uint8_t*>(per + (N + 16) * cap);  // [R]
 
     // ---- state in
     {
       const float* Jg = a.p.J + a.p.j_off[inst];
       const int ld = a.p.ld[inst];
-      for (int e = tid; e < n * 64; e += blockDim.x) {
-        const int i = e >> 6, c = e & 63;
+      for (int e = tid; e < n * N; e += blockDim.x) {
+        const int i = e / N, c = e % N;
         J[e] = c < n ? Jg[(int64_t)i * ld + c] : 0.0f;
       }
-      if (fit) {
-        for (int e = 64 * c0 + tid; e < 64 * c1; e += blockDim.x) {
-          const int c = e >> 6, i = e & 63;
-          Hs[e] = i < n ? a.fields[(base + c) * (int64_t)a.field_ld + i]
-                        : 0.0f;
-        }
-        for (int c = tid; c < R; c += blockDim.x) {
-          const int64_t g = base + c;
-          Ss[2 * c] = a.s.spins[g * a.p.words];
-          Ss[2 * c + 1] = words > 1 ? a.s.spins[g * a.p.words + 1] : 0u;
-          E[c] = a.s.energies[g];
-          B[c] = a.s.beta_idx[g];
-          beta_c[c] = a.s.chain_beta[g];
-          bestE[c] = a.s.best_energy[g];
-          const_cast<float*>(Bt)[c] = betas[c];
-        }
+      for (int e = N * c0 + tid; e < N * c1; e += blockDim.x) {
+        const int c = e / N, i = e % N;
+        Hs[e] = i < n ? a.fields[(base + c) * (int64_t)a.field_ld + i] : 0.0f;
+      }
+      for (int c = tid; c < R; c += blockDim.x) {
+        const int64_t g = base + c;
+        Ss[2 * c] = a.s.spins[g * a.p.words];
+        Ss[2 * c + 1] = words > 1 ? a.s.spins[g * a.p.words + 1] : 0u;
+        E[c] = a.s.energies[g];
+        B[c] = a.s.beta_idx[g];
+        beta_c[c] = a.s.chain_beta[g];
+        bestE[c] = a.s.best_energy[g];
+        Bt[c] = betas[c];
       }
       for (int c = tid; c < R; c += blockDim.x) dense[c] = 1;
       if (RANDOM && warp == NW)
@@ -210,14 +215,14 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
         // ------------------------------------------------------- sweeps
         const int32_t* perm = perm_s + 64 * (sweep & 1);
         const int32_t* inv = inv_s + 64 * (sweep & 1);
-        const bool two = n > 32;
+        const bool two = kTwo && n > 32;
         const int k1 = lane + 32;
-        const bool in0 = lane < n, in1 = k1 < n;
+        const bool in0 = lane < n, in1 = kTwo && k1 < n;
         const int i0 = in0 ? (RANDOM ? perm[lane] : lane) : 0;
         const int i1 = in1 ? (RANDOM ? perm[k1] : k1) : 0;
         for (int c = c0 + warp; c < c1; c += NW) {
-          float* H = Hc(c);
-          uint32_t* S = Sc(c);
+          float* H = Hs + N * c;
+          uint32_t* S = Ss + 2 * c;
           float h0 = in0 ? H[i0] : 0.0f, h1 = in1 ? H[i1] : 0.0f;
           const uint32_t wa = S[0], wb = words > 1 ? S[1] : 0u;
           // the spins by position, as masks (bit l: position l, l + 32)
@@ -275,8 +280,8 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
             uint32_t unsure = 0u, f0 = 0u, f1 = 0u;
             auto turn = [&](int t, bool hf) {
               const int js = t & 31;
-              const float* row = J + 64 * (RANDOM ? perm[t] : t);
-              const float r0 = row[i0], r1 = row[i1];
+              const float* row = J + N * (RANDOM ? perm[t] : t);
+              const float r0 = row[i0], r1 = kTwo ? row[i1] : 0.0f;
               const float th = __shfl_sync(0xffffffffu, hf ? th1 : th0, js);
               const float tl = __shfl_sync(0xffffffffu, hf ? tl1 : tl0, js);
               const bool sb = (((hf ? S1 : S0) >> js) & 1u) != 0u;
@@ -344,7 +349,7 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
             if (acc) {
               const bool sb = ((hf ? S1 : S0) & bit) != 0u;
               const float d = sb ? -scale : scale;
-              const float* row = J + 64 * i;
+              const float* row = J + N * i;
               if (in0) h0 = fmaf(d, row[i0], h0);
               if (in1) h1 = fmaf(d, row[i1], h1);
               const float dn = scale * y;
@@ -374,17 +379,12 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
             dense[c] = kDenseFlips * (__popc(S0 ^ B0) + __popc(S1 ^ B1)) > n;
             S[0] = na;
             if (words > 1) S[1] = nb;
-            if (fit) {
-              dE[c] = make_float2(d0, d1);
-            } else {
-              // no room for the pair: the energy now
-              E[c] = (float)((double)E[c] + ((double)d0 + (double)d1));
-            }
+            dE[c] = make_float2(d0, d1);
           }
         }
       } else {
         // ---------------------------------------------------- work ahead
-        if (fit && xch && rank == 0)
+        if (xch && rank == 0)
           for (int k = lane; k < R - 1; k += 32) {
             const uint32_t x = draw1(a.seed, TAG_PT, (uint32_t)inst, sweep,
                                      (uint32_t)lread, (uint32_t)k);
@@ -406,19 +406,17 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
       // ------------------------- energies, best states, exchange: warp 0
       if (warp == 0) {
         for (int c = c0 + lane; c < c1; c += 32) {
-          float e = E[c];
-          if (fit) {
-            const float2 d = dE[c];
-            e = (float)((double)e + ((double)d.x + (double)d.y));
-            E[c] = e;
-            if (rank != 0) cl.map_shared_rank(E, 0)[c] = e;
-          }
+          const float2 d = dE[c];
+          const float e =
+              (float)((double)E[c] + ((double)d.x + (double)d.y));
+          E[c] = e;
+          if (rank != 0) cl.map_shared_rank(E, 0)[c] = e;
           // strict < (pysa/simulation.py:150-171)
           if (e < bestE[c]) {
             bestE[c] = e;
             const int64_t g = base + c;
             a.s.best_sweep[g] = (int32_t)sweep;
-            const uint32_t* S = Sc(c);
+            const uint32_t* S = Ss + 2 * c;
             for (int w = 0; w < words; ++w)
               a.s.best_spins[g * a.p.words + w] = S[w];
           }
@@ -432,46 +430,37 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
           // entering slot k1 carries from pair to pair, so every pair's
           // other replica, its energy and the betas' difference are read up
           // front and the pass keeps the carried one in registers
-          if (fit) {
-            for (int k = lane; k < R - 1; k += 32) {
-              const int t1 = R - k - 1, t2 = R - k - 2;
-              const int b2 = B[t2];
-              B2[k] = b2;
-              E2[k] = make_float2(E[b2], __fsub_rn(Bt[t1], Bt[t2]));
-            }
-            __syncwarp();
+          for (int k = lane; k < R - 1; k += 32) {
+            const int t1 = R - k - 1, t2 = R - k - 2;
+            const int b2 = B[t2];
+            B2[k] = b2;
+            E2[k] = make_float2(E[b2], __fsub_rn(Bt[t1], Bt[t2]));
           }
+          __syncwarp();
           if (lane == 0) {
-            int cb = B[R - 1];
-            float ce = E[cb];
-            bool redo = !fit;
-            if (fit) {
-              // without the exact rule; a pair that needs it has the pass
-              // made again below
-              const int cb0 = cb;
-              const float ce0 = ce;
-              uint32_t unsure = 0u;
+            // without the exact rule; a pair that needs it has the pass made
+            // again below
+            const int cb0 = B[R - 1];
+            const float ce0 = E[cb0];
+            int cb = cb0;
+            float ce = ce0;
+            uint32_t unsure = 0u;
 #pragma unroll 4
-              for (int k = 0; k < R - 1; ++k) {
-                const int b2 = B2[k];
-                const float2 e2 = E2[k], x2 = X2[k];
-                const float de = __fmul_rn(__fsub_rn(ce, e2.x), e2.y);
-                const bool sw = de >= x2.y;
-                unsure |=
-                    (!sw && !(de < __uint_as_float(LT[k]))) ? 1u : 0u;
-                B[R - k - 1] = sw ? b2 : cb;  // final: no later pair
-                cb = sw ? cb : b2;
-                ce = sw ? ce : e2.x;
-              }
-              if (unsure) {
-                for (int k = 0; k < R - 1; ++k) B[R - k - 2] = B2[k];
-                B[R - 1] = cb0;
-                cb = cb0;
-                ce = ce0;
-                redo = true;
-              }
+            for (int k = 0; k < R - 1; ++k) {
+              const int b2 = B2[k];
+              const float2 e2 = E2[k], x2 = X2[k];
+              const float de = __fmul_rn(__fsub_rn(ce, e2.x), e2.y);
+              const bool sw = de >= x2.y;
+              unsure |= (!sw && !(de < __uint_as_float(LT[k]))) ? 1u : 0u;
+              B[R - k - 1] = sw ? b2 : cb;  // final: no later pair
+              cb = sw ? cb : b2;
+              ce = sw ? ce : e2.x;
             }
-            if (redo) {
+            if (unsure) {
+              for (int k = 0; k < R - 1; ++k) B[R - k - 2] = B2[k];
+              B[R - 1] = cb0;
+              cb = cb0;
+              ce = ce0;
               for (int k = 0; k < R - 1; ++k) {
                 const int t1 = R - k - 1, t2 = R - k - 2, b2 = B[t2];
                 const float e2 = E[b2];
@@ -515,22 +504,21 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
     }
 
     // ---- state out
-    if (fit) {
-      for (int e = 64 * c0 + tid; e < 64 * c1; e += blockDim.x) {
-        const int c = e >> 6, i = e & 63;
-        if (i < n) a.fields[(base + c) * (int64_t)a.field_ld + i] = Hs[e];
-      }
-      for (int c = c0 + tid; c < c1; c += blockDim.x) {
-        const int64_t g = base + c;
-        a.s.spins[g * a.p.words] = Ss[2 * c];
-        if (words > 1) a.s.spins[g * a.p.words + 1] = Ss[2 * c + 1];
-        a.s.energies[g] = E[c];
-        a.s.chain_beta[g] = beta_c[c];
-        a.s.best_energy[g] = bestE[c];
-      }
-      if (rank == 0)
-        for (int c = tid; c < R; c += blockDim.x) a.s.beta_idx[base + c] = B[c];
+    for (int e = N * c0 + tid; e < N * c1; e += blockDim.x) {
+      const int c = e / N, i = e % N;
+      if (i < n) a.fields[(base + c) * (int64_t)a.field_ld + i] = Hs[e];
     }
+    for (int c = c0 + tid; c < c1; c += blockDim.x) {
+      const int64_t g = base + c;
+      a.s.spins[g * a.p.words] = Ss[2 * c];
+      if (words > 1) a.s.spins[g * a.p.words + 1] = Ss[2 * c + 1];
+      a.s.energies[g] = E[c];
+      a.s.chain_beta[g] = beta_c[c];
+      a.s.best_energy[g] = bestE[c];
+    }
+    if (rank == 0)
+      for (int c = tid; c < R; c += blockDim.x) a.s.beta_idx[base + c] = B[c];
+    sync_read();  // before the next read's state
   }
   __syncthreads();
   if (tid == 0 && a.advance) {  // the last CTA advances the sweep counter
@@ -544,33 +532,18 @@ __global__ void __launch_bounds__(32 * (kMaxSmallWarps + 1), 1)
   }
 }
 
-cudaError_t launch_small(SmallArgs a, bool random, cudaStream_t st) {
-  if (a.p.num_reads <= 0) return cudaSuccess;
-  // a warp per replica of an average read; reads with more replicas take
-  // turns, and keep their state in global memory
-  const int64_t avg = (a.p.num_chains + a.p.num_reads - 1) / a.p.num_reads;
-  a.cap = (int32_t)(avg < kMaxReplicas ? (avg > 1 ? avg : 1) : kMaxReplicas);
-  a.cap += a.cap & 1;  // pairs of words stay 8-byte aligned
-  // a cluster per read while the reads leave SMs idle and a CTA keeps four
-  // chains or more; the chains of a CTA in equal turns of its warps
-  int cs = 1;
-  while (cs < 8 && a.p.num_reads * cs * 2 <= kSmallFill &&
-         a.cap / (2 * cs) >= 4)
-    cs *= 2;
-  const int per = (a.cap + cs - 1) / cs;
-  const int turns = (per + kMaxSmallWarps - 1) / kMaxSmallWarps;
-  const int nw = (per + turns - 1) / turns;
-  const size_t smem = SmallSmem::bytes(a.cap);
-  const void* f = random ? (const void*)k_sweep_small<true>
-                         : (const void*)k_sweep_small<false>;
-  static std::atomic<uint64_t> allowed[2];
-  cudaError_t e =
-      allow_smem(f, SmallSmem::bytes(kMaxReplicas), allowed[random]);
+template <bool RANDOM, int N>
+static cudaError_t launch_small_t(const SmallArgs& a, int64_t ctas, int cs,
+                                  bool helper, cudaStream_t st) {
+  using Smem = SmallSmem<N>;
+  const void* f = (const void*)k_sweep_small<RANDOM, N>;
+  static std::atomic<uint64_t> allowed;
+  cudaError_t e = allow_smem(f, Smem::bytes(kMaxReplicas), allowed);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(a.p.num_reads * cs));
-  cfg.blockDim = dim3(32 * (nw + 1));
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(32 * (a.warps + (helper ? 1 : 0)));
+  cfg.dynamicSmemBytes = Smem::bytes(a.cap);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -578,8 +551,70 @@ cudaError_t launch_small(SmallArgs a, bool random, cudaStream_t st) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return random ? cudaLaunchKernelEx(&cfg, k_sweep_small<true>, a)
-                : cudaLaunchKernelEx(&cfg, k_sweep_small<false>, a);
+  return cudaLaunchKernelEx(&cfg, k_sweep_small<RANDOM, N>, a);
+}
+
+cudaError_t launch_small(SmallArgs a, bool random, int sms, cudaStream_t st) {
+  if (a.p.num_reads <= 0) return cudaSuccess;
+  // couplings of up to 32 or 64 columns (instances wider than 64, swept
+  // elsewhere, may share the batch)
+  const bool narrow = a.p.max_n <= 32;
+  auto launch = [&](int64_t ctas, int cs, bool helper) {
+    if (narrow)
+      return random ? launch_small_t<true, 32>(a, ctas, cs, helper, st)
+                    : launch_small_t<false, 32>(a, ctas, cs, helper, st);
+    return random ? launch_small_t<true, 64>(a, ctas, cs, helper, st)
+                  : launch_small_t<false, 64>(a, ctas, cs, helper, st);
+  };
+  // The replicas of an average read (of every read in a batch of one
+  // instance).  Reads with far more have a launch of their own below.
+  const int64_t avg = (a.p.num_chains + a.p.num_reads - 1) / a.p.num_reads;
+  const bool mixed = a.p.num_instances > 1;
+  const int64_t room = !mixed ? avg : 2 * avg > 32 ? 2 * avg : 32;
+  a.above = 0;
+  a.cap = (int32_t)(room < kMaxReplicas ? room : kMaxReplicas);
+  a.cap += a.cap & 1;  // pairs of words stay 8-byte aligned
+  // a cluster per read while the reads leave SMs idle (a sixteenth more CTAs
+  // than SMs is still one each for nearly all) and a CTA keeps four chains
+  int cs = 1;
+  while (cs < 8 && a.p.num_reads * cs * 32 <= sms * 17 &&
+         (avg + 1) / (2 * cs) >= 4)
+    cs *= 2;
+  // warps of a CTA: its chains in equal turns, as few turns as the CTAs that
+  // an SM then holds at once (64 registers a thread, shared memory) allow
+  // without more rounds of CTAs
+  // (a short call's time goes into moving the state, by every warp there is)
+  const bool helper = random || (a.use_pt && avg > 1) || a.num_sweeps < 16;
+  const int64_t per = (avg + cs - 1) / cs, ctas = a.p.num_reads * cs;
+  const int64_t smem = 1024 + (int64_t)(narrow ? SmallSmem<32>::bytes(a.cap)
+                                               : SmallSmem<64>::bytes(a.cap));
+  double best = 0.0;
+  a.warps = 0;
+  for (int64_t t = (per + kMaxSmallWarps - 1) / kMaxSmallWarps; t <= per; ++t) {
+    const int64_t w = (per + t - 1) / t;
+    if (a.warps && w == a.warps) continue;
+    int64_t held = 32 / (w + (helper ? 1 : 0));
+    if (held > 233472 / smem) held = 233472 / smem;
+    if (held < 1) held = 1;
+    const int64_t rounds = (ctas + held * sms - 1) / (held * sms);
+    const double cost = (double)rounds * ((double)t + 0.5);
+    if (a.warps == 0 || cost < best) {
+      best = cost;
+      a.warps = (int32_t)w;
+    }
+    if (rounds == 1) break;  // more turns gain nothing
+  }
+  const int32_t advance = a.advance;
+  const bool more = mixed && a.cap < kMaxReplicas;
+  a.advance = more ? 0 : advance;
+  cudaError_t e = launch(ctas, cs, helper);
+  if (e != cudaSuccess || !more) return e;
+  // reads of more replicas: an SM each, all its warps
+  a.above = a.cap;
+  a.cap = kMaxReplicas;
+  a.warps = kMaxSmallWarps;
+  a.advance = advance;
+  return launch(a.p.num_reads < sms ? a.p.num_reads : sms, 1, true);
 }
 
 }  // namespace pysa_gb
