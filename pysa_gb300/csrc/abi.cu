@@ -923,7 +923,8 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
              ws->csr_item_start;
   ca.seed = o->seed;
   ca.width = ws->csr_width;
-  ca.pad_ = 0;
+  ca.sms = sm_count();
+  ca.pick = 0;
   ca.keys = philox_keys(o->seed);
   for (int sw = 0; sw < num_sweeps; ++sw) {
     if (use_tc && (phases & 1)) {

@@ -23,7 +23,9 @@ struct CsrArgs {
   const SweepItem* items;
   uint64_t seed;
   int32_t width;  // 0: grouped rows; 4/8/16/32: fixed records
-  int32_t pad_;
+  int32_t sms;    // SMs of the device
+  // set by launch_csr: instances of every schedule, 1 narrow, 2 wide ones
+  int32_t pick;
   PhiloxKeys keys;  // of seed
 };
 
@@ -35,6 +37,6 @@ struct CsrArgs {
 cudaError_t launch_csr_schedule(const CsrArgs& a, bool random,
                                 cudaStream_t st);
 // One sweep of every work item (a CTA each).
-cudaError_t launch_csr(const CsrArgs& a, bool random, cudaStream_t st);
+cudaError_t launch_csr(CsrArgs a, bool random, cudaStream_t st);
 
 }  // namespace pysa_gb

@@ -23,9 +23,10 @@
 // Bound by instruction issue and, per level, by the latency of one quad's four
 // dependent attempts.  Measured against one thread per chain visiting the
 // positions one by one (times per sweep with the exchange): 64 x 64 lattice,
-// 4000 chains 1.44 -> 0.13 ms in visiting order (79 levels), 1.66 -> 0.25 ms
-// in random order (half of it makes the orders and the schedule); 100 x 100, 2000 chains
-// 3.7 -> 0.39 ms; 33 x 33, 16000 chains 0.43 -> 0.19 ms.
+// 4000 chains 1.44 -> 0.12 ms in visiting order (79 levels), 1.66 -> 0.21 ms
+// in random order (half of it makes the orders and the schedule); ring of 1000,
+// every quad a level, 4000 chains 0.36 -> 0.18, 100 000 0.62 -> 0.48; 2000 spins
+// with 48 neighbours, 4000 chains 6.7 -> 1.3, 100 000 9.8 -> 8.3.
 //
 // Row layout: the entries of row i are grouped by column % 8 (ascending
 // column inside a group) and rows[9 i + k] .. rows[9 i + k + 1] delimit group
@@ -54,11 +55,22 @@ namespace pysa_gb {
 // order, nu, nl.  A unit is quad q, or (when nu > quads) q << 4 | first
 // position in it << 2 | positions - 1.  That takes nu + nl + 4 <= n entries,
 // which quads fit for n >= 10; below that, and where there is no such
-// workspace, every quad is a level of its own.
-constexpr int kSchedMinN = 10;
+// workspace, every quad is a level of its own.  So it is up to n = 32, and in
+// random order to n = 64, where the schedule takes longer than the levels it
+// saves (n = 24, 20 000 chains, random order: 52 us a sweep with it, 39 without).
+__host__ __device__ constexpr int sched_min_n(bool random) {
+  return random ? 65 : 33;
+}
 constexpr int kSchedThreads = 512;
+constexpr int kSchedRounds = 48;
+constexpr int kSchedNames = 32768;  // units named by a stretch of units
 // Widest instance whose quads may be cut (shared memory, 16 bits per unit).
 constexpr int kSchedCutN = 8192;
+
+// Whether a schedule is made by rounds alone (see k_csr_schedule).
+__host__ __device__ constexpr bool sched_by_rounds(bool random, int width) {
+  return random && (width == 4 || width == 8);
+}
 
 // Dynamic shared memory a CTA of these kernels may take (a little is static).
 constexpr size_t kCsrSmem = 232448 - 256;
@@ -82,8 +94,13 @@ __host__ __device__ constexpr size_t sched_bytes(int nu, int n, bool random,
 }
 
 // CTA per instance.  Units are levelled 512 at a time (earlier ones are
-// final), the levels of a chunk raised until none changes; then a counting
-// sort, stable in the position.  When the quads give fewer than 8 per level,
+// final), the levels of a chunk raised until none changes.  That takes as many
+// rounds as the longest chain of units in the chunk, and a round as long as a
+// row, so it is kept for records of 4 entries and, in random order, of 8; other
+// rows, and in visiting order a chunk that is not done after kSchedRounds
+// rounds, take the units in order (a sweep with its schedule in random order,
+// 2000 spins with 32 neighbours 4.03 -> 0.47 ms, 1500 with 100 19.2 -> 3.4).
+// Then a counting sort, stable in the position.  When the quads give fewer than 8 per level,
 // they are cut between positions that do not touch (neither reads the
 // other's spin) and levelled again; the cut schedule is kept when it has
 // less than two thirds of the levels.
@@ -96,7 +113,7 @@ __global__ void __launch_bounds__(kSchedThreads)
   const int inst = blockIdx.x;
   if (a.p.csr_row_off[inst] < 0) return;  // dense
   const int n = a.p.n[inst], nq = csr_quads(n);
-  if (n < kSchedMinN) return;
+  if (n < sched_min_n(RANDOM)) return;
   const uint32_t sweep = (uint32_t)(*a.s.sweep_counter);
   int32_t* row =
       a.perm + ((int64_t)(RANDOM ? sweep % (uint32_t)a.perm_slots : 0u) *
@@ -116,10 +133,18 @@ __global__ void __launch_bounds__(kSchedThreads)
   };
   auto column = [&](int64_t e) { return __ldg(colp + e) & 0x7fffffff; };
   // positions of the spins, and the uncut/cut units' tables behind it
-  uint16_t* inv = reinterpret_cast<uint16_t*>(ssm);  // [n], random
-  unsigned char* tab = ssm + (RANDOM ? 2 * (((size_t)n + 1) & ~1ull) : 0);
+  uint16_t* names = reinterpret_cast<uint16_t*>(ssm);  // see in_order
+  uint16_t* inv =                                      // [n], random
+      names + (sched_by_rounds(RANDOM, a.width) ? 0 : kSchedNames);
+  unsigned char* tab = reinterpret_cast<unsigned char*>(inv) +
+                       (RANDOM ? 2 * (((size_t)n + 1) & ~1ull) : 0);
   bool odd = false;  // a coupling that is no integer below 2^18
+  __shared__ int longest;  // entries of the longest grouped row
+  if (tid == 0) longest = 1;
+  __syncthreads();
   for (int t = tid; t < n; t += blockDim.x) {
+    if (a.width == 0)
+      atomicMax(&longest, rows[(int64_t)t * 9 + 8] - rows[(int64_t)t * 9]);
     if (RANDOM)
       inv[row[t] & 0xFFFF] = (uint16_t)t;
     else
@@ -132,6 +157,7 @@ __global__ void __launch_bounds__(kSchedThreads)
   }
   // up to 32 such couplings add up without rounding, whatever the order
   const bool any_order = !__syncthreads_or(odd) && a.width > 0;
+  const int row_len = a.width > 0 ? a.width : longest;
   auto spin_at = [&](int t) { return RANDOM ? row[t] & 0xFFFF : t; };
   auto pos_of = [&](int i) { return RANDOM ? (int)inv[i] : i; };
 
@@ -177,6 +203,7 @@ __global__ void __launch_bounds__(kSchedThreads)
         __syncthreads();
       }
       nu = carry;
+      if (nu == nq) return;  // nothing to cut (uniform)
       first = reinterpret_cast<uint16_t*>(mem);                  // [nu + 1]
       mem += 2 * (((size_t)nu + 2) & ~1ull);
       for (int t = tid; t < n; t += blockDim.x)
@@ -193,12 +220,98 @@ __global__ void __launch_bounds__(kSchedThreads)
     for (int u = tid; u < nu; u += blockDim.x) lev[u] = 0;
     for (int u = tid; u <= nu; u += blockDim.x) cnt[u] = 0u;
     __syncthreads();
+    auto first_of = [&](int u) { return cut ? (int)first[u] : 4 * u; };
+    auto end_of = [&](int u) {
+      return cut ? (int)first[u + 1] : 4 * u + 4 < n ? 4 * u + 4 : n;
+    };
+    // Levels of units ub ... ue - 1, one after another (the earlier ones are
+    // final).  The CTA gathers the units that a stretch of units names; then
+    // one warp goes through them in shared memory, the next unit's names on
+    // their way (about 150 cycles a unit of up to 128 names).
+    auto in_order = [&](int ub, int ue) {
+      const int per = 4 * row_len, step = max(kSchedNames / per, 1);
+      for (int c0 = ub; c0 < ue; c0 += step) {
+        const int c1 = c0 + step < ue ? c0 + step : ue;
+        for (int k = tid; k < (c1 - c0) * per; k += blockDim.x) {
+          const int u = c0 + k / per, j = k % per;
+          const int t = first_of(u) + j / row_len;
+          int name = u;  // itself: no dependence
+          if (t < end_of(u)) {
+            int64_t e, e1;
+            entries(spin_at(t), e, e1);
+            e += j % row_len;
+            if (e < e1) name = unit_of(pos_of(column(e)));
+          }
+          names[k] = (uint16_t)name;
+        }
+        __syncthreads();
+        if (warp == 0 && per <= 128) {
+          int nx[4];
+          auto load = [&](int u) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              nx[i] = lane + 32 * i < per
+                          ? names[(u - c0) * per + lane + 32 * i]
+                          : u;
+          };
+          load(c0);
+          for (int u = c0; u < c1; ++u) {
+            int at[4], lv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) at[i] = nx[i];
+            const int own = lev[u];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) lv[i] = lev[at[i]];
+            if (u + 1 < c1) load(u + 1);
+            int m = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (at[i] < u) m = max(m, lv[i] + 1);
+            m = max(__reduce_max_sync(0xffffffffu, m), own);
+            if (lane == 0) lev[u] = m;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (at[i] > u)
+                atomicMax(const_cast<int32_t*>(lev) + at[i], m + 1);
+            __syncwarp();
+          }
+        } else if (warp == 0) {
+          for (int u = c0; u < c1; ++u) {
+            const uint16_t* name = names + (u - c0) * per;
+            int m = 0;
+#pragma unroll 4
+            for (int j = lane; j < per; j += 32) {
+              const int at = name[j], lv = lev[at];
+              if (at < u) m = max(m, lv + 1);
+            }
+            m = max(__reduce_max_sync(0xffffffffu, m), lev[u]);
+            if (lane == 0) lev[u] = m;
+#pragma unroll 4
+            for (int j = lane; j < per; j += 32) {
+              const int at = name[j];
+              if (at > u) atomicMax(const_cast<int32_t*>(lev) + at, m + 1);
+            }
+            __syncwarp();
+          }
+        }
+        __syncthreads();
+      }
+    };
     for (int u0 = 0; u0 < nu; u0 += blockDim.x) {
       const int u = u0 + tid;
       int tb = 0, te = 0;
       if (u < nu) {
-        tb = cut ? (int)first[u] : 4 * u;
-        te = cut ? (int)first[u + 1] : (4 * u + 4 < n ? 4 * u + 4 : n);
+        tb = first_of(u);
+        te = end_of(u);
+      }
+      if (a.width != 4 && !sched_by_rounds(RANDOM, a.width)) {
+        if (4 * row_len <= kSchedNames) {
+          in_order(0, nu);
+        } else {  // a row of more entries than fit: every unit a level
+          for (int v = tid; v < nu; v += blockDim.x) lev[v] = v;
+          __syncthreads();
+        }
+        break;
       }
       // the units of the spins that this one reads, the first kDeps of them
       // kept in registers over the rounds (all for rows of 4 entries)
@@ -216,7 +329,11 @@ __global__ void __launch_bounds__(kSchedThreads)
         }
         nd = kDeps;
       }
-      for (;;) {
+      for (int round = 0;; ++round) {
+        if (!RANDOM && round == kSchedRounds) {  // uniform
+          in_order(u0, u0 + (int)blockDim.x < nu ? u0 + (int)blockDim.x : nu);
+          break;
+        }
         bool up = false;
         int m = 0;
         auto meet = [&](int uc) {
@@ -307,7 +424,10 @@ __global__ void __launch_bounds__(kSchedThreads)
       put_high(n - 2, (uint32_t)nu);
       put_high(n - 1, (uint32_t)nl);
     }
-    if (n > kSchedCutN || nq >= 8 * nl) return;  // wide enough (uniform)
+    // wide enough, or too dear for every sweep (uniform)
+    if (n > kSchedCutN || nq >= 8 * nl ||
+        (RANDOM && (a.width == 0 || a.width > 8)))
+      return;
     __syncthreads();
   }
 }
@@ -321,7 +441,8 @@ __global__ void __launch_bounds__(kSchedThreads)
 template <int D>
 struct QuadSlab {
   static constexpr int STRIDE = 2 * D + 4;  // words per record
-  static constexpr int QUAD = 4 * STRIDE;   // words per buffer
+  // words per buffer (grouped rows: 32 entries of one row)
+  static constexpr int QUAD = D > 0 ? 4 * STRIDE : 64;
   // 16-byte pieces of columns and values per record, and per lane and quad
   static constexpr int PIECES = D / 2;
   static constexpr int PER_LANE = (4 * PIECES + 31) / 32;
@@ -364,17 +485,24 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
   const int64_t chain = item.chain0 + lane;
   const uint32_t sweep = (uint32_t)(*a.s.sweep_counter);
 
+  const int32_t* row =
+      a.perm + ((int64_t)(RANDOM ? sweep % (uint32_t)a.perm_slots : 0u) *
+                    a.p.num_instances + inst) * (int64_t)a.p.max_n;
+  const bool scheduled = a.perm && n >= sched_min_n(RANDOM);
+  if (a.pick != 0) {  // a launch of its own for narrow schedules (launch_csr)
+    const bool narrow =
+        !scheduled || ((uint32_t)row[n - 2] >> 16) <
+                          2u * ((uint32_t)row[n - 1] >> 16);
+    if (narrow != (a.pick == 1)) return;
+  }
   // spins in, each word's 32 spins x 32 chains transposed
 #pragma unroll 4
   for (int w = warp; w < words; w += W)
     spin_s[w * 32 + lane] = warp_transpose(
         valid ? a.s.spins[chain * (int64_t)a.p.words + w] : 0u, lane);
-  const int32_t* row =
-      a.perm + ((int64_t)(RANDOM ? sweep % (uint32_t)a.perm_slots : 0u) *
-                    a.p.num_instances + inst) * (int64_t)a.p.max_n;
   int nu = nq, nl = nq;
   bool any_order = false;
-  if (a.perm && n >= kSchedMinN) {
+  if (scheduled) {
     any_order = ((uint32_t)row[n - 3] >> 16) != 0u;
     nu = (int)((uint32_t)row[n - 2] >> 16);
     nl = (int)((uint32_t)row[n - 1] >> 16);
@@ -407,6 +535,12 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
   // records of quad q: 16-byte pieces and h into registers ...
   uint4 rg[Q::PER_LANE > 0 ? Q::PER_LANE : 1];
   float rh = 0.0f;
+  // grouped rows: bounds of the next unit's quad, and of the one being decided
+  // with the first entries of its four rows
+  int rb = 0, re = 0, cb = 0, ce = 0;
+  float ch = 0.0f;
+  uint32_t cc[4] = {0u, 0u, 0u, 0u};
+  float cv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   // the lane's first piece: record pr, columns 4 pk ... or values past them
   const int pr = D > 0 ? lane / (D > 0 ? Q::PIECES : 1) : 0;
   const int pk = D > 0 ? lane % (D > 0 ? Q::PIECES : 1) : 0;
@@ -422,7 +556,20 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
         if (r < 4 && t < n) rg[e] = __ldg(psrc + spin_at(t) * (D / 4));
       }
       if (lane < 4 && 4 * q + lane < n) rh = __ldg(h + spin_at(4 * q + lane));
+    } else {
+      // group starts of position lane / 8, ends and h in lanes 0 .. 3
+      const int t = 4 * q + (lane >> 3), te = 4 * q + lane;
+      rb = t < n ? __ldg(rows + (int64_t)spin_at(t) * 9 + (lane & 7)) : 0;
+      const bool own = lane < 4 && te < n;
+      re = own ? __ldg(rows + (int64_t)spin_at(te) * 9 + 8) : 0;
+      rh = own ? __ldg(h + spin_at(te)) : 0.0f;
     }
+  };
+  // 32 entries of a grouped row, one a lane
+  auto chunk = [&](int e0, int end, uint32_t& c, float& v) {
+    const int e = e0 + lane;
+    c = e < end ? 4u * (uint32_t)__ldg(colp + e) : 0u;
+    v = e < end ? __ldg(valp + e) : 0.0f;
   };
   // ... and from there into slab buffer b: columns become byte offsets of
   // spin words (times 4; bit 31 kept unless the sums need no groups)
@@ -447,6 +594,14 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
             __float_as_uint(rh),
             4 * q + lane < n ? 4u * (uint32_t)spin_at(4 * q + lane) : 0u);
       __syncwarp();
+    } else {
+      cb = rb;
+      ce = re;
+      ch = rh;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        chunk(__shfl_sync(0xffffffffu, cb, 8 * k),
+              __shfl_sync(0xffffffffu, ce, k), cc[k], cv[k]);
     }
   };
   float tl[4], th[4];
@@ -536,20 +691,51 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
       return attempt(exact_t, q, k, tlk, thk, ho.y,
                      sum + __uint_as_float(ho.x));
     } else {
-      const int i = spin_at(4 * q + k);
-      const int32_t* r9 = rows + (int64_t)i * 9;
-      float sum = 0.0f;
+      // 32 entries at a time, the next ones on their way; a lane each holds
+      // the end of a group, where the partial sum joins the total (an empty
+      // group adds nothing)
+      const int beg = __shfl_sync(0xffffffffu, cb, 8 * k);
+      const int end = __shfl_sync(0xffffffffu, ce, k);
+      const int start = __shfl_sync(0xffffffffu, cb, 8 * k + (lane & 7));
+      const int bound = lane == 8 ? end : start;  // in lanes 1 .. 8
+      uint32_t c = k < 2 ? (k ? cc[1] : cc[0]) : (k == 2 ? cc[2] : cc[3]);
+      float v = k < 2 ? (k ? cv[1] : cv[0]) : (k == 2 ? cv[2] : cv[3]);
+      float sum = 0.0f, part = 0.0f;
+      for (int e0 = beg; e0 < end; e0 += 32) {
+        uint32_t cn = 0u;
+        float vn = 0.0f;
+        if (e0 + 32 < end) chunk(e0 + 32, end, cn, vn);
+        const int bit = bound - 1 - e0;
+        const uint32_t last = __reduce_or_sync(
+            0xffffffffu,
+            lane >= 1 && lane <= 8 && bit >= 0 && bit < 32 ? 1u << bit : 0u);
+        const int m = end - e0 < 32 ? end - e0 : 32;
+        // through shared memory: two broadcast loads for four entries
+        uint32_t* s = slab + ((e0 - beg) & 32 ? Q::QUAD : 0);
+        s[lane] = c | (((last >> lane) & 1u) << 31);
+        s[32 + lane] = __float_as_uint(v);
+        __syncwarp();
+#pragma unroll 2
+        for (int j = 0; j < m; j += 4) {
+          const uint4 c4 = *reinterpret_cast<const uint4*>(s + j);
+          const float4 v4 = *reinterpret_cast<const float4*>(s + 32 + j);
+          const uint32_t cs[4] = {c4.x, c4.y, c4.z, c4.w};
+          const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        float part = 0.0f;
-        const int e1 = __ldg(r9 + g + 1);
-        for (int e = __ldg(r9 + g); e < e1; ++e)
-          part += signed_value(4u * (uint32_t)__ldg(colp + e),
-                               __ldg(valp + e));
-        sum += part;
+          for (int i = 0; i < 4; ++i) {
+            part += signed_value(cs[i] & 0x7fffffffu, vs[i]);
+            const bool end_of_group = (int32_t)cs[i] < 0;
+            sum = end_of_group ? sum + part : sum;
+            part = end_of_group ? 0.0f : part;
+          }
+        }
+        c = cn;
+        v = vn;
       }
-      return attempt(exact_t, q, k, tlk, thk, 4u * (uint32_t)i,
-                     sum + __ldg(h + i));
+      __syncwarp();
+      return attempt(exact_t, q, k, tlk, thk,
+                     4u * (uint32_t)spin_at(4 * q + k),
+                     sum + __shfl_sync(0xffffffffu, ch, k));
     }
   };
   auto pick = [&](const float (&v)[4], int k) {
@@ -560,16 +746,17 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
   // the other fetches and draws for the next.  This warp's units: places
   // first(l) + its number in the group, + the group's size, ... of every
   // other level.
-  const int WG = W >> 1, wi = warp % WG;
+  // (Grouped rows may have a lone warp: it takes every level.)
+  const int G = D == 0 && W == 1 ? 1 : 2, WG = W / G, wi = warp % WG;
   const int qshift = cut ? 4 : 0;
   const uint16_t* first = sched + nu;
   auto sweep_all = [&](auto any_order_t) {
-    int l = warp / WG - 2, place = 0, end = 0;
+    int l = warp / WG - G, place = 0, end = 0;
     // on to this warp's next unit
     auto settle = [&]() {
       place += WG;
       while (place >= end) {
-        l += 2;
+        l += G;
         if (l >= nl) return;
         place = (int)first[l] + wi;
         end = (int)first[l + 1];
@@ -677,11 +864,8 @@ __global__ void __launch_bounds__(32 * kCsrWarps, 1)
 }
 
 template <bool RANDOM, bool ISING, int D>
-static cudaError_t launch_csr_t(const CsrArgs& a, cudaStream_t st) {
+static cudaError_t launch_csr_t(const CsrArgs& a, int W, cudaStream_t st) {
   const int n = a.p.max_n;
-  // a level holds a few to a few dozen units, more of them the wider the
-  // instance; two groups of warps share the levels
-  int W = n <= 512 ? 8 : n <= 2048 ? 16 : kCsrWarps;
   auto bytes = [&](int w) {
     return (size_t)((n + 31) / 32) * 128 +
            (size_t)w * (2 * QuadSlab<D>::QUAD * 4 + 256) +
@@ -698,24 +882,28 @@ static cudaError_t launch_csr_t(const CsrArgs& a, cudaStream_t st) {
 }
 
 template <bool RANDOM, bool ISING>
-static cudaError_t launch_csr_w(const CsrArgs& a, cudaStream_t st) {
+static cudaError_t launch_csr_w(const CsrArgs& a, int W, cudaStream_t st) {
   switch (a.width) {
-    case 4: return launch_csr_t<RANDOM, ISING, 4>(a, st);
-    case 8: return launch_csr_t<RANDOM, ISING, 8>(a, st);
-    case 16: return launch_csr_t<RANDOM, ISING, 16>(a, st);
-    case 32: return launch_csr_t<RANDOM, ISING, 32>(a, st);
-    default: return launch_csr_t<RANDOM, ISING, 0>(a, st);
+    case 4: return launch_csr_t<RANDOM, ISING, 4>(a, W, st);
+    case 8: return launch_csr_t<RANDOM, ISING, 8>(a, W, st);
+    case 16: return launch_csr_t<RANDOM, ISING, 16>(a, W, st);
+    case 32: return launch_csr_t<RANDOM, ISING, 32>(a, W, st);
+    default: return launch_csr_t<RANDOM, ISING, 0>(a, W, st);
   }
 }
 
 cudaError_t launch_csr_schedule(const CsrArgs& a, bool random,
                                 cudaStream_t st) {
-  if (a.num_items <= 0 || !a.perm) return cudaSuccess;
+  if (a.num_items <= 0 || !a.perm || a.p.max_n < sched_min_n(random))
+    return cudaSuccess;
   // the larger of all quads and, up to kSchedCutN, as many units as spins
   const int n = a.p.max_n, nc = n < kSchedCutN ? n : kSchedCutN;
   const size_t whole = sched_bytes(csr_quads(n), n, random, false);
   const size_t parts = sched_bytes(nc, nc, random, true);
-  const size_t smem = (whole > parts ? whole : parts) + 16;
+  // (no more than needed: the L1 cache keeps the rest)
+  const size_t smem =
+      (sched_by_rounds(random, a.width) ? 0 : 2 * (size_t)kSchedNames) +
+      (whole > parts ? whole : parts) + 16;
   const void* f = random ? (const void*)k_csr_schedule<true>
                          : (const void*)k_csr_schedule<false>;
   static std::atomic<uint64_t> allowed[2];
@@ -728,14 +916,44 @@ cudaError_t launch_csr_schedule(const CsrArgs& a, bool random,
   return cudaGetLastError();
 }
 
-cudaError_t launch_csr(const CsrArgs& a, bool random, cudaStream_t st) {
+// Warps of a CTA.  A level holds a few to a few dozen units, more of them the
+// wider the instance, so while every SM has at most one CTA it gets the most
+// that have work.  Beyond that CTAs share an SM's 32 warps (64 registers a
+// thread): narrow schedules, whose levels hold a unit or two, in CTAs of few
+// warps, so that all are resident; wide ones in larger CTAs.  Which one an
+// instance has, the device knows: both are launched, and a CTA of the other
+// kind leaves at once.  Measured, us a sweep at 2 / 4 / 8 / 16 / 32 warps: ring
+// of 1000, 100 000 chains 482 / 564 / 912 / 1605 / 3020 (one thread per chain 622),
+// 20 000 chains 205 / 197 / 333 / 469 / 755 (393); 64 x 64 lattice, 100 000 chains
+// 3457 / 2027 / 1852 / 1885 / 2019 (3385), 20 000 1077 / 616 / 575 / 482 / 488
+// (1558), 4000 1007 / 507 / 261 / 155 / 119.
+cudaError_t launch_csr(CsrArgs a, bool random, cudaStream_t st) {
   if (a.num_items <= 0) return cudaSuccess;
   const bool ising = a.p.problem_type == PYSA_GB_ISING;
-  if (random)
-    return ising ? launch_csr_w<true, true>(a, st)
-                 : launch_csr_w<true, false>(a, st);
-  return ising ? launch_csr_w<false, true>(a, st)
-               : launch_csr_w<false, false>(a, st);
+  auto launch = [&](int W) {
+    if (random)
+      return ising ? launch_csr_w<true, true>(a, W, st)
+                   : launch_csr_w<true, false>(a, W, st);
+    return ising ? launch_csr_w<false, true>(a, W, st)
+                 : launch_csr_w<false, false>(a, W, st);
+  };
+  const int n = a.p.max_n;
+  const int most = n <= 512 ? 8 : n <= 2048 ? 16 : kCsrWarps;
+  if (a.num_items <= a.sms) return launch(most);
+  auto fit = [&](int warps, int least) {  // a power of two
+    int w = most;
+    while (w > least && w > warps) w /= 2;
+    return w;
+  };
+  const int share = (a.num_items + a.sms - 1) / a.sms;  // CTAs an SM gets
+  const int few = fit(32 / share, a.width == 0 ? 1 : 2);
+  if (a.width == 0) return launch(few);
+  if (n <= 512) return launch(4);
+  a.pick = 1;
+  cudaError_t e = launch(few);
+  if (e != cudaSuccess) return e;
+  a.pick = 2;
+  return launch(fit(160 / (a.num_items / a.sms), 4));
 }
 
 }  // namespace pysa_gb
