@@ -817,10 +817,12 @@ int pysa_gb_sweeps(const pysa_gb_problems* p, pysa_gb_state* s,
       const int count = ws->tc_variant_count[v];
       if (count == 0) continue;
       // the queue, and before a fold's first launch its items' progress
+      // (fold 2 in launches of one sweep: before each, so that every sweep
+      // starts in sub-blocks, whatever its last block was)
       int32_t* done = ws->tc_sched + 2 + ws->tc_variant_start[v];
       cudaError_t e =
           cudaMemsetAsync(ws->tc_sched, 0, 2 * sizeof(int32_t), st);
-      if (e == cudaSuccess && tc_swept == 0)
+      if (e == cudaSuccess && (tc_swept == 0 || (!fuse && folds[v] == 2)))
         e = cudaMemsetAsync(done, 0, sizeof(int32_t) * (size_t)count, st);
       if (e != cudaSuccess) return cuda_fail(e, "tc schedule reset");
       ta.item_done = reinterpret_cast<uint32_t*>(done);

@@ -1996,14 +1996,16 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
             uint32_t mf = 0u;
 #pragma unroll
             for (int w4 = 0; w4 < 4; ++w4) mf = max(mf, stat_s[(Gb & 1) * 4 + w4]);
-            // (of a whole block's 64 spins: a last block of one spin would
-            // call any chain cold, and its next block took 40 rounds: 65
-            // spins, random order, 71 us a sweep, 29 so.  Not at fold 2,
-            // where the two forms round differently)
-            d64 = a.decision_mode == 1 ||
-                  (a.decision_mode == 0 &&
-                   (F == 2 ? (int)mf <= round_limit
-                           : (int)mf * 64 <= round_limit * kmax));
+            // (of a whole block's 64 spins, and a last block of under 16 says
+            // too little: one of one spin would call any chain cold, and its
+            // next block took 40 rounds: 65 spins, random order, 71 us a
+            // sweep, 29 so.  Not at fold 2, where the two forms round
+            // differently)
+            if (F == 2)
+              d64 = a.decision_mode == 1 ||
+                    (a.decision_mode == 0 && (int)mf <= round_limit);
+            else if (a.decision_mode == 0 && kmax >= 16)
+              d64 = (int)mf * 64 <= round_limit * kmax;
           }
           if (threadIdx.x == 0) {
             stamp(a, Gb, 4);
