@@ -1920,8 +1920,11 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tc(const TcArgs a) {
     #pragma unroll
             for (int j = 0; j < 16; ++j) c3[j] = 0.0f;
             named_sync_dec();  // sub-block 0 decided
-            bool hok = hgo && valid &&
-                       tc_wait(&sh.jbb_full[Gb & 1], (Gb >> 1) & 1, sh, status);
+            // (slots without a chain too: the deciders read their corrections,
+            // and a NaN left there by another kernel would send every one of
+            // their sub-blocks to the exact rule)
+            const bool hok =
+                hgo && tc_wait(&sh.jbb_full[Gb & 1], (Gb >> 1) & 1, sh, status);
             if (hok) {
               float c2[16];
     #pragma unroll
