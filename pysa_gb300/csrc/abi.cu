@@ -665,7 +665,7 @@ int pysa_gb_prepare(const pysa_gb_problems* p, pysa_gb_state* s,
   a.set_energies = set_energies;
   a.init_best = init_best;
   a.best_global = best_global;
-  launch_prepare(a, (cudaStream_t)stream);
+  launch_prepare(a, sm_count(), (cudaStream_t)stream);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "prepare");
   return PYSA_GB_OK;

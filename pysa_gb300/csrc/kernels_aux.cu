@@ -599,27 +599,28 @@ static cudaError_t launch_fields_t(const PrepArgs& a, int csize,
 // then shorter (n = 2048, 256 tiles: 2.21 ms at 1, 2.16 at 2, 1.87 at 4, 2.00
 // at 8; n = 1024, 512 tiles: 1.10, 0.96, 0.96; 13 waves of n = 64 .. 1536:
 // 6.5, 7.0, 8.6).
-static cudaError_t launch_fields(const PrepArgs& a, cudaStream_t st) {
+static cudaError_t launch_fields(const PrepArgs& a, int sms,
+                                 cudaStream_t st) {
   const int64_t chains = a.p.num_chains;
   const int64_t per = chains / (a.p.num_instances > 0 ? a.p.num_instances : 1);
   const int n = a.p.max_n;
-  constexpr int64_t kFill = 2 * 152;  // CTAs that keep the GPU busy
-  if (per >= 64 && n <= 32 && chains / 64 >= kFill)
+  const int64_t fill = 2 * sms;  // CTAs that keep the GPU busy
+  if (per >= 64 && n <= 32 && chains / 64 >= fill)
     return launch_fields_t<1, 1>(a, 1, st);
-  if (per >= 64 && n <= 128 && chains / 64 >= kFill)
+  if (per >= 64 && n <= 128 && chains / 64 >= fill)
     return launch_fields_t<4, 1>(a, 1, st);
   const int passes = (n + 255) / 256;
-  if (per >= 32 && chains / 32 * passes >= kFill) {
+  if (per >= 32 && chains / 32 * passes >= fill) {
     const int64_t tiles = chains / 32;
     int cs = 1;
     while (cs < 8 && cs < passes &&
-           (tiles * cs < kFill ||
-            (cs < 4 && tiles < 8 * kFill && passes % (2 * cs) == 0)))
+           (tiles * cs < fill ||
+            (cs < 4 && tiles < 8 * fill && passes % (2 * cs) == 0)))
       cs *= 2;
     return launch_fields_t<4, 2>(a, cs, st);
   }
   int cs = 1;
-  while (cs < 8 && cs < passes && (chains + 7) / 8 * cs < kFill) cs *= 2;
+  while (cs < 8 && cs < passes && (chains + 7) / 8 * cs < fill) cs *= 2;
   return launch_fields_t<1, 8>(a, cs, st);
 }
 
@@ -643,9 +644,9 @@ __global__ void k_read_init(const PrepArgs a) {
   }
 }
 
-void launch_prepare(const PrepArgs& a, cudaStream_t st) {
+void launch_prepare(const PrepArgs& a, int sms, cudaStream_t st) {
   if (a.p.num_chains > 0 && a.p.num_instances > 0) {
-    launch_fields(a, st);
+    launch_fields(a, sms, st);
     if (a.p.csr_row_off) {
       int warps = (a.p.max_n + 255) / 256;
       warps = warps < 1 ? 1 : warps > kFieldWarps ? kFieldWarps : warps;
