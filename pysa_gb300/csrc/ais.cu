@@ -237,9 +237,9 @@ struct AisThreshold {
 // exact rule.  For few samples: the kernels that hold several samples per
 // warp or thread need fewer instructions each, but too few warps then leave
 // every SM waiting.  A lane keeps the energy change of the position it is
-// numbered after; they are added in f64 after every 32 positions.  Measured for
-// n = 96, 1000 samples, 200 steps: 12.7 ms with 8 samples per warp, 1.57 ms
-// here (random order 1.84).
+// numbered after; they are added in f64, over the lanes once a sweep.  Measured
+// for n = 96, 1000 samples, 200 steps: 12.7 ms with 8 samples per warp, 1.46 ms
+// here (random order 1.73).
 template <int NC, bool RANDOM>
 __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
   extern __shared__ __align__(16) float Jt[];  // [n][32 NC]
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
     const int32_t* perm =
         a.perm + ((int64_t)k * a.num_instances + inst) * a.max_n;
     const AisThreshold at(beta, scale, lr, uniform_ref);
-    double dE = 0.0;  // the sweep's energy change
+    double dE = 0.0;  // the sweep's energy change, this lane's part
     // one sweep; EXACT asks ais_accept where the thresholds have no answer,
     // otherwise returns whether some decision needed it
     auto sweep = [&](auto exact_t) {
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
 #pragma unroll(NC < 8 ? 4 : 2)
           for (int t = t0; t < te; ++t) turn(t);
         }
-        dE -= warp_sum((double)gain);
+        dE -= (double)gain;
       }
       return unsure != 0u;
     };
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(512) k_ais_turn(const AisArgs a) {
       dE = 0.0;
       sweep(std::true_type{});
     }
-    E += dE;
+    E += warp_sum(dE);
     if (a.order == 0)
       lw += ais_dlw(beta, beta_old, (float)E, n, ones(), logp, log1p_,
                     uniform_ref);
@@ -607,18 +607,22 @@ static cudaError_t launch_small_t(const AisArgs& a, int64_t max_samples,
 
 // Few samples: a warp each.  Many: threads (n <= 32) or warps holding several
 // samples, which need fewer instructions per attempt once the GPU is full.
-// Whole calls with 200 (n = 20) or 50 (n >= 50) steps, warp per sample against
-// the kernel for many: n = 20, 4096 samples 2.0 against 2.3 ms; n = 96, 24000
-// samples 9.5 against 12.1; n = 50, 16000 4.0 against 4.4; n = 200, 16000
-// 17.5 against 24.4.
-constexpr int64_t kTurnSamples = 4096;  // n <= 32
+// A thread a sample takes n attempts one after another whatever the number of
+// samples, a warp a sample the same time for any n but more the more samples:
+// 200 steps, warp against thread, n = 8, 2000 samples 0.53 and 0.31 ms, n = 16
+// 0.56 and 0.62, n = 24, 4000 samples 1.00 and 0.95, n = 31, 4870 samples 1.42
+// and 1.42.  Whole calls with 50 steps, warp per sample against several a warp:
+// n = 96, 24000 samples 9.5 and 12.1 ms; n = 50, 16000 4.0 and 4.4; n = 200, 16000
+// 17.5 and 24.4.
+constexpr int64_t kTurnPerSpin = 160;  // n <= 32
 constexpr int64_t kTurnSamplesWide = 24576;
 
 cudaError_t launch_ais(const AisArgs& a, int64_t max_samples, cudaStream_t st) {
   const int64_t total = max_samples * a.num_instances;
   const int nc = (a.max_n + 31) / 32;
   if (nc <= 1) {
-    if (total <= kTurnSamples) return launch_turn_t<1>(a, max_samples, st);
+    if (total <= kTurnPerSpin * (int64_t)a.max_n)
+      return launch_turn_t<1>(a, max_samples, st);
     if (a.max_n <= 8) return launch_small_t<8>(a, max_samples, st);
     if (a.max_n <= 16) return launch_small_t<16>(a, max_samples, st);
     if (a.max_n <= 24) return launch_small_t<24>(a, max_samples, st);
