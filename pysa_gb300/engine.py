@@ -769,23 +769,22 @@ class PTBatch:
     # --------------------------------------------------------- read back
     def _to_host(self, t: torch.Tensor) -> np.ndarray:
         """A device tensor as a new host array.  Large ones pass a pinned
-        buffer of at most 32 MB that the batch keeps: a copy straight into
-        fresh pages has the device fault them in (24.6 MB: 1 to 22 ms; so
-        under 1)."""
+        buffer of at most 32 MB: a copy straight into fresh pages has the
+        device fault them in (24.6 MB: 1 to 22 ms; so under 1).  The buffer
+        is this call's alone, and goes back to torch's pinned allocator."""
         nb = t.numel() * t.element_size()
         if nb < 4 << 20:
             return t.cpu().numpy()
-        if getattr(self, "_pin", None) is None:
-            self._pin = torch.empty(min(nb, 32 << 20), dtype=torch.uint8,
-                                    pin_memory=True)
+        pin = torch.empty(min(nb, 32 << 20), dtype=torch.uint8,
+                          pin_memory=True)
         src = t.contiguous().view(-1).view(torch.uint8)
         out = torch.empty(t.shape, dtype=t.dtype)
         dst = out.view(-1).view(torch.uint8)
-        step = self._pin.numel()
+        step = pin.numel()
         for o in range(0, nb, step):
             m = min(step, nb - o)
-            self._pin[:m].copy_(src[o:o + m])
-            dst[o:o + m].copy_(self._pin[:m])
+            pin[:m].copy_(src[o:o + m])
+            dst[o:o + m].copy_(pin[:m])
         return out.numpy()
 
     def fetch(self) -> dict:

@@ -85,3 +85,37 @@ def test_two_threads_of_different_sizes(kind, large, small, count):
     for a, b in zip(alone, both):
         for k in a:
             assert np.array_equal(a[k], b[k]), k
+
+
+def test_two_threads_fetch_one_batch():
+    """Results of over 4 MB pass a pinned buffer: two threads that read one
+    batch at the same time each get its state, not the other's pieces."""
+    from pysa_gb300 import Instance, PTBatch, pack_spins
+    n, R, reads = 512, 8, 16384
+    b = PTBatch("ising", [Instance(_dense(n), np.zeros(n, np.float32),
+                                   np.geomspace(0.01, 1.0, R).astype(
+                                       np.float32), reads)], kernel="plain")
+    x = np.random.default_rng(0).integers(0, 2, (R * reads, n), np.int8)
+    words = pack_spins(x, "qubo", b.words)
+    b.set_states(words)
+    b.run(2, seed=1)
+    want = b.fetch()
+    assert not np.array_equal(want["spins"], want["best_spins"])
+    wrong, errors = [], []
+
+    def read():
+        try:
+            for _ in range(40):
+                got = b.fetch()
+                wrong.append(not all(np.array_equal(got[k], want[k])
+                                     for k in want))
+        except Exception as e:  # noqa: BLE001 (reported by the test)
+            errors.append(e)
+
+    ts = [threading.Thread(target=read) for _ in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    assert len(wrong) == 80 and not any(wrong)
