@@ -307,8 +307,9 @@ int pysa_gb_set_decision_mode(int32_t mode);
 /* Decision mode 0's switch point: a block is decided in rounds while the
  * previous block's largest flip count of a chain was at most `flips` (0..64),
  * in sequential sub-blocks otherwise.  12, the default, is 4 for n > 1024 and,
- * up to n = 512, in work items of at most 32 chains.  Results depend on it as on the decision mode; process-wide, for launches
- * enqueued after the call.  No counterpart in the reference. */
+ * up to n = 512, in work items of at most 32 chains.  Results depend on it as
+ * on the decision mode; process-wide, for launches enqueued after the call.
+ * No counterpart in the reference. */
 int pysa_gb_set_block_round_limit(int32_t flips);
 
 /* The switch point that mode 0 would use now for an instance of n spins (64
@@ -357,8 +358,8 @@ int pysa_gb_tc_setup(const pysa_gb_problems *p,
                      void *stream);
 
 /* Local fields H = J s + h for every chain, f32 products added up in f32
- * pairs by exact two-sums (in f64 where a sum leaves the f32 range) and
- * rounded once, and (if set_energies) energies E = s.(J s / 2 + h)
+ * pairs by exact two-sums (sparse instances in triples; in f64 where a sum
+ * leaves the f32 range) and rounded once, and (if set_energies) energies E = s.(J s / 2 + h)
  * (pysa/ising.py:32-37, pysa/qubo.py:32-37).  Also sets chain_beta from
  * beta_idx and, if init_best, best_* from the current state
  * (best_global: best_energy = +inf). */

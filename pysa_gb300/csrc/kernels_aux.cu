@@ -80,10 +80,10 @@ struct Triple {
   }
 };
 
-// Sparse instances: f_i = sum over row i's stored entries of J_ij s_j in f64
-// (the products are exact; padding entries have value 0), from the fixed
-// records (width > 0: entries csr_ent_off + width i ...) or the grouped
-// rows (csr_rows, 9 offsets per row).
+// Sparse instances: the terms J_ij s_j of row i's stored entries in order (the
+// products are exact; padding entries have value 0), each given to `add`, from
+// the fixed records (width > 0: entries csr_ent_off + width i ...) or the
+// grouped rows (csr_rows, 9 offsets per row).
 template <typename Add>
 __device__ __forceinline__ void csr_row_terms(const pysa_gb_problems& p,
                                               int inst, int i,
@@ -905,9 +905,10 @@ __global__ void __launch_bounds__(256) k_energy64(
 // f32 rate and one state's n^2 of them took nearly all of the time, so every
 // lane adds its products, which are exact, into triples of f32 (two states at
 // a time) that carry 72 bits, more than the f64 sum they stand in for, and
-// converts once at the end, after the lanes and warps have been added.  Bound by their 14 paired f32 instructions a
-// product and two states.  QUBO, n = 1284, 128 states: 366 us with f64, 99 so.  A state whose sum leaves the f32 range (or meets an infinity or NaN) is
-// added in f64 as before.
+// converts once at the end, after the lanes and warps have been added.  Bound by
+// their 14 paired f32 instructions a product and two states.  QUBO, 128 states,
+// n = 912: 335 us with f64, 103 so; n = 1284: 602 and 192.  A state whose sum
+// leaves the f32 range (or meets an infinity or NaN) is added in f64.
 constexpr int kE64Chunk = 1024;  // rows whose multipliers are staged
 constexpr int kE64Rows = 128;    // rows of a unit
 
