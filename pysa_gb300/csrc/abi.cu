@@ -68,6 +68,7 @@ int pysa_gb_internal_fail(int code, const char* msg) {
 }
 
 static int cuda_fail(cudaError_t e, const char* where) {
+  cudaGetLastError();  // reported here, and not again by a later call
   return fail(PYSA_GB_ERR_CUDA,
               std::string(where) + ": " + cudaGetErrorString(e));
 }
@@ -665,8 +666,7 @@ int pysa_gb_prepare(const pysa_gb_problems* p, pysa_gb_state* s,
   a.set_energies = set_energies;
   a.init_best = init_best;
   a.best_global = best_global;
-  launch_prepare(a, sm_count(), (cudaStream_t)stream);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_prepare(a, sm_count(), (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "prepare");
   return PYSA_GB_OK;
 }

@@ -43,7 +43,7 @@ struct PermArgs {
 void launch_pack_rows(const float* J, int ld, int n, int nc, int ls,
                       float* packed, int count, int64_t j_step,
                       int64_t p_step, cudaStream_t st);
-void launch_prepare(const PrepArgs& a, int sms, cudaStream_t st);
+cudaError_t launch_prepare(const PrepArgs& a, int sms, cudaStream_t st);
 void launch_exchange(const XArgs& a, cudaStream_t st);
 // Visiting orders of the current sweep and the count - 1 after it (slots
 // sweep % perm_slots).

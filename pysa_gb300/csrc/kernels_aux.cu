@@ -644,9 +644,10 @@ __global__ void k_read_init(const PrepArgs a) {
   }
 }
 
-void launch_prepare(const PrepArgs& a, int sms, cudaStream_t st) {
+cudaError_t launch_prepare(const PrepArgs& a, int sms, cudaStream_t st) {
   if (a.p.num_chains > 0 && a.p.num_instances > 0) {
-    launch_fields(a, sms, st);
+    const cudaError_t e = launch_fields(a, sms, st);
+    if (e != cudaSuccess) return e;
     if (a.p.csr_row_off) {
       int warps = (a.p.max_n + 255) / 256;
       warps = warps < 1 ? 1 : warps > kFieldWarps ? kFieldWarps : warps;
@@ -655,6 +656,7 @@ void launch_prepare(const PrepArgs& a, int sms, cudaStream_t st) {
   }
   if (a.p.num_reads > 0)
     k_read_init<<<(unsigned)a.p.num_reads, 128, 0, st>>>(a);
+  return cudaGetLastError();
 }
 
 // ------------------------------------------------------ replica exchange
