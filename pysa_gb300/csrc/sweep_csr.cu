@@ -73,7 +73,7 @@ __host__ __device__ constexpr bool sched_by_rounds(bool random, int width) {
 }
 
 // Dynamic shared memory a CTA of these kernels may take (a little is static).
-constexpr size_t kCsrSmem = 232448 - 256;
+constexpr size_t kCsrSmem = 232448 - 2560;
 
 __host__ __device__ constexpr int csr_quads(int n) { return (n + 3) >> 2; }
 
@@ -100,15 +100,16 @@ __host__ __device__ constexpr size_t sched_bytes(int nu, int n, bool random,
 // rows, and in visiting order a chunk that is not done after kSchedRounds
 // rounds, take the units in order (a sweep with its schedule in random order,
 // 2000 spins with 32 neighbours 4.03 -> 0.47 ms, 1500 with 100 19.2 -> 3.4).
-// Then a counting sort, stable in the position.  When the quads give fewer than 8 per level,
-// they are cut between positions that do not touch (neither reads the
-// other's spin) and levelled again; the cut schedule is kept when it has
+// Then a counting sort, stable in the position.  When the quads give fewer than
+// 8 per level, they are cut between positions that do not touch (neither reads
+// the other's spin) and levelled again; the cut schedule is kept when it has
 // less than two thirds of the levels.
 template <bool RANDOM>
 __global__ void __launch_bounds__(kSchedThreads)
     k_csr_schedule(const CsrArgs a) {
   extern __shared__ __align__(16) unsigned char ssm[];
   __shared__ int max_level;
+  __shared__ int at_s[kSchedThreads + 1];  // see in_order_grouped
   __shared__ int warp_sum_s[kSchedThreads / 32];
   const int inst = blockIdx.x;
   if (a.p.csr_row_off[inst] < 0) return;  // dense
@@ -139,12 +140,7 @@ __global__ void __launch_bounds__(kSchedThreads)
   unsigned char* tab = reinterpret_cast<unsigned char*>(inv) +
                        (RANDOM ? 2 * (((size_t)n + 1) & ~1ull) : 0);
   bool odd = false;  // a coupling that is no integer below 2^18
-  __shared__ int longest;  // entries of the longest grouped row
-  if (tid == 0) longest = 1;
-  __syncthreads();
   for (int t = tid; t < n; t += blockDim.x) {
-    if (a.width == 0)
-      atomicMax(&longest, rows[(int64_t)t * 9 + 8] - rows[(int64_t)t * 9]);
     if (RANDOM)
       inv[row[t] & 0xFFFF] = (uint16_t)t;
     else
@@ -157,7 +153,6 @@ __global__ void __launch_bounds__(kSchedThreads)
   }
   // up to 32 such couplings add up without rounding, whatever the order
   const bool any_order = !__syncthreads_or(odd) && a.width > 0;
-  const int row_len = a.width > 0 ? a.width : longest;
   auto spin_at = [&](int t) { return RANDOM ? row[t] & 0xFFFF : t; };
   auto pos_of = [&](int i) { return RANDOM ? (int)inv[i] : i; };
 
@@ -226,26 +221,23 @@ __global__ void __launch_bounds__(kSchedThreads)
     };
     // Levels of units ub ... ue - 1, one after another (the earlier ones are
     // final).  The CTA gathers the units that a stretch of units names; then
-    // one warp goes through them in shared memory, the next unit's names on
-    // their way (about 150 cycles a unit of up to 128 names).
+    // one warp goes through them in shared memory.  Fixed records: the next
+    // unit's names are on their way (about 150 cycles a unit).
     auto in_order = [&](int ub, int ue) {
-      const int per = 4 * row_len, step = max(kSchedNames / per, 1);
+      const int per = 4 * a.width, step = kSchedNames / per;
       for (int c0 = ub; c0 < ue; c0 += step) {
         const int c1 = c0 + step < ue ? c0 + step : ue;
         for (int k = tid; k < (c1 - c0) * per; k += blockDim.x) {
           const int u = c0 + k / per, j = k % per;
-          const int t = first_of(u) + j / row_len;
-          int name = u;  // itself: no dependence
-          if (t < end_of(u)) {
-            int64_t e, e1;
-            entries(spin_at(t), e, e1);
-            e += j % row_len;
-            if (e < e1) name = unit_of(pos_of(column(e)));
-          }
-          names[k] = (uint16_t)name;
+          const int t = first_of(u) + j / a.width;
+          names[k] = (uint16_t)(
+              t < end_of(u)
+                  ? unit_of(pos_of(
+                        column((int64_t)a.width * spin_at(t) + j % a.width)))
+                  : u);  // itself: no dependence
         }
         __syncthreads();
-        if (warp == 0 && per <= 128) {
+        if (warp == 0) {
           int nx[4];
           auto load = [&](int u) {
 #pragma unroll
@@ -275,26 +267,79 @@ __global__ void __launch_bounds__(kSchedThreads)
                 atomicMax(const_cast<int32_t*>(lev) + at[i], m + 1);
             __syncwarp();
           }
-        } else if (warp == 0) {
-          for (int u = c0; u < c1; ++u) {
-            const uint16_t* name = names + (u - c0) * per;
-            int m = 0;
-#pragma unroll 4
-            for (int j = lane; j < per; j += 32) {
-              const int at = name[j], lv = lev[at];
-              if (at < u) m = max(m, lv + 1);
-            }
-            m = max(__reduce_max_sync(0xffffffffu, m), lev[u]);
-            if (lane == 0) lev[u] = m;
-#pragma unroll 4
-            for (int j = lane; j < per; j += 32) {
-              const int at = name[j];
-              if (at > u) atomicMax(const_cast<int32_t*>(lev) + at, m + 1);
-            }
-            __syncwarp();
+        }
+        __syncthreads();
+      }
+    };
+    // The same for grouped rows, which may be very uneven: as many units at a
+    // time as their entries fit; one that does not fit by itself (four rows of
+    // more than kSchedNames entries) is read from the rows.
+    auto in_order_grouped = [&]() {
+      for (int c0 = 0; c0 < nu;) {
+        int len = 0;
+        if (c0 + tid < nu)
+          for (int t = first_of(c0 + tid), te = end_of(c0 + tid); t < te; ++t) {
+            int64_t e, e1;
+            entries(spin_at(t), e, e1);
+            len += (int)(e1 - e);
+          }
+        int upto = len;  // entries up to this thread's unit
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int up = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += up;
+        }
+        if (lane == 31) warp_sum_s[warp] = upto;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) upto += warp_sum_s[w];
+        at_s[tid + 1] = upto;
+        if (tid == 0) at_s[0] = 0;
+        const int fit =
+            __syncthreads_count(c0 + tid < nu && upto <= kSchedNames);
+        const int c1 = c0 + (fit > 0 ? fit : 1);
+        for (int u = c0 + warp; fit > 0 && u < c1; u += kSchedThreads / 32) {
+          uint16_t* name = names + at_s[u - c0];
+          for (int t = first_of(u), te = end_of(u); t < te; ++t) {
+            int64_t e, e1;
+            entries(spin_at(t), e, e1);
+            for (int64_t x = e + lane; x < e1; x += 32)
+              name[x - e] = (uint16_t)unit_of(pos_of(column(x)));
+            name += e1 - e;
           }
         }
         __syncthreads();
+        if (warp == 0)
+          for (int u = c0; u < c1; ++u) {
+            // f(unit named) over the unit's entries, a lane each
+            auto each = [&](auto f) {
+              if (fit > 0) {
+                const int end = at_s[u - c0 + 1];
+#pragma unroll 4
+                for (int j = at_s[u - c0] + lane; j < end; j += 32)
+                  f((int)names[j]);
+              } else {
+                for (int t = first_of(u), te = end_of(u); t < te; ++t) {
+                  int64_t e, e1;
+                  entries(spin_at(t), e, e1);
+                  for (int64_t x = e + lane; x < e1; x += 32)
+                    f(unit_of(pos_of(column(x))));
+                }
+              }
+            };
+            int m = 0;
+            each([&](int at) {
+              const int lv = lev[at];
+              if (at < u) m = max(m, lv + 1);
+            });
+            m = max(__reduce_max_sync(0xffffffffu, m), lev[u]);
+            if (lane == 0) lev[u] = m;
+            each([&](int at) {
+              if (at > u) atomicMax(const_cast<int32_t*>(lev) + at, m + 1);
+            });
+            __syncwarp();
+          }
+        __syncthreads();
+        c0 = c1;
       }
     };
     for (int u0 = 0; u0 < nu; u0 += blockDim.x) {
@@ -305,12 +350,10 @@ __global__ void __launch_bounds__(kSchedThreads)
         te = end_of(u);
       }
       if (a.width != 4 && !sched_by_rounds(RANDOM, a.width)) {
-        if (4 * row_len <= kSchedNames) {
+        if (a.width > 0)
           in_order(0, nu);
-        } else {  // a row of more entries than fit: every unit a level
-          for (int v = tid; v < nu; v += blockDim.x) lev[v] = v;
-          __syncthreads();
-        }
+        else
+          in_order_grouped();
         break;
       }
       // the units of the spins that this one reads, the first kDeps of them
@@ -947,8 +990,7 @@ cudaError_t launch_csr(CsrArgs a, bool random, cudaStream_t st) {
   };
   const int share = (a.num_items + a.sms - 1) / a.sms;  // CTAs an SM gets
   const int few = fit(32 / share, a.width == 0 ? 1 : 2);
-  if (a.width == 0) return launch(few);
-  if (n <= 512) return launch(4);
+  if (n <= 512) return launch(a.width == 0 ? few : 4);
   a.pick = 1;
   cudaError_t e = launch(few);
   if (e != cudaSuccess) return e;

@@ -67,3 +67,48 @@ def test_many_items_agree_with_few(kind, n, reads, update):
         got.append(b.fetch())
     for k in got[1]:
         assert np.array_equal(got[0][k][:36], got[1][k]), k
+
+
+@pytest.mark.parametrize("update", ["sequential", "random"])
+def test_uneven_rows_match_oracle(oracle, update):
+    """A few spins next to nearly all others, the rest next to few: grouped
+    rows of 1 to 600 entries."""
+    rng = np.random.default_rng(9)
+    n = 700
+    J = _graph(4, n, rng)
+    for hub in (0, 1, 5, 350, 699):
+        J[hub, rng.random(n) < rng.uniform(0.3, 0.9)] = rng.normal()
+    J = np.triu(J, 1) + np.triu(J.T, 1)
+    J = (J + J.T).astype(np.float32)
+    h = rng.normal(size=n).astype(np.float32)
+    _check(oracle, J, J, h, "ising", update, 3, 2, 4)
+
+
+def test_rows_past_the_schedule_buffer():
+    """Four neighbouring positions with more than 32 768 entries together:
+    the schedule reads them from the rows, and the sweep equals the one that
+    takes every quad by itself."""
+    import scipy.sparse as sp
+    from pysa_gb300 import Instance, PTBatch, pack_spins
+    n, hubs = 12000, 4
+    rng = np.random.default_rng(2)
+    i = np.repeat(np.arange(hubs), n - hubs)
+    j = np.tile(np.arange(hubs, n), hubs)
+    k = np.arange(hubs, n - 1)
+    A = sp.coo_matrix((np.r_[rng.integers(1, 4, len(i)), np.ones(len(k))],
+                       (np.r_[i, k], np.r_[j, k + 1])), (n, n))
+    A = sp.csr_matrix(A + A.T, dtype=np.float32)
+    betas = (1.0 / np.geomspace(50.0, 3000.0, 3)).astype(np.float32)
+    got = []
+    for scheduled in (True, False):
+        b = PTBatch("ising", [Instance(A, np.zeros(n, np.float32), betas,
+                                       2)], sparse=True)
+        if not scheduled:
+            b.ws.perm = 0
+        x = np.random.default_rng(3).integers(0, 2, (6, n), np.int8)
+        b.set_states(pack_spins(x, "qubo", b.words))
+        b.run(3, seed=4)
+        got.append(b.fetch())
+    for key in got[0]:
+        assert np.array_equal(got[0][key], got[1][key]), key
+    assert (got[0]["spins"] != pack_spins(x, "qubo", b.words)).any()
